@@ -91,7 +91,9 @@ int qtnh_stream_destroy(void* stream);
  * for the many small tensors of a network, reused without device synchronisation. */
 int qtnh_malloc_async(void** ptr, size_t bytes, void* stream);
 int qtnh_free_async(void* ptr, void* stream);
-/* Number of kernels this library has launched since load (all entry points). */
+/* Number of kernels this library has launched since load (all entry points). A launch that
+ * makes several passes over a state (runs of fused gate pairs on states of up to 2^22
+ * amplitudes) counts each pass, and its table preparation not. */
 uint64_t qtnh_kernel_launch_count(void);
 /* Allocation diagnostics (no counterpart in the reference): `allocations` = how many
  * temporary device buffers (scratch) the entry points have taken from the stream-ordered
@@ -301,7 +303,8 @@ int qtnh_apply_gate_runs(void* state, void* scratch, int32_t rank, const uint64_
 /* CUDA-event timing of the fused gate-pair passes (QTNH_ARITH_BF16X6; measurement
  * support): returns the summed duration (ms) and count of the passes recorded since the
  * previous call (synchronizing on them), then enables (enable != 0) or disables
- * recording. */
+ * recording. Several passes of one launch count each; their duration includes the
+ * preparation of the launch's tables. */
 int qtnh_gate_timing(int enable, double* ms, uint64_t* launches);
 
 /* DiagTensor contraction in place: psi[x] *= d[x restricted to targets] with d the

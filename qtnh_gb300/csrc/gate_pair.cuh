@@ -146,6 +146,33 @@ void launch_pair_chain(void* psi, const double2* ga, const double2* gb, const Pa
                        const ChainRec* rin, ChainRec* rout, bool want_fixed, void* out = nullptr,
                        const BitPerm* perm = nullptr);
 
+// The later passes of a chain over a state of at most this many amplitudes (64 MiB: it stays
+// in L2) go in one launch of the persistent kernel, where a pass costs a grid barrier instead
+// of a launch and a setup; above, one launch per pass. Eight layers of random gate pairs, in
+// milliseconds, launch per pass / persistent: 0.65 / 0.46 at 2^20 amplitudes, 0.98 / 0.79 at
+// 2^21, 1.61 / 1.41 at 2^22, 2.78 / 2.76 at 2^23, 4.90 / 4.99 at 2^24, 19.1 / 20.0 at 2^26
+// (from DRAM the launch per pass, whose CTAs run more out of step, streams faster).
+constexpr uint64_t CHAIN_RESIDENT_AMPS = 1ull << 22;
+// One of those passes: two disjoint two-qubit gates, and the permutation after them (perm) if
+// the pass is to write its outputs permuted, out of place.
+struct ChainStep {
+  PairParams p;
+  const double2* ga;
+  const double2* gb;
+  bool want_fixed;  // write fixed point when the scales allow, else doubles
+  bool perm;
+  uint8_t dst[32];  // make_bit_map
+};
+bool make_bit_map(const dims_t& dims, const std::vector<uint16_t>& ptup, uint8_t dst[32]);
+// Whether a chain of pairs of this shape goes that way, and its most passes per launch.
+bool chain_resident(const PairParams& p);
+int chain_resident_passes();
+// Such a launch: *rin describes the state (what the pass before wrote), *rout receives the
+// record of the last pass (zeroed by the caller). The state moves to the other buffer at
+// every step with a permutation.
+void launch_chain_resident(void* cur, void* oth, const std::vector<ChainStep>& steps, uint64_t ngroups,
+                           const ChainRec* rin, ChainRec* rout, cudaStream_t s);
+
 // Reads and clears the tcgen05 kernel's device error flags (bounded waits that expired).
 uint32_t take_umma_error();
 

@@ -339,10 +339,15 @@ bool fuse_permutes() {
 // Optional CUDA-event timing of the tensor-core gate-pass launches (qtnh_gate_timing).
 std::mutex g_pass_mu;
 bool g_pass_timing = false;
-std::vector<std::pair<cudaEvent_t, cudaEvent_t>> g_pass_events;
+struct PassEvents {
+  cudaEvent_t e0, e1;
+  uint64_t passes;  // fused passes between the two
+};
+std::vector<PassEvents> g_pass_events;
 
+// Issues `passes` fused passes, one launch.
 template <typename F>
-void timed_pass(cudaStream_t s, F&& launch) {
+void timed_pass(cudaStream_t s, uint64_t passes, F&& launch) {
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   {
     std::lock_guard<std::mutex> lk(g_pass_mu);
@@ -356,7 +361,7 @@ void timed_pass(cudaStream_t s, F&& launch) {
   if (e1) {
     check_cuda(cudaEventRecord(e1, s), "event record");
     std::lock_guard<std::mutex> lk(g_pass_mu);
-    g_pass_events.emplace_back(e0, e1);
+    g_pass_events.push_back({e0, e1, passes});
   }
 }
 
@@ -437,35 +442,64 @@ bool apply_gate_runs_tc(void* state, void* scratch, dims_t dims, const std::vect
       ++j;
     }
     if (R >= 2 && chain_enabled()) {
+      // the first pass is a launch of its own (per-group scales); the later ones of a state that
+      // L2 holds go in launches of up to chain_resident_passes() passes, which end early only at
+      // a permutation that cannot be folded into the pass before it
+      const uint64_t ngroups = steps[i].p.ngroups;
+      const bool resident = chain_resident(steps[i].p);
+      // one record per launch
       ChainRec* recs = static_cast<ChainRec*>(workspace_alloc(R * sizeof(ChainRec), stream));
       try {
         check_cuda(cudaMemsetAsync(recs, 0, R * sizeof(ChainRec), s), "clear chain records");
-        size_t k = 0, t = i;
+        size_t k = 0, t = i, launches = 0;
+        std::vector<ChainStep> open;
+        auto flush = [&] {
+          if (open.empty()) return;
+          timed_pass(s, open.size(), [&] {
+            launch_chain_resident(cur, oth, open, ngroups, &recs[launches], &recs[launches + 1], s);
+          });
+          ++launches;
+          count_launch(open.size());
+          for (const ChainStep& c : open)
+            if (c.perm) std::swap(cur, oth);
+          open.clear();
+        };
         for (; t <= last; ++t) {
           const LayerStep& sk = steps[t];
           if (sk.perm >= 0) {
+            flush();
             permute(sk);
             continue;
           }
-          double2* psi = static_cast<double2*>(cur);
-          // a chain pass followed by a permutation writes its outputs permuted, out of place
-          BitPerm bp;
-          const bool fuse = k > 0 && t + 1 < steps.size() && steps[t + 1].perm >= 0 && fuse_permutes() &&
-                            make_bit_perm(steps[t + 1].dims, runs[(size_t)steps[t + 1].perm].ptup, sk.p, bp);
-          if (k == 0)
-            timed_pass(s, [&] { launch_pair_umma(psi, gate_ptr(sk.g), gate_ptr(sk.g + 1), sk.p, s, PAIR_KRON, &recs[0]); });
-          else
-            timed_pass(s, [&] {
-              launch_pair_chain(psi, gate_ptr(sk.g), gate_ptr(sk.g + 1), sk.p, s, &recs[k - 1], &recs[k], k + 1 < R,
-                                fuse ? oth : nullptr, fuse ? &bp : nullptr);
+          if (k == 0) {
+            timed_pass(s, 1, [&] {
+              launch_pair_umma(static_cast<double2*>(cur), gate_ptr(sk.g), gate_ptr(sk.g + 1), sk.p, s, PAIR_KRON, &recs[0]);
             });
-          count_launch();
-          ++k;
-          if (fuse) {
-            std::swap(cur, oth);
-            ++t;  // the permutation is done
+            count_launch();
+          } else {
+            // a permutation after the pass: its outputs go permuted, out of place
+            const LayerStep* next = t + 1 < steps.size() && steps[t + 1].perm >= 0 && fuse_permutes() ? &steps[t + 1] : nullptr;
+            bool fuse = false;
+            if (resident) {
+              ChainStep c{sk.p, gate_ptr(sk.g), gate_ptr(sk.g + 1), k + 1 < R, false, {}};
+              fuse = c.perm = next && make_bit_map(next->dims, runs[(size_t)next->perm].ptup, c.dst);
+              open.push_back(c);
+              if ((int)open.size() == chain_resident_passes()) flush();
+            } else {
+              BitPerm bp;
+              fuse = next && make_bit_perm(next->dims, runs[(size_t)next->perm].ptup, sk.p, bp);
+              timed_pass(s, 1, [&] {
+                launch_pair_chain(cur, gate_ptr(sk.g), gate_ptr(sk.g + 1), sk.p, s, &recs[k - 1], &recs[k], k + 1 < R,
+                                  fuse ? oth : nullptr, fuse ? &bp : nullptr);
+              });
+              count_launch();
+              if (fuse) std::swap(cur, oth);
+            }
+            if (fuse) ++t;  // the permutation is done
           }
+          ++k;
         }
+        flush();
         check_cuda(cudaGetLastError(), "gate chain launch");
         i = t;
       } catch (...) {
@@ -477,7 +511,7 @@ bool apply_gate_runs_tc(void* state, void* scratch, dims_t dims, const std::vect
     }
     const LayerStep& st = steps[i];
     if (st.pair)
-      timed_pass(s, [&] { launch_fused_pair(static_cast<double2*>(cur), gate_ptr(st.g), gate_ptr(st.g + 1), st.p,
+      timed_pass(s, 1, [&] { launch_fused_pair(static_cast<double2*>(cur), gate_ptr(st.g), gate_ptr(st.g + 1), st.p,
                                             product(st.dims), s); });
     else
       apply_gate_device(cur, st.dims, targets[st.g], gates[st.g], stream);
@@ -495,20 +529,21 @@ void apply_gate_layer_tc(void* state, const dims_t& dims, const std::vector<std:
 }
 
 void take_pass_times(double& ms, uint64_t& launches) {
-  std::vector<std::pair<cudaEvent_t, cudaEvent_t>> ev;
+  std::vector<PassEvents> ev;
   {
     std::lock_guard<std::mutex> lk(g_pass_mu);
     ev.swap(g_pass_events);
   }
   ms = 0;
-  launches = ev.size();
+  launches = 0;
   for (auto& e : ev) {
     float t = 0;
-    check_cuda(cudaEventSynchronize(e.second), "event synchronize");
-    check_cuda(cudaEventElapsedTime(&t, e.first, e.second), "event elapsed");
+    check_cuda(cudaEventSynchronize(e.e1), "event synchronize");
+    check_cuda(cudaEventElapsedTime(&t, e.e0, e.e1), "event elapsed");
     ms += t;
-    cudaEventDestroy(e.first);
-    cudaEventDestroy(e.second);
+    launches += e.passes;
+    cudaEventDestroy(e.e0);
+    cudaEventDestroy(e.e1);
   }
 }
 

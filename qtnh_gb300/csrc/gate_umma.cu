@@ -89,6 +89,15 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
+      "l"(src), "r"(bytes), "r"(smem_u32(bar))
+      : "memory");
+}
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -836,6 +845,683 @@ __global__ void __launch_bounds__(CH_THREADS, 1) gate_pair_chain_kernel(void* __
   }
 }
 
+// ---- the later passes of a chain over a state that L2 holds: all of them in one launch ----
+
+constexpr int CR_MAXP = 64;  // passes (and permutations) of one launch
+
+// One pass's operator as the chain kernel reads it, built once by chain_prep_kernel (device
+// memory): the six gate digits of both K-steps in the UMMA layout -- and, for seven
+// levels, a zero seventh block stacked along N (it makes the first MMA write every level
+// block) --, the rows' exponents, and the operator itself for the FP64 form.
+struct ChainDigits {
+  uint8_t bdig[2][CH_NLMAX][UM_N * 32];  // K-step, digit (1 KB each)
+  int32_t erow[16];
+  int32_t max_erow;
+  int32_t common;   // one digit scale for all rows
+  int32_t gate_ok;  // 0: entries the digits cannot carry
+  int32_t pad;
+};
+struct ChainGate {
+  ChainDigits d;  // copied to shared memory
+  double2 U16[256];
+};
+static_assert(sizeof(ChainGate) % 16 == 0 && sizeof(ChainDigits) % 16 == 0, "bulk copies go in 16-byte steps");
+
+// What chain_prep_kernel builds: the operators of `npass` passes and the bit tables of
+// `nperm` permutations.
+struct ChainPrepParams {
+  const double2* ga[CR_MAXP];
+  const double2* gb[CR_MAXP];
+  uint8_t mode[CR_MAXP];                // PairGate
+  uint8_t dst[CR_MAXP][32];             // permutation: output bit of every index bit (32: none)
+};
+
+// A pass of one launch of the chain kernel (kernel parameter).
+struct ChainPassP {
+  uint64_t tgt[4];  // masks of the target bits of amplitude index bits 3, 2, 1, 0
+  uint64_t step;    // from one tile of a CTA to its next: 128 x grid in the group index's bits
+  uint8_t ins[4];   // the four target bits, ascending
+  int16_t perm;     // >= 0: the outputs go to the other buffer, permuted by table `perm`
+  uint16_t want_fixed;
+};
+struct ChainPasses {
+  ChainPassP p[CR_MAXP];
+};
+
+// Tables of one launch: block i < npass the operator of pass i, the rest one permutation
+// each. Kept out of the chain kernel: built there by every CTA of every pass (FP64 on a
+// unit at 1/58 of the FP32 rate, in a chain of barriers) they were most of a pass on small
+// states.
+__global__ void __launch_bounds__(128) chain_prep_kernel(const __grid_constant__ ChainPrepParams q, int npass,
+                                                         int nlevels, ChainGate* __restrict__ gates,
+                                                         uint32_t* __restrict__ ptabs) {
+  const int tid = threadIdx.x;
+  if ((int)blockIdx.x >= npass) {
+    const int k = (int)blockIdx.x - npass;
+    uint32_t* tab = ptabs + (size_t)k * 1024;
+    for (int t = tid; t < 1024; t += 128) {
+      const int byte = t >> 8, v = t & 255;
+      uint32_t x = 0;
+      for (int j = 0; j < 8; ++j) {
+        const uint32_t d = q.dst[k][8 * byte + j];
+        if (((v >> j) & 1) && d < 32) x |= 1u << d;
+      }
+      tab[t] = x;
+    }
+    return;
+  }
+  __shared__ double2 U16[256];
+  __shared__ int32_t erow[16];
+  __shared__ int ok_all;
+  const double2* ga = q.ga[blockIdx.x];
+  const double2* gb = q.gb[blockIdx.x];
+  const uint32_t mode = q.mode[blockIdx.x];
+  ChainGate& g = gates[blockIdx.x];
+  if (tid == 0) ok_all = 1;
+  for (int t = tid; t < 256; t += 128) {
+    const double2 u = mode == PAIR_KRON     ? fused_entry<PAIR_KRON>(ga, gb, t)
+                      : mode == PAIR_FULL   ? fused_entry<PAIR_FULL>(ga, gb, t)
+                                            : fused_entry<PAIR_KRON_I2>(ga, gb, t);
+    U16[t] = u;
+    g.U16[t] = u;
+  }
+  __syncthreads();
+  if (tid < 16) {
+    bool ok;
+    erow[tid] = (int32_t)row_exponent(U16, tid, ok);
+    g.d.erow[tid] = erow[tid];
+    if (!ok) ok_all = 0;
+  }
+  __syncthreads();
+  int max_erow = 0, min_erow = 0x7FFFFFFF;
+#pragma unroll
+  for (int o = 0; o < 16; ++o) max_erow = max(max_erow, erow[o]), min_erow = min(min_erow, erow[o]);
+  const bool common = max_erow - min_erow <= oz::CHAIN_COMMON_SPAN;
+  if (tid == 0) {
+    g.d.max_erow = max_erow;
+    g.d.common = common ? 1 : 0;
+    g.d.gate_ok = ok_all;
+  }
+  // B row n = output real (amplitude n / 2, real or imaginary part n % 2), K column k = input
+  // real (amplitude k / 2, part k % 2): real and imaginary parts interleaved, so that the
+  // 8 reals of 4 amplitudes are one core-matrix row (state digits) and 8 adjacent columns
+  // (level sums)
+  const int o = tid >> 2, kc = tid & 3;
+  const int ro = (o & 1) * 16 + (o >> 1);  // the row of the real form R
+  const uint32_t E = oz::digit_scale((uint32_t)(common ? max_erow : erow[o >> 1]));
+  float d[8][oz::NS];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const int k = kc * 8 + e;
+    oz::digits(df::words(real_form(U16, ro, (k & 1) * 16 + (k >> 1))), E, d[e]);
+  }
+  const int at = (o >> 3) * 256 + (kc & 1) * 128 + (o & 7) * 16;
+#pragma unroll
+  for (int j = 0; j < oz::NS; ++j)
+    *reinterpret_cast<uint4*>(&g.d.bdig[kc >> 1][j][at]) =
+        make_uint4(pack_h(d[0][j], d[1][j]), pack_h(d[2][j], d[3][j]), pack_h(d[4][j], d[5][j]), pack_h(d[6][j], d[7][j]));
+  if (nlevels > oz::NS)  // the seventh gate digit: zero (the first MMA then writes level 6 too)
+    *reinterpret_cast<uint4*>(&g.d.bdig[kc >> 1][CH_NLMAX - 1][at]) = make_uint4(0u, 0u, 0u, 0u);
+}
+
+// Shared memory of a chain CTA (one per SM): two buffers of state digits (K-major core
+// layout as UmSmem), two of gate digits (this pass's and the next one's), the stage.
+struct CrSmem {
+  uint8_t adig[2][CH_ND][2][UM_M * 32];  // state digits: buffer, digit, K-step (4 KB each)
+  ChainDigits gd[2];                     // gate digits: pass % 2
+  double2 stage[2][16][UM_M];            // fetched amplitudes (or fixed-point pairs), two tiles ahead
+  uint64_t full[2];                      // digits of the tiles using buffer b are ready
+  uint64_t done[2];                      // MMAs into accumulator set b are complete
+  uint64_t gate[2];                      // the gate digits of the passes using buffer b have landed
+  uint32_t tmem_base;
+  int abort;
+  int no_abort;                          // stays 0: the final waits for work in flight
+  uint32_t okey, ominc, ohi;             // what this CTA's outputs of the pass record (ChainRec)
+  uint32_t all_hi;                       // every CTA's ohi
+  uint32_t mine, t0;                     // this CTA's tiles per pass; its tiles of the earlier passes
+  const void* in;
+  void* out;
+  // the pass's address steps, as IT: s0, s1, step, holes, w0, w1 (s, w: the target bits of
+  // amplitude index bits 1 and 0 and their images); held in registers across the tile loop
+  // they would spill
+  alignas(16) uint64_t addr[8];
+  uint32_t ptab[4][256];                 // the permutation's bit tables
+};
+static_assert(CH_NLMAX * UM_N <= (int)CH_ACC, "chain level sums exceed an accumulator set");
+static_assert(2 * CH_ACC <= CH_TMEM_COLS, "two accumulator sets");
+static_assert(sizeof(CrSmem) + 1024 <= 227 * 1024, "chain shared memory");
+
+__device__ __forceinline__ uint64_t ld_acquire(const uint64_t* p) {
+  uint64_t v;
+  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void red_add_release(uint64_t* p, uint64_t v) {
+  asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ void red_or_relaxed(uint32_t* p, uint32_t v) {
+  asm volatile("red.relaxed.gpu.global.or.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// The image of a part of an element index under a pass's permutation (bit tables).
+__device__ __forceinline__ uint32_t chain_image(const uint32_t (*tab)[256], uint32_t x) {
+  return tab[0][x & 255u] | tab[1][(x >> 8) & 255u] | tab[2][(x >> 16) & 255u] | tab[3][x >> 24];
+}
+// Zero bits inserted at the four target positions of a group index.
+template <typename IT>
+__device__ __forceinline__ IT chain_base(IT b, const ChainPassP& pp) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const IT low = b & ((IT(1) << pp.ins[j]) - 1);
+    b = ((b >> pp.ins[j]) << (pp.ins[j] + 1)) | low;
+  }
+  return b;
+}
+// The target bits as one mask, and the tile part of a CTA's next tile: an addition in the
+// group index's bits, the target bits set so that carries run across them.
+template <typename IT>
+__device__ __forceinline__ IT chain_holes(const ChainPassP& pp) {
+  return (IT)(pp.tgt[0] | pp.tgt[1] | pp.tgt[2] | pp.tgt[3]);
+}
+template <typename IT>
+__device__ __forceinline__ IT chain_next_tile(IT tb, IT step, IT holes) {
+  return ((tb | holes) + step) & ~holes;
+}
+// Index of amplitude 4h of row r relative to the tile's first group.
+template <typename IT>
+__device__ __forceinline__ IT chain_row(const ChainPassP& pp, int h, int r) {
+  return chain_base<IT>((IT)r, pp) | ((h & 2) ? (IT)pp.tgt[0] : IT(0)) | ((h & 1) ? (IT)pp.tgt[1] : IT(0));
+}
+
+// The four amplitudes of row r at `at` into stage slot `slot` (one commit group per tile,
+// empty past the end); s0, s1: the target bits of amplitude index bits 1 and 0.
+template <typename IT>
+__device__ __forceinline__ void chain_fetch(CrSmem& sm, const void* in, bool live, IT at, IT s0, IT s1, uint32_t slot,
+                                            int h, int r) {
+  if (live) {
+    const double2* src = static_cast<const double2*>(in) + at;
+    double2* dst = &sm.stage[slot][4 * h][r];
+    cp_async16(dst, src);
+    cp_async16(dst + UM_M, src + s1);
+    cp_async16(dst + 2 * UM_M, src + s0);
+    cp_async16(dst + 3 * UM_M, src + (s0 + s1));
+  }
+  cp_async_commit();
+}
+
+extern __shared__ __align__(1024) unsigned char resident_smem[];
+
+// A pass's scale in one word: flags, the shift of a fixed-point input (6 bits, signed), the
+// input's exponent (the rest, signed).
+constexpr uint32_t CH_IN_FIXED = 1u, CH_OUT_FIXED = 2u, CH_COMMON = 4u, CH_ODD = 8u;  // CH_ODD: gate digits in buffer 1
+__device__ __forceinline__ uint32_t chain_scale(uint32_t flags, int32_t sh, int Ein) {
+  return flags | ((uint32_t)(sh & 63) << 4) | ((uint32_t)Ein << 10);
+}
+__device__ __forceinline__ int32_t chain_scale_sh(uint32_t sc) { return (int32_t)(sc << 22) >> 26; }
+__device__ __forceinline__ int chain_scale_ein(uint32_t sc) { return (int)sc >> 10; }
+
+// The team's part of a pass, tiles sm.t0 on of the CTA (rbase: chain_row, tb: the first
+// tile's part; the first two tiles are being fetched): digits at the common scale;
+// recombination and store one tile behind. FAST: fixed point in and out, one scale for all
+// rows and a right shift (all passes of a long chain but its first and last); the general
+// form's further registers would spill in the loop. Not inlined for the same reason: the
+// kernel's own state stays out of the loop (and few arguments, or they come from the stack in
+// the loop; the rest is in shared memory). sc: chain_scale. false: a wait expired.
+template <typename IT, int NL, bool FAST, bool PO>
+__device__ __noinline__ bool chain_team_pass(IT rbase, IT tb, uint32_t sc) {
+  CrSmem& sm = *reinterpret_cast<CrSmem*>(resident_smem);
+  const int h = (int)(threadIdx.x >> 7), r = (int)(threadIdx.x & 127);
+  // this thread's 8 reals (amplitudes 4h .. 4h + 3, real and imaginary parts interleaved)
+  // are row r of K core h: K-step h / 2, core h % 2
+  const uint32_t row_off = (uint32_t)((r >> 3) * 256 + (r & 7) * 16 + (h & 1) * 128);
+  const IT* ad = reinterpret_cast<const IT*>(sm.addr);  // s0, s1, step, holes, w0, w1
+  const void* in = sm.in;
+  void* out = sm.out;
+  const uint32_t t0 = sm.t0, t1 = t0 + sm.mine;
+  const int32_t sh = chain_scale_sh(sc);
+  const uint64_t cadd = oz::fixed_addend(sh);
+  // where amplitude 4h of row r goes, relative to the image of the tile part
+  const IT wbase = PO ? (IT)chain_image(sm.ptab, (uint32_t)rbase) : rbase;
+  const bool in_fixed = FAST || (sc & CH_IN_FIXED), out_fixed = FAST || (sc & CH_OUT_FIXED), common = FAST || (sc & CH_COMMON);
+  const ChainDigits& gd = sm.gd[(sc & CH_ODD) ? 1 : 0];
+  // per output 4h + a: the row shift to the common output scale, 8 bits each
+  uint32_t kk = 0;
+  if (!FAST && !common) {
+#pragma unroll
+    for (int a = 0; a < 4; ++a) kk |= (uint32_t)min(62, gd.max_erow - gd.erow[4 * h + a]) << (8 * a);
+  }
+  uint32_t okey = 0, ohi = 0;
+  const uint32_t tlane = sm.tmem_base + ((uint32_t)(r & ~31) << 16) + (uint32_t)(8 * h);
+  // level sums from accumulator set b -> the outputs 4h .. 4h + 3 of group r of the tile
+  // whose tile part is tp
+  auto recombine = [&](IT tp, uint32_t b) {
+    uint32_t v[NL][8];  // level l, output real 8h + 2a + part
+#pragma unroll
+    for (int l = 0; l < NL; ++l) tmem_ld8(tlane + b * CH_ACC + (uint32_t)(32 * l), v[l]);
+    const IT obase = (PO ? (IT)chain_image(sm.ptab, (uint32_t)tp) : tp) | wbase;
+    const IT w0 = ad[4], w1 = ad[5];
+    tmem_wait_ld();
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+      float cr[NL], ci[NL];
+#pragma unroll
+      for (int l = 0; l < NL; ++l) cr[l] = __uint_as_float(v[l][2 * a]), ci[l] = __uint_as_float(v[l][2 * a + 1]);
+      int64_t Tr, Ti;
+      if constexpr (NL == 7) {
+        Tr = oz::fixed_levels_merged(cr), Ti = oz::fixed_levels_merged(ci);
+      } else {
+        Tr = oz::fixed_levels<NL>(cr), Ti = oz::fixed_levels<NL>(ci);
+      }
+      const IT ix = obase + ((a & 2) ? w0 : IT(0)) + ((a & 1) ? w1 : IT(0));
+      if (out_fixed) {
+        if (!FAST && !common) {
+          const uint32_t sk = (kk >> (8 * a)) & 0xFFu;
+          const int64_t rh = ((int64_t)1 << sk) >> 1;  // rounding half (0 for no shift)
+          Tr = (Tr + rh) >> sk, Ti = (Ti + rh) >> sk;
+        }
+        ohi |= oz::fixed_hi_mag(Tr) | oz::fixed_hi_mag(Ti);  // its bit length is the largest's
+        static_cast<longlong2*>(out)[ix] = make_longlong2(Tr, Ti);
+      } else {
+        const int e = gd.max_erow - (int)((kk >> (8 * a)) & 0xFFu) + chain_scale_ein(sc) - 2060;
+        const double2 vv = make_double2(oz::fixed_to_double(Tr, e), oz::fixed_to_double(Ti, e));
+        okey = max(okey, amp_key(vv));
+        static_cast<double2*>(out)[ix] = vv;
+      }
+    }
+  };
+  IT tb_f = chain_next_tile(tb, ad[2], ad[3]);  // tile part of the last tile fetched; tb: of the next one to store
+  bool ok = true;
+  for (uint32_t t = t0; t < t1; ++t) {
+    const uint32_t b = t & 1u;
+    cp_async_wait_one();  // tile t has landed (tile t + 1 may still be in flight)
+    double2 x[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) x[c] = sm.stage[b][4 * h + c][r];
+    tb_f = chain_next_tile(tb_f, ad[2], ad[3]);
+    chain_fetch<IT>(sm, in, t + 2 < t1, tb_f | rbase, ad[0], ad[1], b, h, r);  // only this thread reads its stage slots
+    // digits of this thread's 8 reals: digit j of amplitude 4h + a as one fp16x2 word (real,
+    // imaginary); the four words of digit j fill the thread's core-matrix row
+    uint32_t w[4][CH_ND];
+    if (in_fixed) {
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        const int64_t xr = (int64_t)df::d2u(x[a].x), xi = (int64_t)df::d2u(x[a].y);
+        if (FAST)
+          oz::digit_words_biased(((uint64_t)xr + cadd) >> sh, ((uint64_t)xi + cadd) >> sh, w[a]);
+        else
+          oz::digit_words_biased(oz::fixed_biased(xr, sh, cadd), oz::fixed_biased(xi, sh, cadd), w[a]);
+#pragma unroll
+        for (int j = 0; j < CH_ND; ++j) w[a][j] = unbias_h(w[a][j]);
+      }
+    } else {
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        float dr[CH_ND], di[CH_ND];
+        oz::digits(df::words(x[a].x), (uint32_t)chain_scale_ein(sc), dr);
+        oz::digits(df::words(x[a].y), (uint32_t)chain_scale_ein(sc), di);
+#pragma unroll
+        for (int j = 0; j < CH_ND; ++j) w[a][j] = pack_h(dr[j], di[j]);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < CH_ND; ++j)
+      *reinterpret_cast<uint4*>(&sm.adig[b][j][h >> 1][row_off]) = make_uint4(w[0][j], w[1][j], w[2][j], w[3][j]);
+    fence_proxy_async();
+    tc_fence_before();  // this thread's reads of set b (tile t - 2) precede the MMAs of tile t
+    mbar_arrive(&sm.full[b]);
+    if (t != t0) {
+      if (!mbar_wait_warp(&sm.done[b ^ 1u], ((t - 1) >> 1) & 1u, &sm.abort)) {
+        ok = false;
+        break;
+      }
+      tc_fence_after();
+      recombine(tb, b ^ 1u);
+      tb = chain_next_tile(tb, ad[2], ad[3]);
+    }
+  }
+  if (ok) {  // the last tile
+    const uint32_t t = t1 - 1;
+    if (mbar_wait_warp(&sm.done[t & 1u], (t >> 1) & 1u, &sm.abort)) {
+      tc_fence_after();
+      recombine(tb, t & 1u);
+    } else {
+      ok = false;
+    }
+  }
+  cp_async_wait_all();
+  ohi = __reduce_or_sync(0xffffffffu, ohi);
+  if (!FAST) okey = __reduce_max_sync(0xffffffffu, okey);
+  if ((r & 31) == 0) {
+    if (!FAST && okey) atomicMax(&sm.okey, okey);
+    if (ohi) atomicOr(&sm.ohi, ohi);
+  }
+  return ok;
+}
+
+// Every group of a pass in FP64 (no tensor cores): thread per group, doubles out; the
+// output range is recorded like the first pass's, so a later pass starts no chain on it.
+// Loads bypass L1, which may hold lines of an earlier pass.
+template <typename IT>
+__device__ __noinline__ void chain_pass_fp64(CrSmem& sm, const ChainPassP& pp, const void* in, double2* out,
+                                             const double2* U16, uint64_t ngroups, int in_fixed, int32_t F) {
+  uint32_t okey = 0, ominc = 0;
+  for (uint64_t grp = (uint64_t)blockIdx.x * CH_THREADS + threadIdx.x; grp < ngroups;
+       grp += (uint64_t)gridDim.x * CH_THREADS) {
+    const IT base = chain_base<IT>((IT)grp, pp);
+    auto at = [&](int c) -> IT {
+      return base | ((c & 8) ? (IT)pp.tgt[0] : IT(0)) | ((c & 4) ? (IT)pp.tgt[1] : IT(0)) |
+             ((c & 2) ? (IT)pp.tgt[2] : IT(0)) | ((c & 1) ? (IT)pp.tgt[3] : IT(0));
+    };
+    double2 x[16];
+#pragma unroll
+    for (int c = 0; c < 16; ++c) {
+      const IT ix = at(c);
+      if (in_fixed) {
+        const longlong2 y = __ldcg(static_cast<const longlong2*>(in) + ix);
+        x[c] = make_double2(oz::fixed_to_double(y.x, 40 - F), oz::fixed_to_double(y.y, 40 - F));
+      } else {
+        x[c] = __ldcg(static_cast<const double2*>(in) + ix);
+      }
+    }
+    uint32_t gkey = 0;
+#pragma unroll 1
+    for (int o = 0; o < 16; ++o) {
+      const double2 v = group_output_fp64(U16, x, o);
+      gkey = max(gkey, amp_key(v));
+      const IT ix = at(o);
+      out[pp.perm >= 0 ? (IT)chain_image(sm.ptab, (uint32_t)ix) : ix] = v;
+    }
+    okey = max(okey, gkey);
+    if (gkey) ominc = max(ominc, 2047u - oz::key_exponent(gkey));
+  }
+  if (okey) atomicMax(&sm.okey, okey);
+  if (ominc) atomicMax(&sm.ominc, ominc);
+}
+
+// The later passes of a chain in one cooperative launch: `npass` passes over the state with
+// a grid-wide barrier between them. Bound: per pass the state is read and written once
+// (32 B per amplitude); on small states the pass's fixed cost is all there is, so what can
+// be done once is done once (tensor memory, barriers) or ahead (operators built by
+// chain_prep_kernel, the next pass's digits copied during this one). Measured, microseconds
+// per pass, against a launch per pass (gate_pair_chain_kernel, whose CTAs each build the
+// operator): 5.6 against 10.5 at 2^12 amplitudes (of which the barrier about 1.8, one tile's
+// chain of load, digits, MMAs and recombination 3.4), 11.0 against 16.1 at 2^20.
+//
+// The input of pass k is what the previous pass wrote: doubles with the largest group key
+// of all of them, or 64-bit fixed point at scale F with the largest |hi word| (pass 0:
+// *rin). Both are cut into digits at one scale for the whole state -- no per-group exponent
+// exchange, and for fixed point no per-element exponent alignment (oz::digits_fixed). The
+// output is fixed point at scale F = 2100 - E - max erow (want_fixed) or doubles; the last
+// pass's is recorded in *rout. When the input is doubles whose largest magnitude lies
+// outside 2^-200..2^201 or the gate has entries the digits cannot carry (then gate_ok is 0),
+// every group is computed in FP64 (from the converted fixed-point input where that is the
+// input) and doubles are written.
+//
+// Pipeline (one CTA per SM): group r of a tile belongs to four threads (warps q, q + 4,
+// q + 8, q + 12 of the lane quarter q = r / 32), each owning 4 of its 16 amplitudes. The
+// CTA's tiles are numbered through all passes (t): in iteration t the team writes the digits
+// of tile t into digit buffer t % 2 and arrives on full[t % 2]; then it waits for the MMAs
+// of tile t - 1 (accumulator set (t - 1) % 2) and recombines and stores that tile; the last
+// tile of a pass is recombined before the barrier. The MMA warp issues tile t's MMAs into
+// accumulator set t % 2 as soon as its digits are complete, so the tensor cores work on
+// tile t while the team recombines tile t - 1: the team never waits for its own MMAs unless
+// they take longer than a digit phase. Buffer reuse: digits of tile t overwrite buffer
+// t % 2 after the team waited for the MMAs of tile t - 2 that read it; the MMAs of tile t
+// overwrite set t % 2 after every thread arrived on full for tile t, i.e. after its reads
+// of tile t - 2's sums (tcgen05.fence before the arrive).
+//
+// Between passes: every thread's stores, a CTA barrier, then one thread adds the CTA to the
+// pass's barrier word and waits until all are counted. The word has eight counters of 8
+// bits, one per class of the range of a CTA's outputs (bit length of the largest |hi word|,
+// from three bits below the input's on), so the next pass's scale comes with the barrier
+// in the same load; in the first and last class, which are open ended, the exact value is
+// read from memory. Everything else the next pass needs -- addresses, tables, gate digits --
+// is prepared while the barrier completes. The waits are bounded; on expiry the CTA stops,
+// and the others' waits expire too. State loads are cp.async.cg and the FP64 form's and the
+// records' __ldcg, so nothing of an earlier pass is read from L1.
+//
+// A pass with perm >= 0 (states of at most 2^32 elements) writes out of place to the other
+// buffer, element x to index P(x) (bit tables in shared memory; P(tile part | row part |
+// offset) is the OR of the three parts' images), so the pass and the permutation after it
+// take one pass over the state.
+template <typename IT, int NL>
+__global__ void __launch_bounds__(CH_THREADS, 1) gate_chain_resident_kernel(void* buf0, void* buf1,
+                                                                        const ChainGate* __restrict__ gates,
+                                                                        const uint32_t* __restrict__ ptabs,
+                                                                        const ChainRec* rin, ChainRec* rmid,
+                                                                        ChainRec* rout, uint64_t* words,
+                                                                        uint64_t ngroups, int npass,
+                                                                        const __grid_constant__ ChainPasses ps) {
+  CrSmem& sm = *reinterpret_cast<CrSmem*>(resident_smem);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t mine = ((uint32_t)(ngroups / UM_M) - blockIdx.x + gridDim.x - 1) / gridDim.x;  // tiles per pass, >= 1
+  const int q = warp & 3, h = warp >> 2;  // lane quarter; this thread's amplitudes 4h .. 4h + 3
+  const int r = q * 32 + lane;            // group row of the tile (TMEM lane)
+
+  if (tid == 0) {
+    sm.abort = 0;
+    sm.no_abort = 0;
+    sm.okey = sm.ominc = sm.ohi = 0;
+    sm.mine = mine;
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&sm.full[b], CH_TEAM);
+      mbar_init(&sm.done[b], 1);
+      mbar_init(&sm.gate[b], 1);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == CH_WARPS) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem_base)),
+                 "r"(CH_TMEM_COLS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = sm.tmem_base;
+  auto load_gate_digits = [&](int k) {  // (one thread of the MMA warp)
+    mbar_arrive_expect_tx(&sm.gate[k & 1], (uint32_t)sizeof(ChainDigits));
+    bulk_g2s(&sm.gd[k & 1], &gates[k].d, (uint32_t)sizeof(ChainDigits), &sm.gate[k & 1]);
+  };
+  if (warp == CH_WARPS && lane == 0) {
+    load_gate_digits(0);
+    if (npass > 1) load_gate_digits(1);
+  }
+
+  // what pass k needs besides its input's range: this thread's row and first tile (rbase, tb),
+  // the address steps, the permutation's tables, the gate digits
+  IT rbase, tb, s0, s1, tb1;
+  auto prepare = [&](int k, void* in, void* other, uint32_t t0) {
+    const ChainPassP& pp = ps.p[k];
+    rbase = chain_row<IT>(pp, h, r);
+    tb = chain_base<IT>((IT)((uint64_t)blockIdx.x * UM_M), pp);
+    tb1 = chain_next_tile(tb, (IT)pp.step, chain_holes<IT>(pp));
+    s0 = (IT)pp.tgt[2], s1 = (IT)pp.tgt[3];
+    const bool po = pp.perm >= 0;
+    const uint32_t* src = ptabs + (size_t)(po ? pp.perm : 0) * 1024;
+    if (po) {
+      for (int t = tid; t < 1024; t += CH_THREADS) (&sm.ptab[0][0])[t] = __ldg(src + t);
+    }
+    if (tid == CH_TEAM) {
+      auto image = [&](uint32_t x) -> IT {
+        return (IT)(__ldg(src + (x & 255u)) | __ldg(src + 256 + ((x >> 8) & 255u)) | __ldg(src + 512 + ((x >> 16) & 255u)) |
+                    __ldg(src + 768 + (x >> 24)));
+      };
+      sm.in = in, sm.out = po ? other : in, sm.t0 = t0;
+      IT* ad = reinterpret_cast<IT*>(sm.addr);
+      ad[0] = s0, ad[1] = s1, ad[2] = (IT)pp.step, ad[3] = chain_holes<IT>(pp);
+      ad[4] = po ? image((uint32_t)s0) : s0;
+      ad[5] = po ? image((uint32_t)s1) : s1;
+    }
+    if (!mbar_wait_warp(&sm.gate[k & 1], (uint32_t)((k >> 1) & 1), &sm.no_abort)) {
+      atomicOr(&g_umma_error, 1u);
+      sm.abort = 1;
+    }
+  };
+
+  void* in = buf0;
+  void* other = buf1;
+  // what the input is (the same in every CTA)
+  ChainRec ri;
+  ri.fmt = __ldcg(&rin->fmt), ri.F = __ldcg(&rin->F), ri.maxhi = __ldcg(&rin->maxhi);
+  ri.maxkey = __ldcg(&rin->maxkey), ri.minc = __ldcg(&rin->minc);
+  uint32_t t0 = 0;  // this CTA's tiles of the earlier passes that ran on the tensor cores
+  int k = 0;
+  prepare(0, in, other, t0);
+  __syncthreads();
+  for (; k < npass && sm.abort == 0; ++k) {
+    // the first two tiles are on their way before anything else
+    if (warp < CH_WARPS) {
+      chain_fetch<IT>(sm, in, true, tb | rbase, s0, s1, t0 & 1u, h, r);
+      chain_fetch<IT>(sm, in, 1 < mine, tb1 | rbase, s0, s1, (t0 + 1) & 1u, h, r);
+    }
+    const bool po = ps.p[k].perm >= 0;
+    void* out = po ? other : in;
+    const ChainDigits& gd = sm.gd[k & 1];
+
+    // ---- the scales ----
+    const bool common = gd.common != 0, in_fixed = ri.fmt == 1;
+    int32_t sh = 0;
+    int Ein;
+    bool in_ok = true;
+    if (in_fixed) {
+      sh = oz::fixed_shift(ri.maxhi);
+      Ein = oz::fixed_exponent(sh, ri.F);
+      if (sh > 15) in_ok = false;  // (not reached: outputs stay below 2^62, sh <= 15)
+    } else {
+      // doubles: one scale for the whole state, if its largest magnitude is in the digit range
+      // and (when recorded) no nonzero half group lies more than 2^CHAIN_RANGE below it
+      const uint32_t E = oz::key_exponent(ri.maxkey);
+      in_ok = tc_scale_ok(E) && (ri.minc == 0 || (int)E - (2047 - (int)ri.minc) <= CHAIN_RANGE);
+      Ein = (int)oz::digit_scale(E);
+    }
+    const int hi_len = in_fixed ? 32 - __clz((int)ri.maxhi) : 24;  // (the barrier's classes count from it)
+    const bool uni = in_ok && gd.gate_ok != 0;
+    const bool out_fixed = uni && ps.p[k].want_fixed != 0;
+    const int32_t F_in = ri.F;
+    ri.fmt = out_fixed ? 1 : 0;  // (now describing the output)
+    ri.F = 2100 - Ein - gd.max_erow;
+
+    if (warp == CH_WARPS) {
+      // ---- MMA warp: one elected thread issues each tile's 12 MMAs into set t % 2 ----
+      const uint32_t bbase = smem_u32(&gd.bdig[0][0][0]);
+      uint32_t issued = 0;
+      for (uint32_t m = 0; uni && m < mine; ++m) {
+        const uint32_t t = t0 + m, b = t & 1u;
+        if (!mbar_wait_warp(&sm.full[b], (t >> 1) & 1u, &sm.abort)) {
+          atomicOr(&g_umma_error, 1u);
+          sm.abort = 1;
+          break;
+        }
+        tc_fence_after();
+        if (lane == 0) {
+          const uint32_t abase = smem_u32(&sm.adig[b][0][0][0]);
+          // state digit j x gate digits 0 .. NL - 1 - j (stacked along N) -> levels j .. NL - 1;
+          // the first MMA (j = 0, all levels) overwrites, the rest accumulate
+#pragma unroll
+          for (int j = 0; j < CH_ND; ++j) {
+#pragma unroll
+            for (int ks = 0; ks < 2; ++ks) {
+              const uint64_t ad = smem_desc(abase + (uint32_t)((j * 2 + ks) * UM_M * 32));
+              const uint64_t bd = smem_desc(bbase + (uint32_t)(ks * CH_NLMAX * UM_N * 32));
+              umma_f16(tmem + b * CH_ACC + (uint32_t)(j * UM_N), ad, bd, ch_idesc((uint32_t)(UM_N * (NL - j))),
+                       (j | ks) != 0 ? 1u : 0u);
+            }
+          }
+          umma_commit(&sm.done[b]);
+        }
+        __syncwarp();
+        issued = m + 1;
+      }
+      // the team may have stopped early: let the last issued MMAs finish before tensor memory
+      // is freed (no commit on that barrier follows, so its phase parity is stable)
+      if (issued) {
+        const uint32_t t = t0 + issued - 1;
+        mbar_wait_warp(&sm.done[t & 1u], (t >> 1) & 1u, &sm.no_abort);
+      }
+    } else if (uni) {
+      const bool fast = in_fixed && out_fixed && common && sh >= 1;
+      const uint32_t sc = chain_scale((in_fixed ? CH_IN_FIXED : 0u) | (out_fixed ? CH_OUT_FIXED : 0u) |
+                                          (common ? CH_COMMON : 0u) | ((k & 1) ? CH_ODD : 0u),
+                                      sh, Ein);
+      bool ok;
+      if (sizeof(IT) == 4 && po)
+        ok = fast ? chain_team_pass<IT, NL, true, sizeof(IT) == 4>(rbase, tb, sc)
+                  : chain_team_pass<IT, NL, false, sizeof(IT) == 4>(rbase, tb, sc);
+      else
+        ok = fast ? chain_team_pass<IT, NL, true, false>(rbase, tb, sc)
+                  : chain_team_pass<IT, NL, false, false>(rbase, tb, sc);
+      if (!ok) {
+        atomicOr(&g_umma_error, 2u);
+        sm.abort = 1;
+      }
+    } else {
+      cp_async_wait_all();
+    }
+    if (!uni)
+      chain_pass_fp64<IT>(sm, ps.p[k], in, static_cast<double2*>(out), gates[k].U16, ngroups, in_fixed ? 1 : 0, F_in);
+    else
+      t0 += mine;
+    if (po) other = in, in = out;
+
+    // ---- end of the pass: the record, and (before another pass) the grid barrier ----
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const bool more = k + 1 < npass;
+    if ((!out_fixed || !more) && tid == 0) {  // doubles, or the launch's last pass: through the record in memory
+      ChainRec* rec = more ? &rmid[k] : rout;
+      if (sm.okey) atomicMax(&rec->maxkey, sm.okey);
+      if (sm.ominc) atomicMax(&rec->minc, sm.ominc);
+      if (sm.ohi) atomicOr(&rec->maxhi, sm.ohi);
+      if (!more && blockIdx.x == 0) rec->fmt = ri.fmt, rec->F = ri.F;
+    }
+    if (!more) break;
+    if (tid == 0 && sm.abort == 0) {
+      if (out_fixed && sm.ohi) red_or_relaxed(&rmid[k].maxhi, sm.ohi);
+      // class of this CTA's range against the input's
+      const int cls = min(7, max(0, 3 + (32 - __clz((int)sm.ohi)) - hi_len));
+      red_add_release(&words[16 * k], 1ull << (8 * cls));  // (with the barrier above: all of the CTA's stores)
+      sm.okey = sm.ominc = sm.ohi = 0;
+    }
+    if (warp == CH_WARPS && lane == 0 && k + 2 < npass) load_gate_digits(k + 2);
+    prepare(k + 1, in, other, t0);
+    if (tid == 0) {
+      const long long c0 = clock64();
+      uint64_t w = 0;
+      bool all = false;
+      while (sm.abort == 0 && !all) {
+        w = ld_acquire(&words[16 * k]);
+        // the sum of the eight counts (at most 255 CTAs)
+        const uint64_t pairs = (w & 0x00FF00FF00FF00FFull) + ((w >> 8) & 0x00FF00FF00FF00FFull);
+        all = (uint32_t)((pairs * 0x0001000100010001ull) >> 48) == gridDim.x;
+        if (!all && clock64() - c0 > UM_WAIT_CYCLES) {
+          atomicOr(&g_umma_error, 2u);
+          sm.abort = 1;
+        }
+      }
+      const int top = (63 - __clzll((long long)(w | 1ull))) >> 3;  // the highest class that was counted
+      const int len = hi_len + top - 3;
+      sm.all_hi = (top == 0 || top == 7) ? __ldcg(&rmid[k].maxhi) : (uint32_t)((1ull << len) - 1);
+    }
+    __syncthreads();
+    ri.maxhi = sm.all_hi;
+    if (!out_fixed) ri.maxkey = __ldcg(&rmid[k].maxkey), ri.minc = __ldcg(&rmid[k].minc);
+  }
+  // stopped early (k: the first pass not run): the digits of its next pass may be on their way
+  if (k < npass && sm.abort != 0 && k + 1 < npass && warp == CH_WARPS)
+    mbar_wait_warp(&sm.gate[(k + 1) & 1], (uint32_t)(((k + 1) >> 1) & 1), &sm.no_abort);
+
+  // ---- teardown: all tensor-memory reads are done; free it ----
+  tc_fence_before();
+  __syncthreads();
+  if (warp == CH_WARPS) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(CH_TMEM_COLS) : "memory");
+  }
+}
+
 template <typename IT, uint32_t MODE>
 void launch_umma(double2* psi, const double2* ga, const double2* gb, const PairParams& p, cudaStream_t s,
                  ChainRec* rec = nullptr) {
@@ -912,7 +1598,81 @@ void launch_pair_chain(void* psi, const double2* ga, const double2* gb, const Pa
   }
 }
 
-bool make_bit_perm(const dims_t& dims, const std::vector<uint16_t>& ptup, const PairParams& p, BitPerm& bp) {
+// The bits of x moved to the positions outside the holes (ascending).
+static uint64_t spread_bits(uint64_t x, const uint32_t (&ins)[4]) {
+  for (int j = 0; j < 4; ++j) {
+    const uint64_t low = x & ((1ull << ins[j]) - 1);
+    x = ((x >> ins[j]) << (ins[j] + 1)) | low;
+  }
+  return x;
+}
+
+void launch_chain_resident(void* cur, void* oth, const std::vector<ChainStep>& steps, uint64_t ngroups,
+                         const ChainRec* rin, ChainRec* rout, cudaStream_t s) {
+  const int npass = (int)steps.size();
+  if (npass < 1 || npass > CR_MAXP) throw Error(QTNH_ERR_RUNTIME, "chain launch length");
+  // one CTA per SM (all its TMEM); the barrier counts at most 255
+  const int grid = (int)std::min<uint64_t>(ngroups / UM_M, (uint64_t)std::min(sm_count(), 255));
+  ChainPrepParams q;
+  ChainPasses ps;
+  int nperm = 0;
+  for (int k = 0; k < npass; ++k) {
+    const ChainStep& st = steps[(size_t)k];
+    q.ga[k] = st.ga;
+    q.gb[k] = st.gb;
+    q.mode[k] = PAIR_KRON;
+    ChainPassP& pp = ps.p[k];
+    for (int j = 0; j < 4; ++j) {
+      pp.ins[j] = (uint8_t)st.p.ins_pos[j];
+      pp.tgt[j] = (uint64_t)st.p.off[8 >> j];
+    }
+    pp.step = spread_bits((uint64_t)grid * UM_M, st.p.ins_pos);
+    pp.want_fixed = st.want_fixed ? 1 : 0;
+    pp.perm = -1;
+    if (st.perm) {
+      if (!oth || oth == cur) throw Error(QTNH_ERR_UNSUPPORTED, "permuted chain output");
+      std::memcpy(q.dst[nperm], st.dst, sizeof(st.dst));
+      pp.perm = (int16_t)nperm++;
+    }
+  }
+  // workspace: the barrier's words and the records between the passes, zeroed; the
+  // operators; the permutation tables
+  const size_t words_bytes = (size_t)npass * 128;  // a line each
+  const size_t zero_bytes = words_bytes + (size_t)npass * sizeof(ChainRec);
+  const size_t gate_off = (zero_bytes + 255) / 256 * 256, gate_bytes = (size_t)npass * sizeof(ChainGate);
+  uint8_t* ws = static_cast<uint8_t*>(workspace_alloc(gate_off + gate_bytes + (size_t)nperm * 4096, s));
+  uint64_t* words = reinterpret_cast<uint64_t*>(ws);
+  ChainRec* rmid = reinterpret_cast<ChainRec*>(ws + words_bytes);
+  ChainGate* gates = reinterpret_cast<ChainGate*>(ws + gate_off);
+  uint32_t* ptabs = reinterpret_cast<uint32_t*>(ws + gate_off + gate_bytes);
+  const int nl = chain_levels();
+  cudaError_t e = cudaMemsetAsync(ws, 0, zero_bytes, s);
+  if (e == cudaSuccess) {
+    chain_prep_kernel<<<npass + nperm, 128, 0, s>>>(q, npass, nl, gates, ptabs);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) {
+    const void* fn = nl == 6 ? (const void*)gate_chain_resident_kernel<uint32_t, 6>
+                             : (const void*)gate_chain_resident_kernel<uint32_t, 7>;
+    const int smem = (int)sizeof(CrSmem);
+    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess) {
+      int np = npass;
+      void* args[] = {&cur, &oth, &gates, &ptabs, &rin, &rmid, &rout, &words, &ngroups, &np, &ps};
+      e = cudaLaunchCooperativeKernel(fn, dim3((unsigned)grid), dim3(CH_THREADS), args, (size_t)smem, s);
+    }
+  }
+  workspace_free(ws, s);
+  check_cuda(e, "gate chain launch");
+}
+
+bool chain_resident(const PairParams& p) { return chain_applies(p) && p.ngroups * 16 <= CHAIN_RESIDENT_AMPS; }
+int chain_resident_passes() { return CR_MAXP; }
+
+// dst[b]: the output bit of index bit b under the permutation ptup (Tensor::permute
+// convention) of a state of dims `dims`, 32 for bits above the state; false if the dims are
+// not all powers of two or the state has more than 2^32 elements.
+bool make_bit_map(const dims_t& dims, const std::vector<uint16_t>& ptup, uint8_t dst[32]) {
   const size_t r = dims.size();
   if (ptup.size() != r) return false;
   uint32_t total = 0;
@@ -932,10 +1692,15 @@ bool make_bit_perm(const dims_t& dims, const std::vector<uint16_t>& ptup, const 
   for (size_t i = r; i-- > 0;) in_lo[i] = acc, acc += w[i];
   acc = 0;
   for (size_t j = r; j-- > 0;) out_lo[j] = acc, acc += log2_or_none(nd[j]);
-  uint32_t dst[32];
   for (int b = 0; b < 32; ++b) dst[b] = 32;  // bits above the state: never set
   for (size_t i = 0; i < r; ++i)
-    for (uint32_t k = 0; k < w[i]; ++k) dst[in_lo[i] + k] = out_lo[ptup[i]] + k;
+    for (uint32_t k = 0; k < w[i]; ++k) dst[in_lo[i] + k] = (uint8_t)(out_lo[ptup[i]] + k);
+  return true;
+}
+
+bool make_bit_perm(const dims_t& dims, const std::vector<uint16_t>& ptup, const PairParams& p, BitPerm& bp) {
+  uint8_t dst[32];
+  if (!make_bit_map(dims, ptup, dst)) return false;
   for (int t = 0; t < 4; ++t)
     for (int v = 0; v < 256; ++v) {
       uint32_t x = 0;

@@ -196,8 +196,12 @@ DF_HD void digit_words_fixed(int64_t x0, int64_t x1, int32_t sh, uint32_t w[NS])
 // positive, left when not), from maxhi, a value with the bit length of the largest |hi
 // word| (fixed_hi_mag): the magnitude bound is taken as 2^(32 + bit length of maxhi).
 DF_HD int32_t fixed_shift(uint32_t maxhi) {
+#ifdef __CUDA_ARCH__
+  const int32_t len = 32 - __clz((int)maxhi);
+#else
   int32_t len = 0;
   while (len < 32 && (maxhi >> len)) ++len;
+#endif
   return 32 + len - 47;
 }
 
