@@ -76,6 +76,38 @@ __global__ void __launch_bounds__(GEMM_THREADS) zgemm_kernel(const c128* __restr
   }
 }
 
+// The same for results whose 64 x 64 tiles would leave SMs idle: a block holds `out` = 2^out_log2
+// consecutive outputs, 256 / out threads each, which take every (256 / out)-th k; their
+// sums are added pairwise through shared memory. Bound: the FP64 unit (one warp's DFMA
+// occupies its sub-partition for 64 cycles), so plain loads through L1 keep up with it
+// whatever the tile, and only the spread over the 152 SMs matters. M 77, N 39, K 45: 196 us
+// (two tiles, two SMs) -> 5.0 us; one output, K 4096: 16.4 ms -> 8.5 us.
+__global__ void __launch_bounds__(256) zgemm_spread_kernel(const c128* __restrict__ A, const c128* __restrict__ B,
+                                                           c128* __restrict__ C, uint64_t M, uint64_t N, uint64_t K,
+                                                           int out_log2) {
+  __shared__ c128 part[256];
+  const int tid = threadIdx.x, out = 1 << out_log2, lanes = 256 >> out_log2;
+  const uint64_t i = ((uint64_t)blockIdx.x << out_log2) + (uint64_t)(tid & (out - 1));
+  const bool live = i < M * N;
+  c128 acc = make_double2(0.0, 0.0);
+  if (live) {
+    const c128* a = A + (i / N) * K;
+    const c128* b = B + i % N;
+#pragma unroll 4
+    for (uint64_t k = (uint64_t)(tid >> out_log2); k < K; k += (uint64_t)lanes)
+      acc = cfma(__ldg(a + k), __ldg(b + k * N), acc);
+  }
+  part[tid] = acc;
+  for (int h = 128; h >= out; h >>= 1) {
+    __syncthreads();
+    if (tid < h) {
+      acc.x += part[tid + h].x, acc.y += part[tid + h].y;
+      part[tid] = acc;
+    }
+  }
+  if (tid < out && live) C[i] = acc;
+}
+
 }  // namespace
 
 // The FP64 GEMM's grid has one block row per 64 rows of C (grid y is at most 65535).
@@ -90,6 +122,25 @@ void zgemm(const c128* A, const c128* B, c128* C, uint64_t M, uint64_t N, uint64
   if (M == 0 || N == 0) return;
   zgemm_check_shape(M, N);
   uint64_t gx = (N + BN - 1) / BN, gy = (M + BM - 1) / BM;
+  // Both kernels run at the FP64 unit's rate where the SMs are evenly loaded, so the tiles are
+  // taken unless they would fill less than 9/10 of the SMs' time: padding (4096 outputs a
+  // tile) and the last wave, against the M N outputs themselves. At K 64, in us, tiles / spread:
+  // 512 x 512 262 / 119, 1024 x 1024 517 / 469, 1500 x 900 770 / 603; 768 x 768 (144 of 152
+  // tiles) 261 / 262 on either, 2048 x 2048 1784 in tiles.
+  const uint64_t sms = (uint64_t)sm_count(), waves = (gx * gy + sms - 1) / sms;
+  if (10 * (M * N) < 9 * (waves * sms * BM * BN)) {
+    // as many outputs a block as leaves every SM one, at most 64 (coalesced loads of B); no more
+    // threads an output than K has terms
+    int out_log2 = 6;
+    while (out_log2 > 0 && (M * N) >> out_log2 < sms && (256ull >> out_log2) < K) --out_log2;
+    const uint64_t blocks = (M * N + (1ull << out_log2) - 1) >> out_log2;
+    if (blocks < (1ull << 31)) {
+      zgemm_spread_kernel<<<(unsigned)blocks, 256, 0, s>>>(A, B, C, M, N, K, out_log2);
+      count_launch();
+      check_cuda(cudaGetLastError(), "zgemm_spread_kernel launch");
+      return;
+    }
+  }
   zgemm_kernel<<<dim3((unsigned)gx, (unsigned)gy), GEMM_THREADS, 0, s>>>(A, B, C, M, N, K);
   count_launch();
   check_cuda(cudaGetLastError(), "zgemm_kernel launch");
