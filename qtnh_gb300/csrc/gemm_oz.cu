@@ -27,18 +27,27 @@
 // The result is therefore accurate to ~2^-48 of the largest product magnitudes of its
 // row and column, independent of K: FP64-level for the 1e-12 relative-L2 bar.
 //
-// Tile: 128 rows of C^ (64 complex rows) x 64 columns, as two halves of 32 columns. Per
-// K-step the stage holds the six A digits (128 rows x 16 bf16 each, 24 KB) and, per half,
-// the six B digits stacked along N (32 rows each, 6 KB), all in the UMMA K-major
-// core-matrix layout (8 rows x 16 bytes; LBO 128 B, SBO 256 B). A digit i meets B digits
-// 0 .. 5 - i of a half in one tcgen05.mma (kind::f16, bf16 in, FP32 out) of N = 32 (6 - i)
-// into the half's level columns i ..: 6 MMAs per half and K-step, 12 per stage, the A
-// digits read once per stage for both halves. Tensor memory: per half 6 levels x 32
-// columns (192), both halves 384 of the SM's 512 columns.
+// Tile: 128 rows of C^ (64 complex rows) x 64 columns. Per K-step the stage holds the six A
+// digits (128 rows x 16 bf16 each, 24 KB) and the six B digits stacked along N (64 rows
+// each, 12 KB), all in the UMMA K-major core-matrix layout (8 rows x 16 bytes; LBO 128 B,
+// SBO 256 B). A digit i meets B digits 0 .. 5 - i, 64 (6 - i) rows, in one tcgen05.mma
+// (kind::f16, bf16 in, FP32 out; two of half the rows where they exceed 256) into the
+// level columns 64 i ..: 8 MMAs per K-step. (Two halves of 32 columns, 12 MMAs, read the A
+// digits twice and took 920 cycles a K-step, which shared memory bounds at 704; this reads
+// 74 KB, 592 cycles against the tensor pipe's 672.) Tensor memory: 6 levels x 64 columns.
 // CTA (persistent, one per SM): warp 0 streams each K-step's 36 KB stage with bulk copies
-// into a 5-stage ring, warp 1's elected thread issues the MMAs and commits, warps 2-9 (two
-// per TMEM lane quarter, one per half) drain the level sums after each chunk and write
+// into a 5-stage ring, warp 1's elected thread issues the MMAs and commits, warps 2-17 (four
+// per TMEM lane quarter, 16 columns each) drain the level sums after each chunk and write
 // the result (or, with split K, the exact partials T and F that a reduction kernel sums).
+// The drain goes from level 5 to level 0 and frees each level by itself, and the next
+// chunk's first two K-steps go A digit 5 first, which touches level 5 only, so the MMAs
+// follow the drain down the levels instead of waiting for all of it. Measured at M 4096,
+// N 2048, K 1024: the whole contraction 1580 us -> 1210 (the GEMM alone 1394 -> ~1020 us,
+// 1.4 PFLOP/s of digit products) against two half tiles, eight drain warps and chunks
+// drained whole. In cycles of a chunk: 9840, of which MMAs 5930, waits for the drain 2180 (it
+// takes 2660) and for stages 1730 (36 KB a K-step from L2). One such K-step instead of two
+// takes 1325 us where two take 1279 and three 1313 (hides less; more in the MMAs); bringing A
+// to L2 ahead of the ring and a sixth stage change nothing.
 // Every wait is bounded by a clock limit; on expiry the CTA records an error flag
 // (qtnh_take_device_errors, bits 16-18), stops and frees its tensor memory.
 //
@@ -59,28 +68,26 @@ __device__ unsigned int g_ozg_error;
 namespace {
 
 constexpr int OG_M = 128;                  // rows of C^ per tile (64 complex rows)
-constexpr int OG_HN = 32;                  // columns of one half tile
-constexpr int OG_H = 2;                    // halves per tile
-constexpr int OG_N = OG_HN * OG_H;         // columns of C per tile
+constexpr int OG_N = 64;                   // columns of C per tile
+constexpr int OG_EN = 16;                  // columns an epilogue thread drains
 constexpr int OG_D = oz::NS;               // digits per real
 constexpr int OG_L = oz::NL;               // levels kept
 constexpr int OG_KSTEP = 16;               // bf16 K per MMA
 constexpr uint32_t OG_CHUNK = 8;           // K-steps whose level sums are exact in FP32
+constexpr uint32_t OG_HEAD = 2;            // first K-steps of a chunk issued digit by digit, behind the drain
 constexpr int OG_A_DIGIT = OG_M * OG_KSTEP * 2;   // 4096 bytes
 constexpr int OG_A_BLOCK = OG_D * OG_A_DIGIT;     // 24576 bytes: six A digits of one K-step
-constexpr int OG_B_DIGIT = OG_HN * OG_KSTEP * 2;  // 1024 bytes
-constexpr int OG_B_HALF = OG_D * OG_B_DIGIT;      // 6144 bytes: six B digits of a half
-constexpr int OG_B_BLOCK = OG_H * OG_B_HALF;      // 12288 bytes
+constexpr int OG_B_DIGIT = OG_N * OG_KSTEP * 2;   // 2048 bytes
+constexpr int OG_B_BLOCK = OG_D * OG_B_DIGIT;     // 12288 bytes: six B digits of one K-step
 constexpr int OG_STAGE = OG_A_BLOCK + OG_B_BLOCK;  // 36864 bytes
 constexpr int OG_STAGES = 5;
-constexpr int OG_THREADS = 320;  // warp 0 producer, warp 1 MMA, warps 2-9 epilogue
-constexpr uint32_t OG_EPI_THREADS = 256;
+constexpr int OG_THREADS = 576;  // warp 0 producer, warp 1 MMA, warps 2-17 epilogue
+constexpr uint32_t OG_EPI_WARPS = 16;
 constexpr uint32_t OG_TMEM_COLS = 512;
-constexpr uint32_t OG_HCOLS = OG_L * OG_HN;  // 192 columns per half
 constexpr long long OG_WAIT_CYCLES = 1ll << 32;  // ~2 s at 2 GHz
 constexpr uint32_t OG_SPECIAL = 0x7FFu;          // largest exponent of a row with an inf/NaN
-static_assert(OG_H * OG_HCOLS <= OG_TMEM_COLS, "level sums exceed tensor memory");
-static_assert(OG_HN * OG_L <= 256, "an MMA's N is at most 256");
+static_assert(OG_L * OG_N <= OG_TMEM_COLS, "level sums exceed tensor memory");
+static_assert(OG_N * OG_L <= 2 * 256, "an MMA's N is at most 256");
 
 struct OzParams {
   const uint8_t* a_planes;  // MT x KS blocks of OG_A_BLOCK bytes
@@ -100,7 +107,7 @@ struct OgSmem {
   uint64_t full[OG_STAGES];
   uint64_t empty[OG_STAGES];
   uint64_t tfull;   // a chunk's level sums are complete
-  uint64_t tempty;  // the epilogue has drained them
+  uint64_t tempty[OG_L];  // the epilogue has drained a level
   uint32_t tmem_base;
   int abort;
 };
@@ -175,11 +182,29 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
                : "memory");
 }
 
-// 8 consecutive 32-bit TMEM columns of this thread's lane.
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-               : "r"(taddr));
+// A digit i of a stage (sd: the descriptor of its first byte) x its B digits j0 .. j1 - 1
+// (stacked) -> levels i + j0 .. i + j1 - 1. One thread issues all: the descriptors are sums
+// of constants and the stage's.
+__device__ __forceinline__ void issue_digit(uint32_t tmem, uint64_t sd, int i, int j0, int j1, uint32_t acc) {
+  const int rows = OG_N * (j1 - j0), parts = rows > 256 ? 2 : 1, n = rows / parts;
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    if (q * n < rows && n > 0) {
+      const int r0 = j0 * OG_N + q * n;  // first stacked B row
+      umma_bf16(tmem + (uint32_t)(i * OG_N + r0), sd + (uint64_t)(i * (OG_A_DIGIT >> 4)),
+                sd + (uint64_t)((OG_A_BLOCK + r0 * OG_KSTEP * 2) >> 4), og_idesc((uint32_t)n), acc);
+    }
+  }
+}
+
+// 16 consecutive 32-bit TMEM columns of this thread's lane.
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[OG_EN]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, "
+      "[%16];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(taddr));
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
@@ -205,7 +230,7 @@ __global__ void __launch_bounds__(OG_THREADS, 1) gemm_oz6_umma_kernel(const __gr
       mbar_init(&sm.empty[s], 1);
     }
     mbar_init(&sm.tfull, 1);
-    mbar_init(&sm.tempty, OG_EPI_THREADS);
+    for (int l = 0; l < OG_L; ++l) mbar_init(&sm.tempty[l], OG_EPI_WARPS);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -246,63 +271,77 @@ __global__ void __launch_bounds__(OG_THREADS, 1) gemm_oz6_umma_kernel(const __gr
   } else if (warp == 1) {
     // ---- MMA: one elected thread; a chunk of up to OG_CHUNK K-steps per accumulation ----
     if (lane == 0) {
-      uint32_t it = 0, ch = 0;
+      uint32_t st = 0, ph = 0, ch = 0;
       bool ok = true;
+      const uint64_t sdesc = smem_desc(smem_u32(&sm.stage[0][0]));
       for (uint64_t tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x) {
         uint64_t mt, nt;
         uint32_t k0, k1;
         tile_coords(tile, mt, nt, k0, k1);
         for (uint32_t c0 = k0; ok && c0 < k1; c0 += OG_CHUNK, ++ch) {
           const uint32_t c1 = min(k1, c0 + OG_CHUNK);
-          if (!mbar_wait_thread(&sm.tempty, (ch & 1u) ^ 1u, &sm.abort)) {
+          // the first K-steps: A digit 5 of all of them, then digit 4, ..: digit i needs levels
+          // i .. 5 of the last chunk drained; on the first K-step it is the first to write level i
+          const uint32_t g = min(c1 - c0, OG_HEAD);
+          uint64_t sd[OG_HEAD];
+          uint64_t* eb[OG_HEAD];
+#pragma unroll
+          for (uint32_t x = 0; x < OG_HEAD; ++x) {
+            sd[x] = sdesc + (uint64_t)(st * (OG_STAGE >> 4));
+            eb[x] = &sm.empty[st];
+            if (x < g) {
+              ok = ok && mbar_wait_thread(&sm.full[st], ph, &sm.abort);
+              if (++st == OG_STAGES) st = 0, ph ^= 1u;
+            }
+          }
+#pragma unroll
+          for (int i = OG_D - 1; i >= 0; --i) {
+            ok = ok && mbar_wait_thread(&sm.tempty[i], (ch & 1u) ^ 1u, &sm.abort);
+            if (!ok) break;
+            tc_fence_after();
+            issue_digit(tmem, sd[0], i, 0, 1, 0u);
+            issue_digit(tmem, sd[0], i, 1, OG_L - i, 1u);
+            if (i == 0) umma_commit(eb[0]);  // the stage is free once its MMAs have read it
+#pragma unroll
+            for (uint32_t x = 1; x < OG_HEAD; ++x) {
+              if (x >= g) break;
+              issue_digit(tmem, sd[x], i, 0, OG_L - i, 1u);
+              if (i == 0) umma_commit(eb[x]);
+            }
+          }
+          for (uint32_t ks = c0 + g; ok && ks < c1; ++ks) {
+            ok = mbar_wait_thread(&sm.full[st], ph, &sm.abort);
+            if (!ok) break;
+            tc_fence_after();
+            const uint64_t d = sdesc + (uint64_t)(st * (OG_STAGE >> 4));
+#pragma unroll
+            for (int i = 0; i < OG_D; ++i) issue_digit(tmem, d, i, 0, OG_L - i, 1u);
+            umma_commit(&sm.empty[st]);
+            if (++st == OG_STAGES) st = 0, ph ^= 1u;
+          }
+          if (!ok) {
             atomicOr(&g_ozg_error, 2u);
             sm.abort = 1;
-            ok = false;
             break;
           }
-          tc_fence_after();
-          for (uint32_t ks = c0; ks < c1; ++ks, ++it) {
-            const uint32_t s = it % OG_STAGES, ph = (it / OG_STAGES) & 1u;
-            if (!mbar_wait_thread(&sm.full[s], ph, &sm.abort)) {
-              atomicOr(&g_ozg_error, 2u);
-              sm.abort = 1;
-              ok = false;
-              break;
-            }
-            tc_fence_after();
-            const uint32_t abase = smem_u32(&sm.stage[s][0]);
-#pragma unroll
-            for (int h = 0; h < OG_H; ++h) {
-              const uint64_t bd = smem_desc(abase + (uint32_t)(OG_A_BLOCK + h * OG_B_HALF));
-#pragma unroll
-              for (int i = 0; i < OG_D; ++i) {
-                // A digit i x B digits 0 .. 5 - i (stacked) -> levels i .. 5 of half h; the first
-                // MMA of a chunk (i = 0, all six levels) overwrites, the rest accumulate
-                const uint64_t ad = smem_desc(abase + (uint32_t)(i * OG_A_DIGIT));
-                umma_bf16(tmem + (uint32_t)(h * OG_HCOLS + i * OG_HN), ad, bd, og_idesc((uint32_t)(OG_HN * (OG_L - i))),
-                          (ks > c0 || i > 0) ? 1u : 0u);
-              }
-            }
-            umma_commit(&sm.empty[s]);  // the stage is free once these MMAs have read it
-          }
-          if (ok) umma_commit(&sm.tfull);
+          umma_commit(&sm.tfull);
         }
       }
     }
   } else {
-    // ---- epilogue: warp w drains TMEM lanes 32 (w % 4) .. +31 of half (w - 2) / 4 ----
+    // ---- epilogue: warp w drains TMEM lanes 32 (w % 4) .. +31, columns 16 ((w - 2) / 4) .. +15 ----
     const int q = warp & 3, h = (warp - 2) >> 2, r = q * 32 + lane;
-    const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(h * OG_HCOLS);
+    const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(h * OG_EN);
     uint32_t ch = 0;
     bool ok = true;
     for (uint64_t tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x) {
       uint64_t mt, nt;
       uint32_t k0, k1;
       tile_coords(tile, mt, nt, k0, k1);
-      long long T[OG_HN];
-      float F[OG_HN];
+      long long T[OG_EN];
+      float F[OG_EN];
 #pragma unroll
-      for (int c = 0; c < OG_HN; ++c) T[c] = 0, F[c] = 0.0f;
+      for (int c = 0; c < OG_EN; ++c) T[c] = 0, F[c] = 0.0f;
       for (uint32_t c0 = k0; c0 < k1; c0 += OG_CHUNK, ++ch) {
         if (!mbar_wait_warp(&sm.tfull, ch & 1u, &sm.abort)) {
           atomicOr(&g_ozg_error, 4u);
@@ -311,52 +350,70 @@ __global__ void __launch_bounds__(OG_THREADS, 1) gemm_oz6_umma_kernel(const __gr
           break;
         }
         tc_fence_after();
+        // level 5 first: the next chunk's MMAs on a level start when all warps have read it
+        uint32_t va[OG_EN], vb[OG_EN];
+        auto freed = [&](int l) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sm.tempty[l]);
+        };
+        auto add = [&](const uint32_t(&v)[OG_EN], int shift) {
 #pragma unroll
-        for (int g = 0; g < OG_HN / 8; ++g) {
-          uint32_t v[OG_L][8];
+          for (int c = 0; c < OG_EN; ++c) oz::gemm_add_high(__uint_as_float(v[c]), shift, T[c]);
+        };
+        tmem_ld16(tbase + 5 * OG_N, va);
+        tmem_wait_ld();
+        freed(5);
+        tmem_ld16(tbase + 4 * OG_N, vb);
+        tmem_wait_ld();
+        freed(4);
 #pragma unroll
-          for (int l = 0; l < OG_L; ++l) tmem_ld8(tbase + (uint32_t)(l * OG_HN + 8 * g), v[l]);
-          tmem_wait_ld();
-#pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            // the level sums are exact integers of at most 2^24 in magnitude
-            float lv[OG_L];
-#pragma unroll
-            for (int l = 0; l < OG_L; ++l) lv[l] = __uint_as_float(v[l][c]);
-            oz::gemm_accumulate(lv, T[8 * g + c], F[8 * g + c]);
-          }
-        }
-        tc_fence_before();
-        mbar_arrive(&sm.tempty);
+        for (int c = 0; c < OG_EN; ++c) oz::gemm_add_low(__uint_as_float(vb[c]), __uint_as_float(va[c]), F[c]);
+        tmem_ld16(tbase + 3 * OG_N, va);
+        tmem_wait_ld();
+        freed(3);
+        tmem_ld16(tbase + 2 * OG_N, vb);
+        add(va, 0);
+        tmem_wait_ld();
+        freed(2);
+        tmem_ld16(tbase + 1 * OG_N, va);
+        add(vb, 8);
+        tmem_wait_ld();
+        freed(1);
+        tmem_ld16(tbase, vb);
+        add(va, 16);
+        tmem_wait_ld();
+        freed(0);
+        add(vb, 24);
       }
       if (!ok) break;
       const uint64_t R = mt * OG_M + (uint64_t)r;  // row of C^: complex row R / 2, part R % 2
-      const uint64_t n0 = nt * OG_N + (uint64_t)(h * OG_HN);
+      const uint64_t n0 = nt * OG_N + (uint64_t)(h * OG_EN);
       if (p.S > 1) {
         const uint64_t ld = (uint64_t)p.NT * OG_N;
         const uint64_t base = ((uint64_t)(k0 / p.SK) * p.MT * OG_M + R) * ld + n0;
 #pragma unroll
-        for (int c = 0; c < OG_HN; c += 2) {
+        for (int c = 0; c < OG_EN; c += 2) {
           *reinterpret_cast<longlong2*>(p.tpart + base + c) = make_longlong2(T[c], T[c + 1]);
         }
 #pragma unroll
-        for (int c = 0; c < OG_HN; c += 4) {
+        for (int c = 0; c < OG_EN; c += 4) {
           *reinterpret_cast<float4*>(p.fpart + base + c) = make_float4(F[c], F[c + 1], F[c + 2], F[c + 3]);
         }
         continue;
       }
-      // one slice: the even lane (Re row) writes columns 0..15 of the half, the odd lane
-      // (Im row) columns 16..31; each receives the other part from its partner
+      // one slice: the even lane (Re row) writes the thread's first 8 columns, the odd lane (Im
+      // row) the other 8; each receives the other part from its partner
       const uint64_t m = R >> 1;
       const bool odd = (lane & 1) != 0;
       const uint32_t ea = m < p.M ? p.ea[m] : 0u;
 #pragma unroll
-      for (int x = 0; x < OG_HN / 2; ++x) {
-        // columns x (kept by the even lane) and 16 + x (kept by the odd lane)
-        const uint64_t nlo = n0 + (uint64_t)x, nhi = nlo + OG_HN / 2;
+      for (int x = 0; x < OG_EN / 2; ++x) {
+        // columns x (kept by the even lane) and 8 + x (kept by the odd lane)
+        const uint64_t nlo = n0 + (uint64_t)x, nhi = nlo + OG_EN / 2;
         const uint32_t eblo = nlo < p.N ? p.eb[nlo] : 0u, ebhi = nhi < p.N ? p.eb[nhi] : 0u;
         const double vlo = oz::gemm_finish(T[x], F[x], oz::gemm_scale(ea, eblo));
-        const double vhi = oz::gemm_finish(T[OG_HN / 2 + x], F[OG_HN / 2 + x], oz::gemm_scale(ea, ebhi));
+        const double vhi = oz::gemm_finish(T[OG_EN / 2 + x], F[OG_EN / 2 + x], oz::gemm_scale(ea, ebhi));
         const double keep = odd ? vhi : vlo;
         const double recv = __shfl_xor_sync(0xffffffffu, odd ? vlo : vhi, 1);
         const uint64_t nk = odd ? nhi : nlo;
@@ -398,11 +455,10 @@ __device__ __forceinline__ uint64_t og_a_offset(uint64_t row, uint64_t kc, int i
   const uint64_t mt = row >> 7, rr = row & 127;
   return ((mt * KS + (kc >> 1)) * OG_D + (uint64_t)i) * OG_A_DIGIT + ((rr >> 3) << 8) + ((kc & 1) << 7) + ((rr & 7) << 4);
 }
-// The same for B: column n (tile n / 64, half (n % 64) / 32, row n % 32 of the half).
+// The same for B: column n (tile n / 64, row n % 64).
 __device__ __forceinline__ uint64_t og_b_offset(uint64_t n, uint64_t kc, int j, uint32_t KS) {
-  const uint64_t nt = n >> 6, h = (n >> 5) & 1, rr = n & 31;
-  return (((nt * KS + (kc >> 1)) * OG_H + h) * OG_D + (uint64_t)j) * OG_B_DIGIT + ((rr >> 3) << 8) + ((kc & 1) << 7) +
-         ((rr & 7) << 4);
+  const uint64_t nt = n >> 6, rr = n & 63;
+  return ((nt * KS + (kc >> 1)) * OG_D + (uint64_t)j) * OG_B_DIGIT + ((rr >> 3) << 8) + ((kc & 1) << 7) + ((rr & 7) << 4);
 }
 
 __device__ __forceinline__ uint32_t bf16_pair(float lo, float hi) { return oz::pack(lo, hi); }

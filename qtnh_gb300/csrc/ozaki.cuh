@@ -289,12 +289,16 @@ DF_HD double fixed_to_double(int64_t T, int e) {
 // F += S_4 + 2^-8 S_5 (FP32, below 2^-32 of T's units), and C^ = 2^(ea + eb - 2084) (T +
 // 2^-8 F).
 
-// Adds one chunk's six level sums (exact integers held in floats) to (T, F).
+// Adds one chunk's sum of a level 0..3 (shift 24 - 8 level; an exact integer held in a float).
+DF_HD void gemm_add_high(float v, int shift, long long& T) {
+  T += (long long)((uint64_t)(long long)(int)v << shift);
+}
+// Adds one chunk's sums of levels 4 and 5.
+DF_HD void gemm_add_low(float l4, float l5, float& F) { F = df::add(F, df::fma(l5, 0.00390625f, l4)); }
+// Adds one chunk's six level sums to (T, F).
 DF_HD void gemm_accumulate(const float lv[NL], long long& T, float& F) {
-  const long long s0 = (long long)(int)lv[0], s1 = (long long)(int)lv[1];
-  const long long s2 = (long long)(int)lv[2], s3 = (long long)(int)lv[3];
-  T += (s0 << 24) + (s1 << 16) + (s2 << 8) + s3;
-  F = df::add(F, df::fma(lv[5], 0.00390625f, lv[4]));
+  for (int l = 0; l < 4; ++l) gemm_add_high(lv[l], 24 - 8 * l, T);
+  gemm_add_low(lv[4], lv[5], F);
 }
 
 // Exponent e of C^'s scale 2^e for row exponent ea and column exponent eb.
