@@ -125,13 +125,13 @@ DF_HD dwords words(double x) {
 
 // In range: zero, or biased exponent in [1023 - 90, 1023 + 90] (|x| in [2^-90, 2^91)).
 DF_HD bool in_range_state(dwords w) {
-  uint32_t e = (w.hi >> 20) & 0x7FFu;
-  return (e - 933u) <= 180u || ((w.hi << 1) | w.lo) == 0u;
+  const uint32_t u = w.hi << 1;  // exponent at bits 21-31
+  return u - (933u << 21) < (181u << 21) || (u | w.lo) == 0u;
 }
 // Gate elements: zero or |x| in [2^-30, 2^31).
 DF_HD bool in_range_gate(dwords w) {
-  uint32_t e = (w.hi >> 20) & 0x7FFu;
-  return (e - 993u) <= 60u || ((w.hi << 1) | w.lo) == 0u;
+  const uint32_t u = w.hi << 1;
+  return u - (993u << 21) < (61u << 21) || (u | w.lo) == 0u;
 }
 DF_HD bool in_range_state(double x) { return in_range_state(words(x)); }
 DF_HD bool in_range_gate(double x) { return in_range_gate(words(x)); }
@@ -154,9 +154,9 @@ DF_HD uint32_t funnel_left3(uint32_t lo, uint32_t hi) {
 DF_HD f2 split(dwords w) {
   if (((w.hi << 1) | w.lo) == 0u) return {0.0f, 0.0f};
   const uint32_t sgn = w.hi & 0x80000000u;
-  const uint32_t hi = (((funnel_left3(w.lo, w.hi) & 0x7FFFFFFFu) ^ 0x40000000u)) | sgn;
-  const uint32_t e = (w.hi >> 20) & 0x7FFu;
-  const uint32_t c1 = (e - 919u) << 23;           // 2^(E-23)
+  const uint32_t f = funnel_left3(w.lo, w.hi);  // low 9 exponent bits at 23-31
+  const uint32_t hi = ((f & 0x7FFFFFFFu) | sgn) ^ 0x40000000u;
+  const uint32_t c1 = (f & 0xFF800000u) - (919u << 23);  // 2^(E-23): (e - 919) << 23 (mod 2^32)
   const uint32_t c0 = c1 - (6u << 23);            // 2^(E-29)
   const float lo_hi = sub(u2f(c1 | ((w.lo >> 6) & 0x7FFFFFu)), u2f(c1));
   const float lo_lo = sub(u2f(c0 | (w.lo & 63u)), u2f(c0));
@@ -200,20 +200,23 @@ DF_HD void acc_mac(acc& r, f2 a, f2 b) {
   r.c = add(r.c, add(err, e));
 }
 
-// Exact float -> double through the bit pattern (normal floats); zero and subnormal
-// floats (rounding residue far below the result) give +-0.
-DF_HD double exact_double(float f) {
-  const uint32_t u = f2u(f);
-  const uint32_t e = (u >> 23) & 0xFFu;
-  const uint32_t sgn = u & 0x80000000u;
-  const uint32_t hi = e ? (sgn | ((e + 896u) << 20) | ((u & 0x7FFFFFu) >> 3)) : sgn;
-  const uint32_t lo = e ? (u << 29) : 0u;
-  return u2d(((uint64_t)hi << 32) | lo);
+// 2^-896 times the float u (its exponent bits taken as a double's): exact, zero and
+// subnormal floats included.
+DF_HD double scaled_double(uint32_t u) {
+  const uint32_t hi = (uint32_t)((int32_t)u >> 3) & 0x8FFFFFFFu;
+  return u2d(((uint64_t)hi << 32) | (u << 29));
+}
+// 2^896 d, 0 for a subnormal d (a sum of floats below 2^-126).
+DF_HD double unscaled_double(double d) {
+  const dwords w = words(d);
+  const bool nz = (w.hi & 0x7FF00000u) != 0u;
+  const uint32_t hi = nz ? w.hi + (896u << 20) : w.hi & 0x80000000u;
+  return u2d(((uint64_t)hi << 32) | (nz ? w.lo : 0u));
 }
 
 // s + c rounded once to double: both parts convert exactly, and the one FP64 add
 // (two per complex element) uses the FP64 pipe that the rest of the path leaves idle.
-DF_HD double to_double(acc r) { return exact_double(r.s) + exact_double(r.c); }
+DF_HD double to_double(acc r) { return unscaled_double(scaled_double(f2u(r.s)) + scaled_double(f2u(r.c))); }
 
 DF_HD f2 renorm(acc r) {
   f2 v;
@@ -237,6 +240,127 @@ DF_HD void cmul_acc(cf2 a, cf2 b, acc& re, acc& im) {
   im = acc_first(a.re, b.im);
   acc_mac(im, a.im, b.re);
 }
+
+#ifdef __CUDACC__
+// ---- two float-float numbers per instruction ---------------------------------------
+// Packed FP32 instructions (add/mul/fma.f32x2) do two correctly rounded operations in one
+// issue slot. The kernels of this header are bound by instruction issue, so the real and
+// imaginary parts of a complex accumulator (or two elements of a stream) go through one
+// instruction stream; every result has the bits of the scalar form above.
+struct x2 {
+  uint64_t v;
+};
+
+__device__ __forceinline__ x2 pack(float a, float b) {
+  x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack(x2 p, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p.v));
+}
+__device__ __forceinline__ x2 add2(x2 a, x2 b) {
+  x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ x2 sub2(x2 a, x2 b) {
+  x2 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ x2 mul2(x2 a, x2 b) {
+  x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ x2 fma2(x2 a, x2 b, x2 c) {
+  x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+
+// Right operand of packed products: high parts, and high and low parts negated (the error
+// of a product is formed as p - a b, so that no product has to be negated).
+struct rhs2 {
+  x2 h, nh, nl;
+};
+__device__ __forceinline__ rhs2 make_rhs(f2 a, f2 b) { return {pack(a.h, b.h), pack(-a.h, -b.h), pack(-a.l, -b.l)}; }
+
+// Left operand: high and low parts.
+struct lhs2 {
+  x2 h, l;
+};
+
+// Two accumulators: values s - nc.
+struct acc2 {
+  x2 s, nc;
+};
+
+// p = fl(ah bh), ne = p - a b (two_prod with the error negated).
+__device__ __forceinline__ void two_prod2(lhs2 a, const rhs2& b, x2& p, x2& ne) {
+  p = mul2(a.h, b.h);
+  ne = fma2(a.h, b.nh, p);
+  ne = fma2(a.h, b.nl, ne);
+  ne = fma2(a.l, b.nh, ne);
+  ne = fma2(a.l, b.nl, ne);
+}
+__device__ __forceinline__ acc2 acc2_first(lhs2 a, const rhs2& b) {
+  acc2 r;
+  two_prod2(a, b, r.s, r.nc);
+  return r;
+}
+__device__ __forceinline__ void acc2_mac(acc2& r, lhs2 a, const rhs2& b) {
+  x2 p, ne;
+  two_prod2(a, b, p, ne);
+  const x2 s = add2(r.s, p), bb = sub2(s, r.s);
+  const x2 err = add2(sub2(r.s, sub2(s, bb)), sub2(p, bb));
+  r.s = s;
+  r.nc = add2(r.nc, sub2(ne, err));
+}
+// The two sums, each rounded once to double (to_double).
+__device__ __forceinline__ void to_double2(const acc2& r, double& a, double& b) {
+  float sa, sb, ca, cb;
+  unpack(r.s, sa, sb);
+  unpack(r.nc, ca, cb);
+  a = unscaled_double(scaled_double(f2u(sa)) - scaled_double(f2u(ca)));
+  b = unscaled_double(scaled_double(f2u(sb)) - scaled_double(f2u(cb)));
+}
+
+__device__ __forceinline__ x2 neg2(x2 a) { return {a.v ^ 0x8000000080000000ull}; }
+__device__ __forceinline__ rhs2 make_rhs(x2 h, x2 l) { return {h, neg2(h), neg2(l)}; }
+
+// Two complex products a b (cmul_acc), `a` as its real and imaginary parts, b's parts (and the
+// negated imaginary ones) as right operands.
+__device__ __forceinline__ void cmul2(lhs2 ar, lhs2 ai, const rhs2& br, const rhs2& bi, const rhs2& nbi, acc2& re,
+                                      acc2& im) {
+  re = acc2_first(ar, br);
+  acc2_mac(re, ai, nbi);
+  im = acc2_first(ar, bi);
+  acc2_mac(im, ai, br);
+}
+__device__ __forceinline__ lhs2 make_lhs(f2 a, f2 b) { return {pack(a.h, b.h), pack(a.l, b.l)}; }
+__device__ __forceinline__ void cmul2(const cf2 (&a)[2], const cf2 (&b)[2], acc2& re, acc2& im) {
+  const rhs2 br = make_rhs(b[0].re, b[1].re), bi = make_rhs(b[0].im, b[1].im);
+  const rhs2 nbi{bi.nh, bi.h, pack(b[0].im.l, b[1].im.l)};
+  cmul2(make_lhs(a[0].re, a[1].re), make_lhs(a[0].im, a[1].im), br, bi, nbi, re, im);
+}
+
+// A complex matrix element as left operands of the products with (re, im) and with
+// (im, re): (gr, gr) and (-gi, gi).
+struct gate2 {
+  lhs2 r, i;
+};
+__device__ __forceinline__ gate2 make_gate2(cf2 g) {
+  return {{pack(g.re.h, g.re.h), pack(g.re.l, g.re.l)}, {pack(-g.im.h, g.im.h), pack(-g.im.l, g.im.l)}};
+}
+// (re, im) += g x, in the order of the scalar kernels: gr x, then gi (i x).
+__device__ __forceinline__ void gate2_mac(acc2& r, bool first, const gate2& g, const rhs2& x, const rhs2& ix) {
+  if (first) r = acc2_first(g.r, x);
+  else acc2_mac(r, g.r, x);
+  acc2_mac(r, g.i, ix);
+}
+#endif
 
 }  // namespace df
 }  // namespace qtnh_impl

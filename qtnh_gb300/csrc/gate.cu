@@ -9,9 +9,10 @@
 // fixed), loads them with 128-bit loads, applies the D x D gate from shared memory and
 // stores them back. Consecutive threads own consecutive groups, so loads and stores are
 // coalesced unless a target is the innermost index, in which case every thread touches D
-// contiguous elements. For D = 8, 9 and 16 the threads of a block share the groups
-// through shared memory, one thread per (output, group) (gate_coop_kernel); any other D
-// runs a general FP64 kernel out of a copy of the state (gate_kernel_any).
+// contiguous elements. The float-float form also takes D = 9 that way; for D = 8 and 16 (and 9
+// in FP64) the threads of a block share the groups through shared memory, one thread per
+// (output, group) (gate_coop_kernel); any other D runs a general FP64 kernel out of a copy
+// of the state (gate_kernel_any).
 //
 // DiagTensor contraction (the reference stubs DiagTensor: src/tensor/diag.cpp:65-117)
 // is defined as contraction with D[in, out] = d[in] * delta(in, out); with the in-place
@@ -40,7 +41,30 @@ struct GateParams {
   // ins_width[j] zero bits at bit ins_pos[j].
   int nins;
   uint32_t ins_pos[8], ins_width[8];
+  // States of fewer than 2^31 elements: `other` with 32-bit strides and divisors (fast_div).
+  uint32_t fdim[KMAX], fmul[KMAX], fshift[KMAX], fstride[KMAX];
 };
+
+// x / d for x < 2^31 by the multiplier and shift of fast_divisor (T. Granlund, P. L. Montgomery,
+// "Division by invariant integers using multiplication", PLDI 1994).
+__device__ __forceinline__ uint32_t fast_div(uint32_t x, uint32_t mul, uint32_t shift) {
+  return (__umulhi(x, mul) + x) >> shift;
+}
+inline void fast_divisor(uint64_t d, uint32_t& mul, uint32_t& shift) {
+  shift = 0;
+  while ((1ull << shift) < d) ++shift;
+  mul = (uint32_t)((((1ull << shift) - d) << 32) / d + 1);
+}
+
+__device__ __forceinline__ uint32_t group_base(uint32_t grp, const GateParams& p) {
+  uint32_t b = 0;
+  for (int j = p.other.n - 1; j > 0; --j) {
+    const uint32_t q = fast_div(grp, p.fmul[j], p.fshift[j]);
+    b += (grp - q * p.fdim[j]) * p.fstride[j];
+    grp = q;
+  }
+  return b + grp * (p.other.n > 0 ? p.fstride[0] : 0u);
+}
 
 __device__ __forceinline__ uint64_t group_base(uint64_t grp, const GateParams& p) {
   if (p.nins >= 0) {
@@ -144,51 +168,54 @@ __device__ __noinline__ void gate_group_fp64(c128* __restrict__ psi, uint64_t ba
 // Float-float variant (see df32.cuh): the FP32 pipe does the arithmetic, complex128 in
 // HBM. A warp whose groups have any element outside the split range takes the FP64
 // path (a warp-uniform branch); so does every group when a gate element is out of range.
-template <int D>
-__global__ void __launch_bounds__(256, (D <= 4 ? 3 : 1)) gate_kernel_f32x2(c128* __restrict__ psi,
-                                                                         const c128* __restrict__ gate,
-                                                                         const __grid_constant__ GateParams p) {
+// Bound by instruction issue (a packed FP32 instruction takes two slots; its gain is in the
+// moves and the shared-memory reads it saves). A thread keeps one group in registers, also
+// for D = 9, whose gate elements all lanes then read as one (in the cooperative form below a
+// warp reads them and the group's amplitudes for every product). As many blocks as are
+// resident at once: each splits the gate first. Measured: D = 2 on 2^26 amplitudes 556 -> 432 us,
+// on 3^14 D = 3 56 -> 42 us and D = 9 128 -> 88 us. Copying ahead into shared memory made
+// D = 2 465 and D = 3 46 us; two groups at a time 470 us.
+template <int D, int B, typename IT>
+__global__ void __launch_bounds__(256, B) gate_kernel_f32x2(c128* __restrict__ psi, const c128* __restrict__ gate,
+                                                          const __grid_constant__ GateParams p) {
   __shared__ c128 g[D * D];
-  __shared__ df::cf2 gs[D * D];
+  __shared__ df::gate2 gs[D * D];
   __shared__ int gate_ok;
-  if (threadIdx.x == 0) gate_ok = 1;
+  const IT total = (IT)p.other.total, step = (IT)gridDim.x * 256;
+  const int tid = threadIdx.x;
+  if (tid == 0) gate_ok = 1;
   __syncthreads();
-  for (int t = threadIdx.x; t < D * D; t += blockDim.x) {
+  for (int t = tid; t < D * D; t += 256) {
     c128 v = gate[t];
     g[t] = v;
     bool ok = df::in_range_gate(v.x) && df::in_range_gate(v.y);
     if (!ok) gate_ok = 0;
-    gs[t] = ok ? df::csplit(v.x, v.y) : df::cf2{{0.f, 0.f}, {0.f, 0.f}};
+    gs[t] = df::make_gate2(ok ? df::csplit(v.x, v.y) : df::cf2{{0.f, 0.f}, {0.f, 0.f}});
   }
   __syncthreads();
   const bool gok = gate_ok != 0;
-  for (uint64_t grp = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; grp < p.other.total;
-       grp += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t base = group_base(grp, p);
+  for (IT grp = (IT)blockIdx.x * 256 + tid; grp < total; grp += step) {
+    const IT base = group_base(grp, p);
     c128 x[D];
+#pragma unroll
+    for (int i = 0; i < D; ++i) x[i] = psi[base + (IT)p.off[i]];
     bool ok = gok;
 #pragma unroll
-    for (int i = 0; i < D; ++i) {
-      x[i] = psi[base + p.off[i]];
-      ok = ok && df::in_range_state(x[i].x) && df::in_range_state(x[i].y);
-    }
+    for (int i = 0; i < D; ++i) ok = ok && df::in_range_state(x[i].x) && df::in_range_state(x[i].y);
     if (__all_sync(__activemask(), ok)) {
-      df::cf2 xs[D];
+      df::acc2 y[D];
 #pragma unroll
-      for (int i = 0; i < D; ++i) xs[i] = df::csplit(x[i].x, x[i].y);
+      for (int i = 0; i < D; ++i) {
+        const df::f2 re = df::split(x[i].x), im = df::split(x[i].y);
+        const df::rhs2 xi = df::make_rhs(re, im), ix = df::make_rhs(im, re);
+#pragma unroll
+        for (int o = 0; o < D; ++o) df::gate2_mac(y[o], i == 0, gs[i * D + o], xi, ix);
+      }
 #pragma unroll
       for (int o = 0; o < D; ++o) {
-        df::acc re, im;
-        df::cmul_acc(gs[o], xs[0], re, im);
-#pragma unroll
-        for (int i = 1; i < D; ++i) {
-          const df::cf2 gi = gs[i * D + o];
-          df::acc_mac(re, gi.re, xs[i].re);
-          df::acc_mac(re, df::neg(gi.im), xs[i].im);
-          df::acc_mac(im, gi.re, xs[i].im);
-          df::acc_mac(im, gi.im, xs[i].re);
-        }
-        psi[base + p.off[o]] = make_double2(df::to_double(re), df::to_double(im));
+        c128 v;
+        df::to_double2(y[o], v.x, v.y);
+        psi[base + (IT)p.off[o]] = v;
       }
     } else {
       gate_group_fp64<D>(psi, base, p.off, g);
@@ -196,7 +223,7 @@ __global__ void __launch_bounds__(256, (D <= 4 ? 3 : 1)) gate_kernel_f32x2(c128*
   }
 }
 
-// Gates of 8 or more amplitudes per group: the threads of a block share the groups'
+// Gates of 8 or 16 amplitudes per group (and 9 in FP64): the threads of a block share the groups'
 // amplitudes through shared memory, one thread per (output, group) and GB = 256 / D
 // groups per batch, instead of one thread holding a whole group in registers (which spills
 // in FP64 and leaves one 8-warp block per SM in float-float). Thread t takes group t % GB
@@ -287,43 +314,79 @@ struct DiagParams {
   int k;
   uint64_t dim[8], stride[8], mult[8];
   uint32_t dim_log2[8], stride_log2[8];
+  uint32_t dim_mul[8], dim_shift[8], stride_mul[8], stride_shift[8];  // fast_div, 32-bit indices only
 };
 
-// Streaming kernels move DU elements per thread per step, all loads issued before any
-// arithmetic, so that enough bytes are in flight per SM to keep HBM busy. IT is the index
+// The FP64 streaming kernels move DU elements per thread per step, all loads issued before
+// any arithmetic, so that enough bytes are in flight per SM to keep HBM busy. IT is the index
 // type (32-bit when the state and the grid stride fit).
 constexpr int DU = 4;
-// Elements of a thread's DU per step that the default arithmetic mode multiplies in native
-// FP64 beside the float-float ones (QTNH_ARITH_F32X2 keeps all DU in float-float).
-constexpr int DIAG_FP64_SLOTS = 1;
-constexpr int LAYER_FP64_SLOTS = 1;
+// Elements per thread and step of the float-float streaming kernels: pairs in packed FP32 (and
+// single ones) and, in the default arithmetic mode, beside them elements in native FP64
+// (QTNH_ARITH_F32X2 keeps all in float-float); steps in the ring; blocks per SM. The FP64 share
+// trades the FP64 unit against instruction issue: 2^26 amplitudes take 418 us with one
+// element in three, 445 with none and 437 with one in five (diagonal, before the index and
+// block count were settled); the layer, whose FP64 elements cost twice as many FP64
+// operations, 489 with one in four, 549 with one in three and 429 with none, which is
+// less precise.
+constexpr int DIAG_FP64_SLOTS = 1, DIAG_PAIRS = 1, DIAG_STEPS = 2, DIAG_BLOCKS = 6;
+constexpr int LAYER_FP64_SLOTS = 1, LAYER_PAIRS = 1, LAYER_SINGLES = 1, LAYER_STEPS = 2, LAYER_BLOCKS = 3;
+constexpr uint64_t DIAG_SMEM = 256;  // diagonals of up to this many entries are split by each block
 
-template <typename IT>
-__device__ __forceinline__ IT diag_index(IT e, const DiagParams& p) {
-  IT idx = 0;
-  for (int j = 0; j < p.k; ++j) {
-    IT q;
-    if (p.stride_log2[j] != 0xFFFFFFFFu) q = e >> p.stride_log2[j];
-    else q = (IT)(e / (IT)p.stride[j]);
-    const IT dg = (p.dim_log2[j] != 0xFFFFFFFFu) ? (q & (IT)(p.dim[j] - 1)) : (IT)(q % (IT)p.dim[j]);
-    idx += dg * (IT)p.mult[j];
+// Index of element e over the targets. Three forms: 64 bits; 32 bits; 32 bits with every extent
+// and stride a power of two.
+struct Index64 {
+  typedef uint64_t type;
+  static __device__ __forceinline__ uint64_t of(uint64_t e, const DiagParams& p) {
+    uint64_t idx = 0;
+    for (int j = 0; j < p.k; ++j) {
+      const uint64_t q = p.stride_log2[j] != 0xFFFFFFFFu ? e >> p.stride_log2[j] : e / p.stride[j];
+      const uint64_t dg = p.dim_log2[j] != 0xFFFFFFFFu ? q & (p.dim[j] - 1) : q % p.dim[j];
+      idx += dg * p.mult[j];
+    }
+    return idx;
   }
-  return idx;
-}
+};
+struct Index32 {
+  typedef uint32_t type;
+  static __device__ __forceinline__ uint32_t of(uint32_t e, const DiagParams& p) {
+    uint32_t idx = 0;
+    for (int j = 0; j < p.k; ++j) {
+      const uint32_t q = fast_div(e, p.stride_mul[j], p.stride_shift[j]);
+      idx += (q - fast_div(q, p.dim_mul[j], p.dim_shift[j]) * (uint32_t)p.dim[j]) * (uint32_t)p.mult[j];
+    }
+    return idx;
+  }
+};
+struct Index32Pow2 {
+  typedef uint32_t type;
+  static __device__ __forceinline__ uint32_t of(uint32_t e, const DiagParams& p) {
+    uint32_t idx = 0;
+    for (int j = 0; j < p.k; ++j) idx += ((e >> p.stride_log2[j]) & ((uint32_t)p.dim[j] - 1)) * (uint32_t)p.mult[j];
+    return idx;
+  }
+};
 
 __device__ __noinline__ c128 cmul_fp64_outofline(c128 a, c128 b) { return cmul(a, b); }
 
+// A phase as float pairs; one out of the gate range is kept as FP64 and flagged with a NaN hi part.
+__device__ __forceinline__ df::cf2 split_flagged(c128 v) {
+  if (df::in_range_gate(v.x) && df::in_range_gate(v.y)) return df::csplit(v.x, v.y);
+  return df::cf2{{__int_as_float(0x7FC00000), 0.f}, {0.f, 0.f}};
+}
+
 // psi[e] *= d[index of e over the targets] in FP64.
-template <typename IT>
+template <typename IX>
 __global__ void __launch_bounds__(256) diag_kernel(c128* __restrict__ psi, const c128* __restrict__ d,
                                                    const __grid_constant__ DiagParams p) {
+  typedef typename IX::type IT;
   const IT n = (IT)p.n, step = (IT)gridDim.x * blockDim.x * DU;
   for (IT base = (IT)blockIdx.x * blockDim.x * DU + threadIdx.x; base < n; base += step) {
     c128 x[DU], f[DU];
 #pragma unroll
     for (int u = 0; u < DU; ++u) {
       const IT e = base + (IT)(u * blockDim.x);
-      if (e < n) x[u] = psi[e], f[u] = __ldg(d + diag_index<IT>(e, p));
+      if (e < n) x[u] = psi[e], f[u] = __ldg(d + IX::of(e, p));
     }
 #pragma unroll
     for (int u = 0; u < DU; ++u) {
@@ -333,45 +396,102 @@ __global__ void __launch_bounds__(256) diag_kernel(c128* __restrict__ psi, const
   }
 }
 
-// The same in float-float: the diagonal comes pre-split (ds, table_split_kernel; a NaN hi
-// part flags an entry outside the float-float range), the amplitude is split per element.
-// The first NF64 of a thread's DU elements per step are multiplied in native FP64 instead:
+// Asynchronous 16-byte copy to the thread's own slot of a ring in shared memory: the loads of a
+// thread's next steps stay in flight while it computes, at no cost in registers and without
+// a barrier (each thread reads only what it copied).
+__device__ __forceinline__ void cp_async16(c128* dst, const c128* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// Ring of a streaming kernel: E elements per thread and step, 256 apart, S steps.
+template <typename IT, int E>
+__device__ __forceinline__ void stream_fetch(c128 (*slot)[256], const c128* psi, IT base, IT n) {
+#pragma unroll
+  for (int u = 0; u < E; ++u) {
+    const IT e = base + (IT)(u * 256);
+    if (e < n) cp_async16(&slot[u][threadIdx.x], psi + e);
+  }
+  cp_commit();
+}
+template <typename IT, int E, int S>
+__device__ __forceinline__ void stream_fetch_ahead(c128 (*ring)[E][256], const c128* psi, IT base, IT step, IT n) {
+#pragma unroll
+  for (int s = 0; s < S - 1; ++s) stream_fetch<IT, E>(ring[s], psi, base + (IT)s * step, n);
+}
+// The elements of the step at `base` (slot `slot`, advanced), and the fetch S - 1 steps on.
+// Those past n are left as they were in the ring.
+template <typename IT, int E, int S>
+__device__ __forceinline__ void stream_take(c128 (*ring)[E][256], int& slot, const c128* psi, IT base, IT step, IT n,
+                                            c128 (&x)[E]) {
+  stream_fetch<IT, E>(ring[slot == 0 ? S - 1 : slot - 1], psi, base + (IT)(S - 1) * step, n);
+  cp_wait<S - 1>();
+#pragma unroll
+  for (int u = 0; u < E; ++u) x[u] = ring[slot][u][threadIdx.x];
+  slot = slot == S - 1 ? 0 : slot + 1;
+}
+
+// The same in float-float: the diagonal is split into float pairs (a NaN hi part flags an
+// entry outside the float-float range), by each block into shared memory (ds == nullptr, up
+// to DIAG_SMEM entries) or ahead of time (ds, table_split_kernel); the amplitude is split per
+// element. The first NF64 elements of a thread's step are multiplied in native FP64 instead:
 // the FP64 unit and the FP32 pipes then work side by side in one instruction stream (each
 // alone caps the kernel below the HBM rate: FP64 by its throughput, float-float by issue).
-template <typename IT, int NF64>
-__global__ void __launch_bounds__(256) diag_kernel_f32x2(c128* __restrict__ psi, const c128* __restrict__ d,
-                                                         const df::cf2* __restrict__ ds,
-                                                         const __grid_constant__ DiagParams p) {
-  static_assert(NF64 >= 0 && NF64 < DU, "at least one float-float element per step");
-  const IT n = (IT)p.n, step = (IT)gridDim.x * blockDim.x * DU;
-  for (IT base = (IT)blockIdx.x * blockDim.x * DU + threadIdx.x; base < n; base += step) {
-    c128 x[DU], fd[NF64 > 0 ? NF64 : 1];
-    df::cf2 f[DU];
-    IT idx[DU];
+// The others go in NP pairs through packed FP32, and the next step's elements are on their way
+// into a ring in shared memory meanwhile. Bound by issue, with HBM at 82 % of its copy rate:
+// 2^26 amplitudes 454 -> 392 us; 3^14 with a two-qutrit diagonal (in L2) 53 -> 37.5 us, of which
+// the divisions by multiplication give 10; 2^16 12 -> 6.9 us (one launch instead of two).
+template <typename IX, int NF64, int NP, int S, int B>
+__global__ void __launch_bounds__(256, B) diag_kernel_f32x2(c128* __restrict__ psi, const c128* __restrict__ d,
+                                                          const df::cf2* __restrict__ ds, uint64_t entries,
+                                                          const __grid_constant__ DiagParams p) {
+  typedef typename IX::type IT;
+  constexpr int E = NF64 + 2 * NP;
+  __shared__ c128 ring[S][E][256];
+  __shared__ df::cf2 tab[DIAG_SMEM];
+  const IT n = (IT)p.n, step = (IT)gridDim.x * 256 * E;
+  const int tid = threadIdx.x;
+  IT base = (IT)blockIdx.x * 256 * E + tid;
+  stream_fetch_ahead<IT, E, S>(ring, psi, base, step, n);
+  if (!ds) {
+    for (int j = tid; j < (int)entries; j += 256) tab[j] = split_flagged(d[j]);
+    __syncthreads();
+  }
+  int slot = 0;
+  for (; base < n; base += step) {
+    c128 x[E];
+    stream_take<IT, E, S>(ring, slot, psi, base, step, n, x);
 #pragma unroll
-    for (int u = 0; u < DU; ++u) {
-      const IT e = base + (IT)(u * blockDim.x);
-      if (e < n) {
-        idx[u] = diag_index<IT>(e, p), x[u] = psi[e];
-        if (u < NF64) fd[u < NF64 ? u : 0] = __ldg(d + idx[u]);
-        else f[u] = ds[idx[u]];
-      }
+    for (int u = 0; u < NF64; ++u) {
+      const IT e = base + (IT)(u * 256);
+      if (e < n) psi[e] = cmul_fused(x[u], __ldg(d + IX::of(e, p)));
     }
 #pragma unroll
-    for (int u = 0; u < DU; ++u) {
-      const IT e = base + (IT)(u * blockDim.x);
-      if (e >= n) continue;
-      if (u < NF64) {
-        psi[e] = cmul_fused(x[u], fd[u < NF64 ? u : 0]);
-        continue;
-      }
-      const bool ok = f[u].re.h == f[u].re.h && df::in_range_state(x[u].x) && df::in_range_state(x[u].y);
+    for (int w = 0; w < NP; ++w) {
+      const IT e0 = base + (IT)((NF64 + 2 * w) * 256), e1 = e0 + 256;
+      if (e0 >= n) continue;
+      const c128 xa = x[NF64 + 2 * w], xb = e1 < n ? x[NF64 + 2 * w + 1] : xa;
+      const IT i0 = IX::of(e0, p), i1 = e1 < n ? IX::of(e1, p) : i0;
+      const df::cf2 fp[2] = {ds ? ds[i0] : tab[i0], ds ? ds[i1] : tab[i1]};
+      const bool ok = fp[0].re.h == fp[0].re.h && fp[1].re.h == fp[1].re.h && df::in_range_state(xa.x) &&
+                      df::in_range_state(xa.y) && df::in_range_state(xb.x) && df::in_range_state(xb.y);
       if (__all_sync(__activemask(), ok)) {
-        df::acc re, im;
-        df::cmul_acc(df::csplit(x[u].x, x[u].y), f[u], re, im);
-        psi[e] = make_double2(df::to_double(re), df::to_double(im));
+        const df::cf2 xp[2] = {df::csplit(xa.x, xa.y), df::csplit(xb.x, xb.y)};
+        df::acc2 re, im;
+        df::cmul2(xp, fp, re, im);
+        c128 ya, yb;
+        df::to_double2(re, ya.x, yb.x);
+        df::to_double2(im, ya.y, yb.y);
+        psi[e0] = ya;
+        if (e1 < n) psi[e1] = yb;
       } else {
-        psi[e] = cmul_fp64_outofline(x[u], __ldg(d + idx[u]));
+        psi[e0] = cmul_fp64_outofline(xa, __ldg(d + i0));
+        if (e1 < n) psi[e1] = cmul_fp64_outofline(xb, __ldg(d + i1));
       }
     }
   }
@@ -390,15 +510,28 @@ struct LayerTableParams {
   uint64_t f_off[LAYER_MAX_FACTORS];     // offset of the factor's entries in `factors`
 };
 
-__global__ void layer_table_kernel(const c128* __restrict__ factors, c128* __restrict__ table,
-                                   const __grid_constant__ LayerTableParams p) {
-  for (uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; j < p.size; j += (uint64_t)gridDim.x * blockDim.x) {
+// Both phase tables, [lo | hi], and (ts) their split copies. A few thousand entries: the time is
+// one thread's chain of factors, so its loads are taken ahead of the products.
+template <typename IT>
+__global__ void layer_table_kernel(const c128* __restrict__ factors, c128* __restrict__ table, df::cf2* __restrict__ ts,
+                                   const __grid_constant__ LayerTableParams lo,
+                                   const __grid_constant__ LayerTableParams hi) {
+  const uint64_t n = lo.size + hi.size;
+  for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < n; t += (uint64_t)gridDim.x * blockDim.x) {
+    const LayerTableParams& p = t < lo.size ? lo : hi;
+    const IT j = (IT)(t < lo.size ? t : t - lo.size);
     c128 v = make_double2(1.0, 0.0);
-    for (int f = 0; f < p.nf; ++f) {
-      uint64_t dgt = (j / p.f_stride[f]) % p.f_dim[f];
-      v = cmul(v, factors[p.f_off[f] + dgt]);
+    for (int f0 = 0; f0 < p.nf; f0 += 4) {
+      c128 w[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        if (f0 + c < p.nf) w[c] = factors[p.f_off[f0 + c] + (j / (IT)p.f_stride[f0 + c]) % (IT)p.f_dim[f0 + c]];
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        if (f0 + c < p.nf) v = cmul(v, w[c]);
     }
-    table[j] = v;
+    table[t] = v;
+    if (ts) ts[t] = split_flagged(v);
   }
 }
 
@@ -444,76 +577,92 @@ __global__ void diag_product_kernel(const c128* gate, const c128* __restrict__ d
   }
 }
 
-// Split copy of a phase table (float pairs) plus a per-entry range flag in the sign of
-// nothing: entries out of the gate range are kept as FP64 and flagged with NaN hi parts.
+// Split copy of a table of phases.
 __global__ void table_split_kernel(const c128* __restrict__ t, df::cf2* __restrict__ ts, uint64_t n) {
-  for (uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; j < n; j += (uint64_t)gridDim.x * blockDim.x) {
-    c128 v = t[j];
-    if (df::in_range_gate(v.x) && df::in_range_gate(v.y)) ts[j] = df::csplit(v.x, v.y);
-    else ts[j] = df::cf2{{__int_as_float(0x7FC00000), 0.f}, {0.f, 0.f}};
-  }
+  for (uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; j < n; j += (uint64_t)gridDim.x * blockDim.x)
+    ts[j] = split_flagged(t[j]);
 }
 
-// Float-float layer; the first NF64 of a thread's DU elements per step in native FP64
-// (as diag_kernel_f32x2).
-template <typename IT, int NF64>
-__global__ void __launch_bounds__(256) layer_apply_kernel_f32x2(c128* __restrict__ psi, const c128* __restrict__ hi,
+// Float-float layer; the first NF64 elements of a thread's step in native FP64, the others in
+// NP pairs of packed FP32 and NS single (as diag_kernel_f32x2). Bound by the FP64 unit and by
+// issue: 2^26 amplitudes with its tables 542 -> 489 us; 2^16, where the tables count,
+// 32.5 -> 18 us (one launch for both tables and their split copies instead of three).
+template <typename IT, int NF64, int NP, int NS, int S, int B>
+__global__ void __launch_bounds__(256, B) layer_apply_kernel_f32x2(c128* __restrict__ psi, const c128* __restrict__ hi,
                                                                 const c128* __restrict__ lo,
                                                                 const df::cf2* __restrict__ his,
                                                                 const df::cf2* __restrict__ los, uint64_t n64,
                                                                 uint64_t lo_size64, uint32_t lo_log2) {
-  static_assert(NF64 >= 0 && NF64 < DU, "at least one float-float element per step");
-  const IT n = (IT)n64, lo_size = (IT)lo_size64, step = (IT)gridDim.x * blockDim.x * DU;
-  for (IT base = (IT)blockIdx.x * blockDim.x * DU + threadIdx.x; base < n; base += step) {
-    c128 x[DU], ad[NF64 > 0 ? NF64 : 1], bd[NF64 > 0 ? NF64 : 1];
-    df::cf2 a[DU], b[DU];
+  constexpr int E = NF64 + 2 * NP + NS;
+  __shared__ c128 ring[S][E][256];
+  const IT n = (IT)n64, lo_size = (IT)lo_size64, step = (IT)gridDim.x * 256 * E;
+  IT base = (IT)blockIdx.x * 256 * E + threadIdx.x;
+  stream_fetch_ahead<IT, E, S>(ring, psi, base, step, n);
+  int slot = 0;
+  for (; base < n; base += step) {
+    c128 x[E];
+    stream_take<IT, E, S>(ring, slot, psi, base, step, n, x);
 #pragma unroll
-    for (int u = 0; u < DU; ++u) {
-      const IT e = base + (IT)(u * blockDim.x);
-      if (e < n) {
-        IT h, l;
-        hi_lo<IT>(e, lo_size, lo_log2, h, l);
-        x[u] = psi[e];
-        if (u < NF64) {
-          ad[u < NF64 ? u : 0] = __ldg(hi + h);
-          bd[u < NF64 ? u : 0] = __ldg(lo + l);
-        } else {
-          a[u] = his[h];
-          b[u] = los[l];
-        }
+    for (int u = 0; u < NF64; ++u) {
+      const IT e = base + (IT)(u * 256);
+      IT h, l;
+      hi_lo<IT>(e, lo_size, lo_log2, h, l);
+      if (e < n) psi[e] = cmul_fused(x[u], cmul_fused(__ldg(hi + h), __ldg(lo + l)));
+    }
+#pragma unroll
+    for (int u = E - NS; u < E; ++u) {
+      const IT e = base + (IT)(u * 256);
+      if (e >= n) continue;
+      IT h, l;
+      hi_lo<IT>(e, lo_size, lo_log2, h, l);
+      const df::cf2 a = his[h], b = los[l];
+      const bool ok = a.re.h == a.re.h && b.re.h == b.re.h && df::in_range_state(x[u].x) && df::in_range_state(x[u].y);
+      if (__all_sync(__activemask(), ok)) {
+        df::acc pr, pi, re, im;
+        df::cmul_acc(a, b, pr, pi);
+        df::cmul_acc(df::csplit(x[u].x, x[u].y), df::cf2{{pr.s, pr.c}, {pi.s, pi.c}}, re, im);
+        psi[e] = make_double2(df::to_double(re), df::to_double(im));
+      } else {
+        psi[e] = cmul_fp64_outofline(x[u], cmul_fp64_outofline(__ldg(hi + h), __ldg(lo + l)));
       }
     }
 #pragma unroll
-    for (int u = 0; u < DU; ++u) {
-      const IT e = base + (IT)(u * blockDim.x);
-      if (e >= n) continue;
-      if (u < NF64) {
-        psi[e] = cmul_fused(x[u], cmul_fused(ad[u < NF64 ? u : 0], bd[u < NF64 ? u : 0]));
-        continue;
-      }
-      const bool ok = a[u].re.h == a[u].re.h && b[u].re.h == b[u].re.h && df::in_range_state(x[u].x) &&
-                      df::in_range_state(x[u].y);
+    for (int w = 0; w < NP; ++w) {
+      const IT e0 = base + (IT)((NF64 + 2 * w) * 256), e1 = e0 + 256;
+      if (e0 >= n) continue;
+      const c128 xa = x[NF64 + 2 * w], xb = e1 < n ? x[NF64 + 2 * w + 1] : xa;
+      IT h0, l0, h1, l1;
+      hi_lo<IT>(e0, lo_size, lo_log2, h0, l0);
+      hi_lo<IT>(e1 < n ? e1 : e0, lo_size, lo_log2, h1, l1);
+      const df::cf2 ap[2] = {his[h0], his[h1]}, bp[2] = {los[l0], los[l1]};
+      const bool ok = ap[0].re.h == ap[0].re.h && bp[0].re.h == bp[0].re.h && ap[1].re.h == ap[1].re.h &&
+                      bp[1].re.h == bp[1].re.h && df::in_range_state(xa.x) && df::in_range_state(xa.y) &&
+                      df::in_range_state(xb.x) && df::in_range_state(xb.y);
       if (__all_sync(__activemask(), ok)) {
-        df::acc pr, pi;
-        df::cmul_acc(a[u], b[u], pr, pi);
+        df::acc2 pr, pi, re, im;
+        df::cmul2(ap, bp, pr, pi);
         // the unnormalised pairs (sum, error) enter the next product as they are: its
         // TwoProduct multiplies out all four hi/lo terms, and the error part is a few
         // units in the last place of the sum
-        const df::cf2 ph{{pr.s, pr.c}, {pi.s, pi.c}};
-        df::acc re, im;
-        df::cmul_acc(df::csplit(x[u].x, x[u].y), ph, re, im);
-        psi[e] = make_double2(df::to_double(re), df::to_double(im));
+        const df::rhs2 br{pr.s, df::neg2(pr.s), pr.nc}, bi{pi.s, df::neg2(pi.s), pi.nc};
+        const df::rhs2 nbi{bi.nh, bi.h, df::neg2(pi.nc)};
+        const df::cf2 xs0 = df::csplit(xa.x, xa.y), xs1 = df::csplit(xb.x, xb.y);
+        df::cmul2(df::make_lhs(xs0.re, xs1.re), df::make_lhs(xs0.im, xs1.im), br, bi, nbi, re, im);
+        c128 ya, yb;
+        df::to_double2(re, ya.x, yb.x);
+        df::to_double2(im, ya.y, yb.y);
+        psi[e0] = ya;
+        if (e1 < n) psi[e1] = yb;
       } else {
-        IT h, l;
-        hi_lo<IT>(e, lo_size, lo_log2, h, l);
-        psi[e] = cmul_fp64_outofline(x[u], cmul_fp64_outofline(__ldg(hi + h), __ldg(lo + l)));
+        psi[e0] = cmul_fp64_outofline(xa, cmul_fp64_outofline(__ldg(hi + h0), __ldg(lo + l0)));
+        if (e1 < n) psi[e1] = cmul_fp64_outofline(xb, cmul_fp64_outofline(__ldg(hi + h1), __ldg(lo + l1)));
       }
     }
   }
 }
 
-// 32-bit indices when n plus one grid stride of DU elements per thread fits.
-inline bool index32(uint64_t n, int grid) { return n + (uint64_t)grid * 256 * DU < (1ull << 32); }
+// 32-bit indices when n plus the steps fetched ahead (32 elements per thread) fits.
+inline bool index32(uint64_t n, int grid) { return n + (uint64_t)grid * 256 * 32 < (1ull << 32); }
 
 // Merge the non-target axes into runs and describe them (state strides in s_in).
 void other_axes(const dims_t& dims, const std::vector<uint16_t>& targets, RestDesc& out) {
@@ -585,9 +734,22 @@ void apply_gate_device(void* state, const dims_t& dims, const std::vector<uint16
   const c128* g = static_cast<const c128*>(gate);
   int grid = grid_for((p.other.total + 255) / 256, 8);
   const bool ff = arithmetic_mode() != QTNH_ARITH_FP64;
-#define QTNH_GATE_CASE(DD)                                                  \
+  // 32-bit indices when the state and one grid stride of groups fit
+  const bool i32 = product(dims) + (uint64_t)grid * 256 * 8 < (1ull << 31);
+  for (int j = 0; i32 && j < p.other.n; ++j) {
+    p.fdim[j] = (uint32_t)p.other.ax[j].dim;
+    fast_divisor(p.other.ax[j].dim, p.fmul[j], p.fshift[j]);
+    p.fstride[j] = (uint32_t)p.other.ax[j].s_in;
+  }
+#define QTNH_GATE_FF(DD, BB)                                                              \
+  {                                                                                           \
+    const int fg = grid_for((p.other.total + 255) / 256, BB);                                 \
+    if (i32) gate_kernel_f32x2<DD, BB, uint32_t><<<fg, 256, 0, s>>>(psi, g, p);           \
+    else gate_kernel_f32x2<DD, BB, uint64_t><<<fg, 256, 0, s>>>(psi, g, p);               \
+  }
+#define QTNH_GATE_CASE(DD, BB)                                          \
   case DD:                                                                  \
-    if (ff) gate_kernel_f32x2<DD><<<grid, 256, 0, s>>>(psi, g, p);          \
+    if (ff) QTNH_GATE_FF(DD, BB)                                        \
     else gate_kernel<DD><<<grid, 256, 0, s>>>(psi, g, p);                   \
     break;
 #define QTNH_GATE_COOP_CASE(DD)                                                            \
@@ -598,12 +760,16 @@ void apply_gate_device(void* state, const dims_t& dims, const std::vector<uint16
     break;                                                                                 \
   }
   switch (D) {
-    QTNH_GATE_CASE(1)
-    QTNH_GATE_CASE(2)
-    QTNH_GATE_CASE(3)
-    QTNH_GATE_CASE(4)
+    QTNH_GATE_CASE(1, 5)
+    QTNH_GATE_CASE(2, 6)
+    QTNH_GATE_CASE(3, 4)
+    QTNH_GATE_CASE(4, 3)
     QTNH_GATE_COOP_CASE(8)
-    QTNH_GATE_COOP_CASE(9)
+    case 9: {
+      if (ff) QTNH_GATE_FF(9, 2)
+      else gate_coop_kernel<9, false><<<grid_for((p.other.total + 27) / 28, 8), 256, 0, s>>>(psi, g, p);
+      break;
+    }
     QTNH_GATE_COOP_CASE(16)
     default: {
       // other sizes: the general kernel out of a copy of the state
@@ -626,6 +792,7 @@ void apply_gate_device(void* state, const dims_t& dims, const std::vector<uint16
       break;
     }
   }
+#undef QTNH_GATE_FF
 #undef QTNH_GATE_CASE
 #undef QTNH_GATE_COOP_CASE
   count_launch();
@@ -643,39 +810,54 @@ void apply_diag_device(void* state, const dims_t& dims, const std::vector<uint16
   p.k = (int)targets.size();
   dims_t st = row_strides(dims);
   uint64_t m = 1;
+  bool pow2 = true;
   for (int j = p.k - 1; j >= 0; --j) {
     p.dim[j] = dims[targets[j]];
     p.stride[j] = st[targets[j]];
     p.dim_log2[j] = log2_or_none(p.dim[j]);
     p.stride_log2[j] = log2_or_none(p.stride[j]);
+    pow2 = pow2 && p.dim_log2[j] != 0xFFFFFFFFu && p.stride_log2[j] != 0xFFFFFFFFu;
+    if (n < (1ull << 31)) {
+      fast_divisor(p.dim[j], p.dim_mul[j], p.dim_shift[j]);
+      fast_divisor(p.stride[j], p.stride_mul[j], p.stride_shift[j]);
+    }
     p.mult[j] = m;
     m *= p.dim[j];
   }
   cudaStream_t s = (cudaStream_t)stream;
   const int grid = grid_for((n + 256 * DU - 1) / (256 * DU), 8);
+  const bool i32 = index32(n, grid), i32g = n + (uint64_t)grid * 256 * 32 < (1ull << 31);
   c128* st_ = static_cast<c128*>(state);
   const c128* d_ = static_cast<const c128*>(diag);
   const bool ff = arithmetic_mode() != QTNH_ARITH_FP64;
   if (ff) {
-    // the diagonal's entries split once into float pairs
-    df::cf2* ds = static_cast<df::cf2*>(workspace_alloc(m * sizeof(df::cf2), stream));
-    table_split_kernel<<<grid_for((m + 255) / 256, 4), 256, 0, s>>>(d_, ds, m);
-    const bool i32 = index32(n, grid);
-    if (arithmetic_mode() == QTNH_ARITH_F32X2) {
-      if (i32) diag_kernel_f32x2<uint32_t, 0><<<grid, 256, 0, s>>>(st_, d_, ds, p);
-      else diag_kernel_f32x2<uint64_t, 0><<<grid, 256, 0, s>>>(st_, d_, ds, p);
-    } else {
-      if (i32) diag_kernel_f32x2<uint32_t, DIAG_FP64_SLOTS><<<grid, 256, 0, s>>>(st_, d_, ds, p);
-      else diag_kernel_f32x2<uint64_t, DIAG_FP64_SLOTS><<<grid, 256, 0, s>>>(st_, d_, ds, p);
+    const bool f64 = arithmetic_mode() != QTNH_ARITH_F32X2;
+    // a diagonal of up to DIAG_SMEM entries is split by each block; a larger one once, ahead
+    df::cf2* ds = nullptr;
+    if (m > DIAG_SMEM) {
+      ds = static_cast<df::cf2*>(workspace_alloc(m * sizeof(df::cf2), stream));
+      table_split_kernel<<<grid_for((m + 255) / 256, 4), 256, 0, s>>>(d_, ds, m);
+      count_launch();
     }
-    count_launch(2);
+    auto run = [&](auto ix, auto slots) {
+      constexpr int NF = decltype(slots)::value, E = NF + 2 * DIAG_PAIRS;
+      diag_kernel_f32x2<decltype(ix), NF, DIAG_PAIRS, DIAG_STEPS, DIAG_BLOCKS>
+          <<<grid_for((n + 256 * E - 1) / (256 * E), DIAG_BLOCKS), 256, 0, s>>>(st_, d_, ds, m, p);
+    };
+    using F64 = std::integral_constant<int, DIAG_FP64_SLOTS>;
+    using F32 = std::integral_constant<int, 0>;
+    if (i32 && pow2) f64 ? run(Index32Pow2(), F64()) : run(Index32Pow2(), F32());
+    else if (i32g) f64 ? run(Index32(), F64()) : run(Index32(), F32());
+    else f64 ? run(Index64(), F64()) : run(Index64(), F32());
+    count_launch();
     const cudaError_t e = cudaGetLastError();
-    workspace_free(ds, stream);
+    if (ds) workspace_free(ds, stream);
     check_cuda(e, "diag_kernel launch");
     return;
   }
-  if (index32(n, grid)) diag_kernel<uint32_t><<<grid, 256, 0, s>>>(st_, d_, p);
-  else diag_kernel<uint64_t><<<grid, 256, 0, s>>>(st_, d_, p);
+  if (i32 && pow2) diag_kernel<Index32Pow2><<<grid, 256, 0, s>>>(st_, d_, p);
+  else if (i32g) diag_kernel<Index32><<<grid, 256, 0, s>>>(st_, d_, p);
+  else diag_kernel<Index64><<<grid, 256, 0, s>>>(st_, d_, p);
   count_launch();
   check_cuda(cudaGetLastError(), "diag_kernel launch");
 }
@@ -715,37 +897,37 @@ void apply_diag_layer_device(void* state, const dims_t& dims, const std::vector<
   const size_t tab = lo_size + hi_size;
   c128* tables = static_cast<c128*>(workspace_alloc(tab * sizeof(c128) * (ff ? 2 : 1), stream));
   const c128* fac = static_cast<const c128*>(factors);
-  layer_table_kernel<<<grid_for((lo_size + 255) / 256, 4), 256, 0, s>>>(fac, tables, *lo);
-  layer_table_kernel<<<grid_for((hi_size + 255) / 256, 4), 256, 0, s>>>(fac, tables + lo_size, *hi);
+  df::cf2* split_tab = ff ? reinterpret_cast<df::cf2*>(tables + tab) : nullptr;
+  const int tgrid = grid_for((tab + 127) / 128, 8);
+  if (tab < (1ull << 32)) layer_table_kernel<uint32_t><<<tgrid, 128, 0, s>>>(fac, tables, split_tab, *lo, *hi);
+  else layer_table_kernel<uint64_t><<<tgrid, 128, 0, s>>>(fac, tables, split_tab, *lo, *hi);
   const int grid = grid_for((n + 256 * DU - 1) / (256 * DU), 8);
   const bool i32 = index32(n, grid);
   c128* st_ = static_cast<c128*>(state);
   const uint32_t lo_log2 = log2_or_none(lo_size);
+  count_launch(2);
   if (ff) {
-    df::cf2* split_tab = reinterpret_cast<df::cf2*>(tables + tab);
-    table_split_kernel<<<grid_for((tab + 255) / 256, 4), 256, 0, s>>>(tables, split_tab, tab);
     const c128* hi_t = tables + lo_size;
     const df::cf2* his = split_tab + lo_size;
-    if (arithmetic_mode() == QTNH_ARITH_F32X2) {
-      if (i32)
-        layer_apply_kernel_f32x2<uint32_t, 0><<<grid, 256, 0, s>>>(st_, hi_t, tables, his, split_tab, n, lo_size, lo_log2);
-      else
-        layer_apply_kernel_f32x2<uint64_t, 0><<<grid, 256, 0, s>>>(st_, hi_t, tables, his, split_tab, n, lo_size, lo_log2);
-    } else {
-      if (i32)
-        layer_apply_kernel_f32x2<uint32_t, LAYER_FP64_SLOTS><<<grid, 256, 0, s>>>(st_, hi_t, tables, his, split_tab, n,
-                                                                                lo_size, lo_log2);
-      else
-        layer_apply_kernel_f32x2<uint64_t, LAYER_FP64_SLOTS><<<grid, 256, 0, s>>>(st_, hi_t, tables, his, split_tab, n,
-                                                                                lo_size, lo_log2);
-    }
-    count_launch(4);
+    const bool f64 = arithmetic_mode() != QTNH_ARITH_F32X2;
+    auto run = [&](auto idx, auto slots) {
+      typedef decltype(idx) IT;
+      constexpr int NF = decltype(slots)::value, E = NF + 2 * LAYER_PAIRS + LAYER_SINGLES;
+      layer_apply_kernel_f32x2<IT, NF, LAYER_PAIRS, LAYER_SINGLES, LAYER_STEPS, LAYER_BLOCKS>
+          <<<grid_for((n + 256 * E - 1) / (256 * E), LAYER_BLOCKS), 256, 0, s>>>(st_, hi_t, tables, his, split_tab, n,
+                                                                             lo_size, lo_log2);
+    };
+    using F64 = std::integral_constant<int, LAYER_FP64_SLOTS>;
+    using F32 = std::integral_constant<int, 0>;
+    if (f64 && i32) run(uint32_t(), F64());
+    else if (f64) run(uint64_t(), F64());
+    else if (i32) run(uint32_t(), F32());
+    else run(uint64_t(), F32());
   } else {
     if (i32)
       layer_apply_kernel<uint32_t><<<grid, 256, 0, s>>>(st_, tables + lo_size, tables, n, lo_size, lo_log2);
     else
       layer_apply_kernel<uint64_t><<<grid, 256, 0, s>>>(st_, tables + lo_size, tables, n, lo_size, lo_log2);
-    count_launch(3);
   }
   cudaError_t e = cudaGetLastError();
   workspace_free(tables, stream);
