@@ -78,6 +78,17 @@ __device__ __forceinline__ void decode(uint64_t idx, const RestDesc& r, uint64_t
   }
 }
 
+// x / d for x < 2^31 by the multiplier and shift of fast_divisor (T. Granlund, P. L. Montgomery,
+// "Division by invariant integers using multiplication", PLDI 1994).
+__device__ __forceinline__ uint32_t fast_div(uint32_t x, uint32_t mul, uint32_t shift) {
+  return (__umulhi(x, mul) + x) >> shift;
+}
+inline void fast_divisor(uint64_t d, uint32_t& mul, uint32_t& shift) {
+  shift = 0;
+  while ((1ull << shift) < d) ++shift;
+  mul = (uint32_t)((((1ull << shift) - d) << 32) / d + 1);
+}
+
 inline void fill_axis(Axis& a, uint64_t dim, uint64_t s_in, uint64_t s_out) {
   a.dim = dim;
   a.log2 = log2_or_none(dim);

@@ -45,17 +45,6 @@ struct GateParams {
   uint32_t fdim[KMAX], fmul[KMAX], fshift[KMAX], fstride[KMAX];
 };
 
-// x / d for x < 2^31 by the multiplier and shift of fast_divisor (T. Granlund, P. L. Montgomery,
-// "Division by invariant integers using multiplication", PLDI 1994).
-__device__ __forceinline__ uint32_t fast_div(uint32_t x, uint32_t mul, uint32_t shift) {
-  return (__umulhi(x, mul) + x) >> shift;
-}
-inline void fast_divisor(uint64_t d, uint32_t& mul, uint32_t& shift) {
-  shift = 0;
-  while ((1ull << shift) < d) ++shift;
-  mul = (uint32_t)((((1ull << shift) - d) << 32) / d + 1);
-}
-
 __device__ __forceinline__ uint32_t group_base(uint32_t grp, const GateParams& p) {
   uint32_t b = 0;
   for (int j = p.other.n - 1; j > 0; --j) {

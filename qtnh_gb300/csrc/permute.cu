@@ -19,7 +19,7 @@
 //     staged in shared memory in XOR-swizzled rows (one padding slot per row where the
 //     row length is not a multiple of 8); the per-element offsets of
 //     the tile come as tables in the kernel parameters (copied to shared memory), and
-//     small tiles are processed several per step so that enough loads are in flight;
+//     tiles are processed several per step so that enough loads are in flight;
 //   * a gather (coalesced stores, indexed loads) when no tile fits.
 
 #include <algorithm>
@@ -36,16 +36,21 @@ namespace {
 
 constexpr int TILE_MAX = 1024;   // elements per transpose tile
 constexpr int TILE_THREADS = 256;
-constexpr int STEP_ELEMS = 2048;  // elements of the tiles moved per step of a block (power-of-two tiles)
+constexpr int STEP_ELEMS = 2048;  // elements of the tiles moved per step of a block, at most
 constexpr int TILE_PER_THREAD = STEP_ELEMS / TILE_THREADS;
+constexpr int DECODE_WARPS = TILE_THREADS / 32;  // up to this many tiles per step are decoded by a warp each
 static_assert(TILE_MAX <= STEP_ELEMS, "one step holds at least one tile");
 
 
 struct TileParams {
   RestDesc rest;
   int T;           // elements per tile
-  int G;           // tiles per step (T is a power of two when G > 1)
+  int G;           // tiles per step (fused split: T is a power of two when G > 1)
   uint32_t T_log2;
+  uint32_t T_mul, T_shift;  // fast_div by T
+  int lanes;                // a warp decodes each tile of a step (G <= DECODE_WARPS)
+  int fast;                 // rest.total < 2^31: then by fast_div
+  uint32_t sfx_mul[KMAX], sfx_shift[KMAX], dim_mul[KMAX], dim_shift[KMAX];  // by the axes after k; by axis k
   int quad;        // fused split: write order runs in aligned quads of consecutive columns
   int tile_slots;
   int64_t rin[TILE_MAX];   // read order: input offset within the tile
@@ -60,56 +65,108 @@ struct RunParams {
   uint32_t L_log2;
 };
 
+// Offsets of tile `idx` of p.rest, one axis per lane (the whole warp calls it, with one idx).
+__device__ __forceinline__ void decode_warp(uint64_t idx, const TileParams& p, uint64_t& bin, uint64_t& bout) {
+  bin = bout = 0;
+  uint64_t sfx = 1;
+  if (!p.fast)
+    for (int k = p.rest.n - 1; k > (int)(threadIdx.x & 31); --k) sfx *= p.rest.ax[k].dim;
+  for (int k = threadIdx.x & 31; k < p.rest.n; k += 32) {
+    uint64_t d;
+    if (p.fast) {
+      const uint32_t q = fast_div((uint32_t)idx, p.sfx_mul[k], p.sfx_shift[k]);
+      d = q - fast_div(q, p.dim_mul[k], p.dim_shift[k]) * (uint32_t)p.rest.ax[k].dim;
+    } else {
+      if (k >= 32) {  // (more axes than lanes)
+        sfx = 1;
+        for (int j = p.rest.n - 1; j > k; --j) sfx *= p.rest.ax[j].dim;
+      }
+      d = (idx / sfx) % p.rest.ax[k].dim;
+    }
+    bin += d * p.rest.ax[k].s_in;
+    bout += d * p.rest.ax[k].s_out;
+  }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    bin += __shfl_xor_sync(0xffffffffu, bin, o);
+    bout += __shfl_xor_sync(0xffffffffu, bout, o);
+  }
+}
+
+// Bound by HBM on large states and, where L2 holds them, by the latency of a step: the bases of a
+// step's tiles are decoded during the loads of the step before, for extents other than
+// powers of two one axis per lane and by multiplication. 14 qutrits in a random order
+// 71 -> 55 us, [5] * 10 108 -> 80, 20 qubits 27 -> 24, 26 qubits 370 -> 356 (in step, and by
+// divisions in turn, before).
 __global__ void __launch_bounds__(TILE_THREADS, 4) tiled_permute_kernel(const c128* __restrict__ in, c128* __restrict__ out,
                                                                      const __grid_constant__ TileParams p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int T = p.T, G = p.G, S = p.tile_slots;
   c128* tile = reinterpret_cast<c128*>(smem_raw);  // G tiles of S slots
-  uint64_t* s_bin = reinterpret_cast<uint64_t*>(tile + (size_t)G * S);
-  uint64_t* s_bout = s_bin + G;
-  int64_t* s_rin = reinterpret_cast<int64_t*>(s_bout + G);
+  uint64_t* s_bin = reinterpret_cast<uint64_t*>(tile + (size_t)G * S);  // [2][G]
+  uint64_t* s_bout = s_bin + 2 * G;                                     // [2][G]
+  int64_t* s_rin = reinterpret_cast<int64_t*>(s_bout + 2 * G);
   int64_t* s_wout = s_rin + T;
   int32_t* s_rslot = reinterpret_cast<int32_t*>(s_wout + T);
   int32_t* s_wslot = s_rslot + T;
-  for (int t = threadIdx.x; t < T; t += blockDim.x) {
+  const uint64_t total = p.rest.total, stride = (uint64_t)gridDim.x * G;
+  auto decode_step = [&](uint64_t r0, int q) {
+    if (p.lanes) {  // warp g takes tile g
+      const int g = threadIdx.x >> 5;
+      if (g < G && r0 + g < total) {
+        uint64_t bin, bout;
+        decode_warp(r0 + g, p, bin, bout);
+        if ((threadIdx.x & 31) == 0) s_bin[q * G + g] = bin, s_bout[q * G + g] = bout;
+      }
+    } else {
+      for (int g = threadIdx.x; g < G && r0 + g < total; g += TILE_THREADS) {
+        uint64_t bin, bout;
+        decode(r0 + g, p.rest, bin, bout);
+        s_bin[q * G + g] = bin;
+        s_bout[q * G + g] = bout;
+      }
+    }
+  };
+  decode_step((uint64_t)blockIdx.x * G, 0);
+  for (int t = threadIdx.x; t < T; t += TILE_THREADS) {
     s_rin[t] = p.rin[t];
     s_wout[t] = p.wout[t];
     s_rslot[t] = p.rslot[t];
     s_wslot[t] = p.wslot[t];
   }
-  const uint64_t total = p.rest.total;
-  for (uint64_t r0 = (uint64_t)blockIdx.x * G; r0 < total; r0 += (uint64_t)gridDim.x * G) {
-    for (int g = threadIdx.x; g < G && r0 + g < total; g += blockDim.x) {
-      uint64_t bin, bout;
-      decode(r0 + g, p.rest, bin, bout);
-      s_bin[g] = bin;
-      s_bout[g] = bout;
-    }
-    __syncthreads();
+  __syncthreads();
+  int q = 0;
+  for (uint64_t r0 = (uint64_t)blockIdx.x * G; r0 < total; r0 += stride, q ^= 1) {
     const uint64_t left = total - r0;
     const int n = (left < (uint64_t)G ? (int)left : G) * T;  // <= STEP_ELEMS
+    const uint64_t* bin = s_bin + q * G;
+    const uint64_t* bout = s_bout + q * G;
     // all of this thread's loads are issued before any is stored to shared memory
     c128 v[TILE_PER_THREAD];
-    int slot[TILE_PER_THREAD];
 #pragma unroll
     for (int k = 0; k < TILE_PER_THREAD; ++k) {
       const int e = threadIdx.x + k * TILE_THREADS;
       if (e < n) {
-        const int g = G > 1 ? e >> p.T_log2 : 0, t = G > 1 ? e & (T - 1) : e;
-        slot[k] = g * S + s_rslot[t];
-        v[k] = __ldg(in + s_bin[g] + s_rin[t]);
+        const int g = G > 1 ? (int)fast_div((uint32_t)e, p.T_mul, p.T_shift) : 0, t = e - g * T;
+        v[k] = __ldg(in + bin[g] + s_rin[t]);
       }
     }
+    decode_step(r0 + stride, q ^ 1);  // (the loads are in flight)
 #pragma unroll
-    for (int k = 0; k < TILE_PER_THREAD; ++k)
-      if (threadIdx.x + k * TILE_THREADS < n) tile[slot[k]] = v[k];
+    for (int k = 0; k < TILE_PER_THREAD; ++k) {
+      const int e = threadIdx.x + k * TILE_THREADS;
+      if (e < n) {
+        const int g = G > 1 ? (int)fast_div((uint32_t)e, p.T_mul, p.T_shift) : 0, t = e - g * T;
+        tile[g * S + s_rslot[t]] = v[k];
+      }
+    }
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < TILE_PER_THREAD; ++k) {
       const int e = threadIdx.x + k * TILE_THREADS;
       if (e < n) {
-        const int g = G > 1 ? e >> p.T_log2 : 0, t = G > 1 ? e & (T - 1) : e;
-        out[s_bout[g] + s_wout[t]] = tile[g * S + s_wslot[t]];
+        const int g = G > 1 ? (int)fast_div((uint32_t)e, p.T_mul, p.T_shift) : 0, t = e - g * T;
+        out[bout[g] + s_wout[t]] = tile[g * S + s_wslot[t]];
       }
     }
     __syncthreads();
@@ -505,8 +562,11 @@ Plan plan_permute(const dims_t& dims, const std::vector<uint16_t>& ptup, int bou
     };
     p.tile_slots = (int)(swz ? PB * PA : PB * (PA + 1));
     const uint32_t tl = log2_or_none((uint64_t)T);
-    p.G = (tl != 0xFFFFFFFFu && T < STEP_ELEMS) ? std::min(STEP_ELEMS / T, 256) : 1;
+    p.G = (tl != 0xFFFFFFFFu || boundary < 0) ? std::min(STEP_ELEMS / T, 256) : 1;
+    // a small tensor: fewer tiles per step rather than SMs without a block
+    if (boundary < 0) p.G = (int)std::max<uint64_t>(1, std::min<uint64_t>(p.G, N / T / (uint64_t)sm_count()));
     p.T_log2 = tl == 0xFFFFFFFFu ? 0 : tl;
+    fast_divisor((uint64_t)T, p.T_mul, p.T_shift);
     // fused split: the tile's trailing output positions that are column axes form a run
     // of consecutive columns (stride 1 innermost); if its length is a multiple of 4,
     // write order goes in aligned quads (every other axis strides by multiples of it)
@@ -569,8 +629,20 @@ Plan plan_permute(const dims_t& dims, const std::vector<uint16_t>& ptup, int bou
       if (!inA[i] && !inB[i]) fill_axis(p.rest.ax[nr++], c.dims[i], in_stride[i], out_stride[i]);
     p.rest.n = nr;
     p.rest.total = N / (uint64_t)T;
-    // the fused split double-buffers its tiles and keeps three slots of tile bases
-    const size_t nbuf = boundary >= 0 ? 2 : 1, nbase = boundary >= 0 ? 3 : 1;
+    // one axis per lane costs less than divisions in turn, shifts in turn less than the lanes
+    // (2^26 elements in a random order: 356 us by shifts, 404 by lanes)
+    p.lanes = 0;
+    for (int k = 0; k < nr; ++k)
+      if (p.rest.ax[k].log2 == 0xFFFFFFFFu && p.G <= DECODE_WARPS) p.lanes = 1;
+    p.fast = p.rest.total < (1ull << 31) ? 1 : 0;
+    uint64_t sfx = 1;
+    for (int k = nr - 1; p.fast && k >= 0; --k) {
+      fast_divisor(sfx, p.sfx_mul[k], p.sfx_shift[k]);
+      fast_divisor(p.rest.ax[k].dim, p.dim_mul[k], p.dim_shift[k]);
+      sfx *= p.rest.ax[k].dim;
+    }
+    // the fused split double-buffers its tiles and keeps three slots of tile bases (else two)
+    const size_t nbuf = boundary >= 0 ? 2 : 1, nbase = boundary >= 0 ? 3 : 2;
     plan.smem = nbuf * (size_t)p.G * p.tile_slots * sizeof(c128) + 2 * nbase * (size_t)p.G * sizeof(uint64_t) +
                 (size_t)T * (2 * sizeof(int64_t) + 2 * sizeof(int32_t));
     // as many blocks per SM as shared memory and registers allow (at most 4)
