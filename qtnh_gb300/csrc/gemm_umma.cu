@@ -25,10 +25,18 @@
 // x 256 columns x one K-slice: warp 0 streams each K-step's six blocks (36 KB) into a 5-stage
 // shared-memory ring with bulk copies (cp.async.bulk, mbarrier transaction counts),
 // warp 1's elected thread issues six tcgen05.mma (M 128, N 256, K 16) per K-step into
-// the two TMEM accumulators and commits the stage back to the producer, and warps 2-5
-// read the finished accumulator (tcgen05.ld) and either pair the Re/Im rows with a
-// shuffle and store complex128 (one slice) or store the FP32 partials. Every wait is
-// bounded by a clock limit (device error flags).
+// the two TMEM accumulators and commits the stage back to the producer, and warps 2-9
+// read the finished accumulators (tcgen05.ld) into registers, free them, and then store
+// the FP32 partials or (one slice) pair the Re/Im rows with a shuffle and store complex128.
+// A K-step takes the tensor cores 768 cycles, in which 36 KB per SM from L2 is more than L2
+// gives all SMs; so where the row tiles are even in number two CTAs form a cluster, take
+// neighbouring row tiles and load half of B's blocks each into both (24 KB from L2). Measured
+// at M 4096, N 4096, K 2048: 880 us, what cuBLAS's rate allows for the operations is 873;
+// without pairs and with four epilogue warps that stored before freeing 1047 us. The
+// partials' sum is 255 us more (1.3 GB, 5.2 TB/s); summing a tile's slices inside this
+// kernel as they become complete took 1055 us in all instead of 880 + 255, for the whole
+// contraction 1312 us against 1340: not worth its code. Every wait is bounded by a clock
+// limit (device error flags).
 
 #include <cuda_bf16.h>
 
@@ -55,7 +63,8 @@ constexpr int GM_STAGES = 5;
 constexpr int GM_A_BLOCK = GM_M * GM_K * 2;  // 4096 bytes: one plane, one tile, one K-step
 constexpr int GM_B_BLOCK = GM_N * GM_K * 2;  // 8192 bytes
 constexpr int GM_STAGE_BYTES = GM_P * (GM_A_BLOCK + GM_B_BLOCK);
-constexpr int GM_THREADS = 192;            // warp 0 producer, warp 1 MMA, warps 2-5 epilogue
+constexpr int GM_EPI_WARPS = 8;             // four TMEM lane quarters x two column halves
+constexpr int GM_THREADS = 64 + 32 * GM_EPI_WARPS;  // warp 0 producer, warp 1 MMA, warps 2-9 epilogue
 constexpr uint32_t GM_TMEM_COLS = 512;     // accumulators D1 (h*h) and D2 (other pairs), GM_N columns each
 constexpr long long GM_WAIT_CYCLES = 1ll << 32;  // ~2 s at 2 GHz
 
@@ -111,6 +120,13 @@ __device__ __forceinline__ bool mbar_wait_thread(uint64_t* bar, uint32_t parity,
   }
   return true;
 }
+// After an expired wait: gives the copies of the stages in flight time to land (~0.5 ms at most).
+__device__ __forceinline__ void mbar_drain(uint64_t* full, uint32_t it, uint32_t stages) {
+  const long long t0 = clock64();
+  for (uint32_t x = it > stages ? it - stages : 0; x < it; ++x)
+    while (!mbar_try_wait(&full[x % stages], (x / stages) & 1u) && clock64() - t0 < (1 << 20)) {
+    }
+}
 // Warp-uniform bounded wait.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort) {
   const long long t0 = clock64();
@@ -126,6 +142,23 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
       "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
       "l"(src), "r"(bytes), "r"(smem_u32(bar))
       : "memory");
+}
+
+// The same into this CTA and the other one of the pair, at the same offsets.
+__device__ __forceinline__ void bulk_g2s_pair(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.multicast::cluster [%0], [%1], %2, [%3], "
+      "%4;" ::"r"(smem_u32(dst)),
+      "l"(src), "r"(bytes), "r"(smem_u32(bar)), "h"((uint16_t)3)
+      : "memory");
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -152,6 +185,15 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
                : "memory");
 }
 
+// The arrival in both CTAs of the pair.
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+          smem_u32(bar)),
+      "h"((uint16_t)3)
+      : "memory");
+}
+
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
@@ -164,15 +206,27 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// 32 consecutive bytes (a whole sector) per lane.
+__device__ __forceinline__ void store_sector(float* dst, const uint32_t* v) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+               "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+               : "memory");
+}
+
+// PAIR: the two CTAs of a cluster take neighbouring row tiles of one column tile and share B's
+// blocks: each loads half of every block into both.
+template <bool PAIR>
 __global__ void __launch_bounds__(GM_THREADS, 1) gemm_bf16x3_umma_kernel(const __grid_constant__ GemmParams p) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   GmSmem& sm = *reinterpret_cast<GmSmem*>(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const uint64_t ntiles = (uint64_t)p.MT * p.NT * p.S;
-  // tile -> (row tile, column tile, K-slice), row tiles fastest (neighbours share B)
+  constexpr uint32_t CL = PAIR ? 2 : 1;
+  const uint32_t rank = PAIR ? cluster_rank() : 0;
+  const uint64_t ntiles = (uint64_t)(p.MT / CL) * p.NT * p.S, first = blockIdx.x / CL, stride = gridDim.x / CL;
+  // tile (of the pair) -> (row tile, column tile, K-slice), row tiles fastest (neighbours share B)
   auto tile_coords = [&](uint64_t tile, uint64_t& mt, uint64_t& nt, uint32_t& k0, uint32_t& k1) {
-    mt = tile % p.MT;
-    const uint64_t rest = tile / p.MT;
+    mt = tile % (p.MT / CL) * CL + rank;
+    const uint64_t rest = tile / (p.MT / CL);
     nt = rest % p.NT;
     const uint32_t sl = (uint32_t)(rest / p.NT);
     k0 = sl * p.SK;
@@ -183,10 +237,10 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_bf16x3_umma_kernel(const _
     sm.abort = 0;
     for (int s = 0; s < GM_STAGES; ++s) {
       mbar_init(&sm.full[s], 1);
-      mbar_init(&sm.empty[s], 1);
+      mbar_init(&sm.empty[s], CL);
     }
     mbar_init(&sm.tfull, 1);
-    mbar_init(&sm.tempty, 128);
+    mbar_init(&sm.tempty, GM_EPI_WARPS);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -197,6 +251,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_bf16x3_umma_kernel(const _
   }
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync_all();  // the other CTA's barriers are ready
   tc_fence_after();
   const uint32_t tmem = sm.tmem_base;
 
@@ -205,7 +260,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_bf16x3_umma_kernel(const _
     if (lane == 0) {
       uint32_t it = 0;
       bool ok = true;
-      for (uint64_t tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x) {
+      for (uint64_t tile = first; ok && tile < ntiles; tile += stride) {
         uint64_t mt, nt;
         uint32_t k0, k1;
         tile_coords(tile, mt, nt, k0, k1);
@@ -215,6 +270,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_bf16x3_umma_kernel(const _
             atomicOr(&g_gemm_error, 1u);
             sm.abort = 1;
             ok = false;
+            mbar_drain(sm.full, it, GM_STAGES);
             break;
           }
           mbar_arrive_expect_tx(&sm.full[s], (uint32_t)GM_STAGE_BYTES);
@@ -224,9 +280,14 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_bf16x3_umma_kernel(const _
           for (int pl = 0; pl < GM_P; ++pl)
             bulk_g2s(&sm.stage[s][pl * GM_A_BLOCK], p.a_planes + pl * p.a_plane_bytes + ablk, GM_A_BLOCK, &sm.full[s]);
 #pragma unroll
-          for (int pl = 0; pl < GM_P; ++pl)
-            bulk_g2s(&sm.stage[s][GM_P * GM_A_BLOCK + pl * GM_B_BLOCK], p.b_planes + pl * p.b_plane_bytes + bblk,
-                     GM_B_BLOCK, &sm.full[s]);
+          for (int pl = 0; pl < GM_P; ++pl) {
+            uint8_t* dst = &sm.stage[s][GM_P * GM_A_BLOCK + pl * GM_B_BLOCK];
+            const uint8_t* src = p.b_planes + pl * p.b_plane_bytes + bblk;
+            if (PAIR)
+              bulk_g2s_pair(dst + rank * (GM_B_BLOCK / 2), src + rank * (GM_B_BLOCK / 2), GM_B_BLOCK / 2, &sm.full[s]);
+            else
+              bulk_g2s(dst, src, GM_B_BLOCK, &sm.full[s]);
+          }
         }
       }
     }
@@ -235,7 +296,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_bf16x3_umma_kernel(const _
     if (lane == 0) {
       uint32_t it = 0, lt = 0;
       bool ok = true;
-      for (uint64_t tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x, ++lt) {
+      for (uint64_t tile = first; ok && tile < ntiles; tile += stride, ++lt) {
         if (!mbar_wait_thread(&sm.tempty, (lt & 1u) ^ 1u, &sm.abort)) {
           atomicOr(&g_gemm_error, 2u);
           sm.abort = 1;
@@ -266,72 +327,72 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_bf16x3_umma_kernel(const _
             else
               umma_bf16(d2, ad, bd, (ks > k0 || q > 1) ? 1u : 0u);
           }
-          umma_commit(&sm.empty[s]);  // the stage is free once these MMAs have read it
+          // the stage is free once these MMAs (and the other CTA's) have read it
+          if (PAIR) umma_commit_pair(&sm.empty[s]);
+          else umma_commit(&sm.empty[s]);
         }
         if (ok) umma_commit(&sm.tfull);
       }
     }
   } else {
-    // ---- epilogue: warps 2-5 read TMEM lanes 32 (warp % 4) .. +31 ----
-    const int q = warp & 3, r = q * 32 + lane;
+    // ---- epilogue: warp w reads TMEM lanes 32 (w % 4) .. +31, columns 128 ((w - 2) / 4) .. +127,
+    // all into registers first: the next tile's MMAs start before anything is stored ----
+    const int q = warp & 3, h = (warp - 2) >> 2, r = q * 32 + lane;
+    constexpr int CW = GM_N / (GM_EPI_WARPS / 4), NCH = CW / 32;
     uint32_t lt = 0;
-    for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++lt) {
+    for (uint64_t tile = first; tile < ntiles; tile += stride, ++lt) {
       if (!mbar_wait_warp(&sm.tfull, lt & 1u, &sm.abort)) {
         atomicOr(&g_gemm_error, 4u);
         sm.abort = 1;
         break;
       }
       tc_fence_after();
+      const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(h * CW);
+      // D1 + D2 (one rounding to nearest)
+      uint32_t v[NCH][32];
+#pragma unroll
+      for (int ch = 0; ch < NCH; ++ch) {
+        uint32_t w[32];
+        tmem_ld32(tbase + (uint32_t)(ch * 32), v[ch]);
+        tmem_ld32(tbase + (uint32_t)(GM_N + ch * 32), w);
+        tmem_wait_ld();
+#pragma unroll
+        for (int x = 0; x < 32; ++x)
+          v[ch][x] = __float_as_uint(__fadd_rn(__uint_as_float(v[ch][x]), __uint_as_float(w[x])));
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sm.tempty);
       uint64_t mt, nt;
       uint32_t k0, k1;
       tile_coords(tile, mt, nt, k0, k1);
       const uint64_t R = mt * GM_M + (uint64_t)r;  // row of C^: complex row R / 2, part R % 2
       const uint64_t m = R >> 1;
       const bool odd = (lane & 1) != 0;
-      const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16);
-      // 32 columns of D1 + D2 (one rounding to nearest)
-      auto load_sum = [&](int ch, uint32_t (&v)[32]) {
-        uint32_t w[32];
-        tmem_ld32(tbase + (uint32_t)(ch * 32), v);
-        tmem_ld32(tbase + (uint32_t)(GM_N + ch * 32), w);
-        tmem_wait_ld();
-#pragma unroll
-        for (int x = 0; x < 32; ++x) v[x] = __float_as_uint(__fadd_rn(__uint_as_float(v[x]), __uint_as_float(w[x])));
-      };
       if (p.S > 1) {
-        // FP32 partials of this slice: row R of C^, 256 columns
-        float* dst = p.partial + ((uint64_t)(k0 / p.SK) * p.MT * GM_M + R) * ((uint64_t)p.NT * GM_N) + nt * GM_N;
-#pragma unroll 1
-        for (int ch = 0; ch < GM_N / 32; ++ch) {
-          uint32_t v[32];
-          load_sum(ch, v);
+        // FP32 partials of this slice: row R of C^, 128 columns
+        float* dst = p.partial + ((uint64_t)(k0 / p.SK) * p.MT * GM_M + R) * ((uint64_t)p.NT * GM_N) + nt * GM_N + h * CW;
 #pragma unroll
-          for (int x = 0; x < 32; x += 4)
-            *reinterpret_cast<uint4*>(dst + ch * 32 + x) = make_uint4(v[x], v[x + 1], v[x + 2], v[x + 3]);
-        }
-        tc_fence_before();
-        mbar_arrive(&sm.tempty);
+        for (int ch = 0; ch < NCH; ++ch)
+#pragma unroll
+          for (int x = 0; x < 32; x += 8) store_sector(dst + ch * 32 + x, &v[ch][x]);
         continue;
       }
-#pragma unroll 1
-      for (int ch = 0; ch < GM_N / 32; ++ch) {
-        uint32_t v[32];
-        load_sum(ch, v);
+#pragma unroll
+      for (int ch = 0; ch < NCH; ++ch) {
         // the even lane (Re row) writes columns 0..15 of the chunk, the odd lane (Im row)
         // columns 16..31; each receives the other part from its partner
-        const uint64_t n0 = nt * GM_N + (uint64_t)ch * 32 + (odd ? 16 : 0);
+        const uint64_t n0 = nt * GM_N + (uint64_t)(h * CW + ch * 32) + (odd ? 16 : 0);
 #pragma unroll
         for (int x = 0; x < 16; ++x) {
-          const uint32_t send = odd ? v[x] : v[16 + x];
+          const uint32_t send = odd ? v[ch][x] : v[ch][16 + x];
           const uint32_t recv = __shfl_xor_sync(0xffffffffu, send, 1);
-          const float re = __uint_as_float(odd ? recv : v[x]);
-          const float im = __uint_as_float(odd ? v[16 + x] : recv);
+          const float re = __uint_as_float(odd ? recv : v[ch][x]);
+          const float im = __uint_as_float(odd ? v[ch][16 + x] : recv);
           const uint64_t n = n0 + (uint64_t)x;
           if (m < p.M && n < p.N) p.C[m * p.N + n] = make_double2((double)re, (double)im);
         }
       }
-      tc_fence_before();
-      mbar_arrive(&sm.tempty);
     }
   }
 
@@ -341,6 +402,8 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_bf16x3_umma_kernel(const _
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(GM_TMEM_COLS) : "memory");
   }
+  __syncwarp();
+  if (PAIR) cluster_sync_all();  // neither CTA leaves while the other may still copy or arrive here
 }
 
 using bx3::pieces;
@@ -505,9 +568,14 @@ static void gemm_core(const Prep& pa, const Prep& pb, void* Cv, uint64_t M, uint
       count_launch();
     }
     const size_t smem = sizeof(GmSmem);
-    check_cuda(cudaFuncSetAttribute(gemm_bf16x3_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+    // two CTAs share B where every row tile has a partner (with an odd number the last pair would
+    // work on padding; one in 64 rows of C either way)
+    const bool pair = p.MT % 2 == 0;
+    const auto kernel = pair ? gemm_bf16x3_umma_kernel<true> : gemm_bf16x3_umma_kernel<false>;
+    check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                "gemm_bf16x3_umma_kernel shared memory");
-    const int grid = (int)std::min<uint64_t>((uint64_t)p.MT * p.NT * p.S, (uint64_t)sm_count());
+    const uint64_t sms = pair ? (uint64_t)sm_count() & ~1ull : (uint64_t)sm_count();
+    const int grid = (int)std::min<uint64_t>((uint64_t)p.MT * p.NT * p.S, sms);
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     {
       std::lock_guard<std::mutex> lk(g_timing_mu);
@@ -517,7 +585,18 @@ static void gemm_core(const Prep& pa, const Prep& pb, void* Cv, uint64_t M, uint
         check_cuda(cudaEventRecord(e0, s), "event record");
       }
     }
-    gemm_bf16x3_umma_kernel<<<grid, GM_THREADS, smem, s>>>(p);
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = pair ? 2 : 1;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(GM_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    check_cuda(cudaLaunchKernelEx(&cfg, kernel, p), "gemm_bf16x3_umma_kernel launch");
     if (e0) {
       check_cuda(cudaEventRecord(e1, s), "event record");
       std::lock_guard<std::mutex> lk(g_timing_mu);
