@@ -80,14 +80,20 @@ def launches():
     return int(lib().qtnh_kernel_launch_count())
 
 
+def _array(ctype, vals):
+    try:
+        return (ctype * max(1, len(vals)))(*vals)
+    except TypeError:  # not plain ints (numpy's, floats, an iterator)
+        vals = [int(v) for v in vals]
+        return (ctype * max(1, len(vals)))(*vals)
+
+
 def _u64(vals):
-    vals = [int(v) for v in vals]
-    return (ctypes.c_uint64 * max(1, len(vals)))(*vals)
+    return _array(ctypes.c_uint64, vals)
 
 
 def _u16(vals):
-    vals = [int(v) for v in vals]
-    return (ctypes.c_uint16 * max(1, len(vals)))(*vals)
+    return _array(ctypes.c_uint16, vals)
 
 
 def _stream(stream=None):
@@ -123,48 +129,43 @@ class Tensor:
         return self.dis + self.loc
 
     def desc(self):
-        self._dims = _u64(self.dims)
-        return TensorDesc(self.kind, len(self.dis), len(self.loc), self.n_dis_in,
-                          ctypes.cast(self._dims, ctypes.POINTER(ctypes.c_uint64)),
-                          ctypes.c_void_p(self.data.data_ptr() if self.data is not None else 0))
+        dims = _u64(self.dis + self.loc)  # (the field keeps it alive)
+        return TensorDesc(self.kind, len(self.dis), len(self.loc), self.n_dis_in, dims,
+                          self.data.data_ptr() if self.data is not None else None)
+
+
+def _plan(t1, t2, wires, repls):
+    """The plan call: its arguments before and after use_default, which the contraction itself
+    takes on (a pass of its own through Python cost more than the plan), and its results."""
+    d1, d2 = t1.desc(), t2.desc()
+    r1, r2 = d1.ndis + d1.nloc, d2.ndis + d2.nloc
+    rep1 = (ctypes.c_uint16 * max(1, r1))(*(repls[0] if repls else ()))  # (default: outputs only)
+    rep2 = (ctypes.c_uint16 * max(1, r2))(*(repls[1] if repls else ()))
+    ndis, nloc, st = ctypes.c_int32(), ctypes.c_int32(), ctypes.c_uint64()
+    out_dims = (ctypes.c_uint64 * max(1, r1 + r2))()
+    args = (ctypes.byref(d1), ctypes.byref(d2), ctypes.c_int32(len(wires)), _u16([x for p in wires for x in p]))
+    outs = (rep1, rep2, ctypes.byref(ndis), ctypes.byref(nloc), out_dims, ctypes.byref(st))
+    check(lib().qtnh_contract_plan(*args, ctypes.c_int32(0 if repls else 1), *outs))
+    dims = out_dims[:ndis.value + nloc.value]
+    return args, outs, dims[:ndis.value], dims[ndis.value:], rep1[:r1], rep2[:r2], st.value
 
 
 def contract_plan(t1, t2, wires, repls=None):
     """Tensor::contract metadata (host only). Returns (dis, loc, repls1, repls2, str)."""
-    r1, r2 = len(t1.dims), len(t2.dims)
-    w = _u16([x for p in wires for x in p])
-    rep1 = (ctypes.c_uint16 * max(1, r1))(*(repls[0] if repls else [X] * r1))
-    rep2 = (ctypes.c_uint16 * max(1, r2))(*(repls[1] if repls else [X] * r2))
-    ndis, nloc, st = ctypes.c_int32(), ctypes.c_int32(), ctypes.c_uint64()
-    out_dims = (ctypes.c_uint64 * max(1, r1 + r2))()
-    d1, d2 = t1.desc(), t2.desc()
-    check(lib().qtnh_contract_plan(ctypes.byref(d1), ctypes.byref(d2), ctypes.c_int32(len(wires)), w,
-                                   ctypes.c_int32(0 if repls else 1), rep1, rep2, ctypes.byref(ndis),
-                                   ctypes.byref(nloc), out_dims, ctypes.byref(st)))
-    dims = [int(out_dims[i]) for i in range(ndis.value + nloc.value)]
-    return (dims[:ndis.value], dims[ndis.value:], [rep1[i] for i in range(r1)], [rep2[i] for i in range(r2)],
-            int(st.value))
+    return _plan(t1, t2, wires, repls)[2:]
 
 
 def contract(t1, t2, wires, repls=None, out=None, stream=None):
     """Tensor::contract on the device. Returns (Tensor result, repls1, repls2, str)."""
-    import torch
-    dis, loc, rep1, rep2, st = contract_plan(t1, t2, wires, repls)
-    n = 1
-    for d in dis + loc:
-        n *= d
+    args, outs, dis, loc, rep1, rep2, st = _plan(t1, t2, wires, repls)
     if out is None:
+        import torch
+        n = 1
+        for d in dis + loc:
+            n *= d
         out = torch.empty(n, dtype=torch.complex128, device="cuda")
-    r1, r2 = len(t1.dims), len(t2.dims)
-    w = _u16([x for p in wires for x in p])
-    a1 = (ctypes.c_uint16 * max(1, r1))(*rep1)
-    a2 = (ctypes.c_uint16 * max(1, r2))(*rep2)
-    ndis, nloc, stv = ctypes.c_int32(), ctypes.c_int32(), ctypes.c_uint64()
-    out_dims = (ctypes.c_uint64 * max(1, r1 + r2))()
-    d1, d2 = t1.desc(), t2.desc()
-    check(lib().qtnh_contract(ctypes.byref(d1), ctypes.byref(d2), ctypes.c_int32(len(wires)), w, ctypes.c_int32(0),
-                              a1, a2, ctypes.byref(ndis), ctypes.byref(nloc), out_dims, ctypes.byref(stv), _ptr(out),
-                              ctypes.c_uint64(out.numel()), _stream(stream)))
+    check(lib().qtnh_contract(*args, ctypes.c_int32(0), *outs, _ptr(out), ctypes.c_uint64(out.numel()),
+                              _stream(stream)))
     return Tensor(DENSE, dis, loc, out.reshape(-1)), rep1, rep2, st
 
 
