@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <memory>
 #include <numeric>
+#include <type_traits>
 
 #include "cuda_common.cuh"
 #include "df32.cuh"
@@ -318,7 +319,7 @@ constexpr int DU = 4;
 // block count were settled); the layer, whose FP64 elements cost twice as many FP64
 // operations, 489 with one in four, 549 with one in three and 429 with none, which is
 // less precise.
-constexpr int DIAG_FP64_SLOTS = 1, DIAG_PAIRS = 1, DIAG_STEPS = 2, DIAG_BLOCKS = 6;
+constexpr int DIAG_FP64_SLOTS = 1, DIAG_PAIRS = 1, DIAG_STEPS = 2, DIAG_BLOCKS = 6, DIAG_HIGH_BLOCKS = 5;
 constexpr int LAYER_FP64_SLOTS = 1, LAYER_PAIRS = 1, LAYER_SINGLES = 1, LAYER_STEPS = 2, LAYER_BLOCKS = 3;
 constexpr uint64_t DIAG_SMEM = 256;  // diagonals of up to this many entries are split by each block
 
@@ -398,6 +399,11 @@ __device__ __forceinline__ void cp_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// Exactly 1 (a nonzero rest of the significand leaves a nonzero low part).
+__device__ __forceinline__ bool is_one(const df::cf2& f) {
+  return f.re.h == 1.0f && f.re.l == 0.0f && f.im.h == 0.0f && f.im.l == 0.0f;
+}
+
 // Ring of a streaming kernel: E elements per thread and step, 256 apart, S steps.
 template <typename IT, int E>
 __device__ __forceinline__ void stream_fetch(c128 (*slot)[256], const c128* psi, IT base, IT n) {
@@ -435,7 +441,13 @@ __device__ __forceinline__ void stream_take(c128 (*ring)[E][256], int& slot, con
 // into a ring in shared memory meanwhile. Bound by issue, with HBM at 82 % of its copy rate:
 // 2^26 amplitudes 454 -> 392 us; 3^14 with a two-qutrit diagonal (in L2) 53 -> 37.5 us, of which
 // the divisions by multiplication give 10; 2^16 12 -> 6.9 us (one launch instead of two).
-template <typename IX, int NF64, int NP, int S, int B>
+// HIGH (every target's stride is a multiple of 32 elements): a warp's 32 elements (512 bytes)
+// have one factor, and if at least a quarter of the entries are exactly 1, as in a
+// controlled phase, elements with that factor stay as they are and are not written: 2^26
+// amplitudes 392 -> 260 us. The test in every step costs more than it gives elsewhere
+// (general entries 392 -> 468 us), so it has a loop of its own. Elements outside the split
+// range are multiplied all the same: infinities and NaNs come out as the product gives them.
+template <typename IX, int NF64, int NP, int S, int B, bool HIGH>
 __global__ void __launch_bounds__(256, B) diag_kernel_f32x2(c128* __restrict__ psi, const c128* __restrict__ d,
                                                           const df::cf2* __restrict__ ds, uint64_t entries,
                                                           const __grid_constant__ DiagParams p) {
@@ -447,43 +459,58 @@ __global__ void __launch_bounds__(256, B) diag_kernel_f32x2(c128* __restrict__ p
   const int tid = threadIdx.x;
   IT base = (IT)blockIdx.x * 256 * E + tid;
   stream_fetch_ahead<IT, E, S>(ring, psi, base, step, n);
+  int ones = 0;
   if (!ds) {
     for (int j = tid; j < (int)entries; j += 256) tab[j] = split_flagged(d[j]);
-    __syncthreads();
+    if (HIGH) ones = __syncthreads_count(tid < (int)entries && is_one(tab[tid]));
+    else __syncthreads();
   }
-  int slot = 0;
-  for (; base < n; base += step) {
-    c128 x[E];
-    stream_take<IT, E, S>(ring, slot, psi, base, step, n, x);
+  auto stream = [&](auto keep) {
+    constexpr bool KEEP = decltype(keep)::value;
+    int slot = 0;
+    for (; base < n; base += step) {
+      c128 x[E];
+      stream_take<IT, E, S>(ring, slot, psi, base, step, n, x);
 #pragma unroll
-    for (int u = 0; u < NF64; ++u) {
-      const IT e = base + (IT)(u * 256);
-      if (e < n) psi[e] = cmul_fused(x[u], __ldg(d + IX::of(e, p)));
-    }
+      for (int u = 0; u < NF64; ++u) {
+        const IT e = base + (IT)(u * 256);
+        if (e >= n) continue;
+        const c128 f = __ldg(d + IX::of(e, p));
+        if (KEEP && __all_sync(__activemask(), f.x == 1.0 && f.y == 0.0 && df::in_range_state(x[u].x) &&
+                                                  df::in_range_state(x[u].y)))
+          continue;
+        psi[e] = cmul_fused(x[u], f);
+      }
 #pragma unroll
-    for (int w = 0; w < NP; ++w) {
-      const IT e0 = base + (IT)((NF64 + 2 * w) * 256), e1 = e0 + 256;
-      if (e0 >= n) continue;
-      const c128 xa = x[NF64 + 2 * w], xb = e1 < n ? x[NF64 + 2 * w + 1] : xa;
-      const IT i0 = IX::of(e0, p), i1 = e1 < n ? IX::of(e1, p) : i0;
-      const df::cf2 fp[2] = {ds ? ds[i0] : tab[i0], ds ? ds[i1] : tab[i1]};
-      const bool ok = fp[0].re.h == fp[0].re.h && fp[1].re.h == fp[1].re.h && df::in_range_state(xa.x) &&
-                      df::in_range_state(xa.y) && df::in_range_state(xb.x) && df::in_range_state(xb.y);
-      if (__all_sync(__activemask(), ok)) {
-        const df::cf2 xp[2] = {df::csplit(xa.x, xa.y), df::csplit(xb.x, xb.y)};
-        df::acc2 re, im;
-        df::cmul2(xp, fp, re, im);
-        c128 ya, yb;
-        df::to_double2(re, ya.x, yb.x);
-        df::to_double2(im, ya.y, yb.y);
-        psi[e0] = ya;
-        if (e1 < n) psi[e1] = yb;
-      } else {
-        psi[e0] = cmul_fp64_outofline(xa, __ldg(d + i0));
-        if (e1 < n) psi[e1] = cmul_fp64_outofline(xb, __ldg(d + i1));
+      for (int w = 0; w < NP; ++w) {
+        const IT e0 = base + (IT)((NF64 + 2 * w) * 256), e1 = e0 + 256;
+        if (e0 >= n) continue;
+        const c128 xa = x[NF64 + 2 * w], xb = e1 < n ? x[NF64 + 2 * w + 1] : xa;
+        const IT i0 = IX::of(e0, p), i1 = e1 < n ? IX::of(e1, p) : i0;
+        const df::cf2 fp[2] = {ds ? ds[i0] : tab[i0], ds ? ds[i1] : tab[i1]};
+        const bool ok = fp[0].re.h == fp[0].re.h && fp[1].re.h == fp[1].re.h && df::in_range_state(xa.x) &&
+                        df::in_range_state(xa.y) && df::in_range_state(xb.x) && df::in_range_state(xb.y);
+        const uint32_t mask = __activemask();
+        if (__all_sync(mask, ok)) {
+          const bool keep_a = KEEP && __all_sync(mask, is_one(fp[0])), keep_b = KEEP && __all_sync(mask, is_one(fp[1]));
+          if (keep_a && keep_b) continue;
+          const df::cf2 xp[2] = {df::csplit(xa.x, xa.y), df::csplit(xb.x, xb.y)};
+          df::acc2 re, im;
+          df::cmul2(xp, fp, re, im);
+          c128 ya, yb;
+          df::to_double2(re, ya.x, yb.x);
+          df::to_double2(im, ya.y, yb.y);
+          if (!keep_a) psi[e0] = ya;
+          if (!keep_b && e1 < n) psi[e1] = yb;
+        } else {
+          psi[e0] = cmul_fp64_outofline(xa, __ldg(d + i0));
+          if (e1 < n) psi[e1] = cmul_fp64_outofline(xb, __ldg(d + i1));
+        }
       }
     }
-  }
+  };
+  if (HIGH && 4 * ones >= (int)entries) stream(std::true_type());
+  else stream(std::false_type());
 }
 
 // ---- diagonal layer ----------------------------------------------------------------
@@ -799,13 +826,14 @@ void apply_diag_device(void* state, const dims_t& dims, const std::vector<uint16
   p.k = (int)targets.size();
   dims_t st = row_strides(dims);
   uint64_t m = 1;
-  bool pow2 = true;
+  bool pow2 = true, high = true;  // high: every target's stride is a multiple of 32
   for (int j = p.k - 1; j >= 0; --j) {
     p.dim[j] = dims[targets[j]];
     p.stride[j] = st[targets[j]];
     p.dim_log2[j] = log2_or_none(p.dim[j]);
     p.stride_log2[j] = log2_or_none(p.stride[j]);
     pow2 = pow2 && p.dim_log2[j] != 0xFFFFFFFFu && p.stride_log2[j] != 0xFFFFFFFFu;
+    high = high && p.stride[j] % 32 == 0;
     if (n < (1ull << 31)) {
       fast_divisor(p.dim[j], p.dim_mul[j], p.dim_shift[j]);
       fast_divisor(p.stride[j], p.stride_mul[j], p.stride_shift[j]);
@@ -830,8 +858,13 @@ void apply_diag_device(void* state, const dims_t& dims, const std::vector<uint16
     }
     auto run = [&](auto ix, auto slots) {
       constexpr int NF = decltype(slots)::value, E = NF + 2 * DIAG_PAIRS;
-      diag_kernel_f32x2<decltype(ix), NF, DIAG_PAIRS, DIAG_STEPS, DIAG_BLOCKS>
-          <<<grid_for((n + 256 * E - 1) / (256 * E), DIAG_BLOCKS), 256, 0, s>>>(st_, d_, ds, m, p);
+      constexpr bool can = std::is_same<decltype(ix), Index32Pow2>::value;
+      if (can && high && !ds)
+        diag_kernel_f32x2<decltype(ix), NF, DIAG_PAIRS, DIAG_STEPS, DIAG_HIGH_BLOCKS, can>
+            <<<grid_for((n + 256 * E - 1) / (256 * E), DIAG_HIGH_BLOCKS), 256, 0, s>>>(st_, d_, ds, m, p);
+      else
+        diag_kernel_f32x2<decltype(ix), NF, DIAG_PAIRS, DIAG_STEPS, DIAG_BLOCKS, false>
+            <<<grid_for((n + 256 * E - 1) / (256 * E), DIAG_BLOCKS), 256, 0, s>>>(st_, d_, ds, m, p);
     };
     using F64 = std::integral_constant<int, DIAG_FP64_SLOTS>;
     using F32 = std::integral_constant<int, 0>;

@@ -103,3 +103,40 @@ def test_diagonal_layer_any_extents(dims, axes, scale, arith):
         shape[a] = dims[a]
         ref = ref * f.reshape(shape)
     close(out, ref)
+
+
+# Entries that are exactly 1 (kept as they are where whole warps share them): targets above and
+# among the lowest five bits, more and fewer ones than a quarter, and an entry next to 1.
+@pytest.mark.parametrize("n,targets", [(5, [0]), (6, [0]), (12, [1, 4]), (12, [6, 7]), (13, [0, 12]), (16, [3, 0, 9]), (14, [])])
+@pytest.mark.parametrize("ones", ["phase", "most", "few", "next", "all"])
+def test_diagonal_with_ones(n, targets, ones, arith):
+    rng = np.random.default_rng(n + len(targets))
+    m = 2 ** len(targets)
+    d = np.exp(1j * rng.uniform(0.1, 6.2, m))
+    if ones == "phase":
+        d[:-1] = 1
+    elif ones == "most":
+        d[1:] = 1
+    elif ones == "few":
+        d[0] = 1
+    elif ones == "next":
+        d[:] = 1 + 2.0 ** -52
+    else:
+        d[:] = 1
+    x = state(rng, [2] * n, "unit")
+    bad = x.copy()
+    bad.reshape(-1)[2 ** n // 2] = complex(np.inf, 1)
+    bad.reshape(-1)[2 ** n // 2 + 1] = complex(1, np.nan)
+    td = torch.from_numpy(d).cuda()
+    f = np.ones([2] * n, dtype=np.complex128)
+    shape = [1] * n
+    for t in targets:
+        shape[t] = 2
+    f = f * (np.transpose(d.reshape([2] * len(targets)), np.argsort(targets)).reshape(shape) if targets else d)
+    close(run(x, lambda t: q.apply_diag(t, [2] * n, targets, td)), x * f)
+    out = run(bad, lambda t: q.apply_diag(t, [2] * n, targets, td))
+    with np.errstate(invalid="ignore"):
+        ref = bad * f
+    fin = np.isfinite(ref)
+    assert np.array_equal(np.isfinite(out), fin)
+    close(out[fin], ref[fin])
