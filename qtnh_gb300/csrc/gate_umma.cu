@@ -482,6 +482,15 @@ struct ChSmem {
 static_assert(CH_NLMAX * UM_N <= (int)CH_ACC, "chain level sums exceed an accumulator set");
 static_assert(2 * CH_ACC <= CH_TMEM_COLS, "two accumulator sets");
 static_assert(sizeof(ChSmem) + 1024 <= 227 * 1024, "chain shared memory");
+
+// Stage slot of amplitude c of row r: rows of odd amplitudes four off, so that neither the
+// fetch in either order nor the reads meet bank conflicts.
+__device__ __forceinline__ int chain_slot(int c, int r) { return c * UM_M + (r ^ ((c & 1) << 2)); }
+// Two neighbouring fixed-point amplitudes (32 bytes, aligned).
+__device__ __forceinline__ void st_pair(void* p, int64_t a, int64_t b, int64_t c, int64_t d) {
+  asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(a), "l"(b), "l"(c), "l"(d) : "memory");
+}
+
 //
 // The input is what the previous pass wrote (rin): doubles with the largest group key of
 // all of them, or 64-bit fixed point at scale rin->F with the largest |hi word|. Both are
@@ -508,7 +517,15 @@ static_assert(sizeof(ChSmem) + 1024 <= 227 * 1024, "chain shared memory");
 // index P(x) of the permutation `perm` (bit tables in shared memory; P(tile part | row
 // part | offset) is the OR of the three parts' images, the row part's and the offsets'
 // computed once), so the pass and the permutation after it take one pass over the state.
-template <typename IT, uint32_t MODE, int NL, bool PO>
+//
+// LOW (bit 0 among the targets, or bits 1 and 2): with the gates' order of amplitudes and rows
+// on the lanes such a pass moves half sectors (bits 1 and 2: scattered ones). Here amplitude
+// index bits go by descending target bit (`order`), so the lowest target bit's two values are
+// neighbouring amplitudes of one thread: fetched as whole sectors by neighbouring lanes and, at
+// bit 0, stored as one (`neighbours`: the output's base allows 32-byte stores). Such a pass took
+// 1.46 times the others' time and takes 1.37 times it; circuits of eight layers on 27 qubits
+// 44.06 -> 43.63 and 41.87 -> 41.18 ms.
+template <typename IT, uint32_t MODE, int NL, bool PO, bool LOW>
 __global__ void __launch_bounds__(CH_THREADS, 1) gate_pair_chain_kernel(void* __restrict__ psiv,
                                                                         const double2* __restrict__ ga,
                                                                         const double2* __restrict__ gb,
@@ -516,7 +533,8 @@ __global__ void __launch_bounds__(CH_THREADS, 1) gate_pair_chain_kernel(void* __
                                                                         const ChainRec* __restrict__ rin,
                                                                         ChainRec* __restrict__ rout, int want_fixed,
                                                                         void* __restrict__ outv,
-                                                                        const BitPerm* __restrict__ perm) {
+                                                                        const BitPerm* __restrict__ perm, uint32_t order,
+                                                                        int neighbours) {
   static_assert(!PO || sizeof(IT) == 4, "permuted output for states of at most 2^32 elements");
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   ChSmem& sm = *reinterpret_cast<ChSmem*>(smem_raw);
@@ -552,7 +570,15 @@ __global__ void __launch_bounds__(CH_THREADS, 1) gate_pair_chain_kernel(void* __
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  for (int t = tid; t < 256; t += CH_THREADS) sm.U16[t] = fused_entry<MODE>(ga, gb, t);
+  // amplitude index bit j of this pass is bit (order >> 4 j) & 15 of the gates' (a0 a1 b0 b1)
+  auto gate_index = [&](int c) {
+    int g = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) g |= ((c >> j) & 1) << ((order >> (4 * j)) & 15u);
+    return g;
+  };
+  for (int t = tid; t < 256; t += CH_THREADS)
+    sm.U16[t] = fused_entry<MODE>(ga, gb, gate_index(t >> 4) * 16 + gate_index(t & 15));
   __syncthreads();
   if (tid < 16) {
     bool ok;
@@ -676,16 +702,35 @@ __global__ void __launch_bounds__(CH_THREADS, 1) gate_pair_chain_kernel(void* __
     uint32_t kk = 0;
 #pragma unroll
     for (int a = 0; a < 4; ++a) kk |= (common ? 0u : (uint32_t)min(62, max_erow - sm.erow[4 * h + a])) << (8 * a);
+    // LOW: lane bit lb takes the place of amplitude index bit 0, so that a load covers both values
+    // of it in 16 of the warp's rows and its lanes read whole sectors
+    const uint32_t lb = p.ins_pos[0], amp0 = (uint32_t)(lane >> lb) & 1u;  // (lb < 3)
+    const int frow = q * 32 + ((lane & ((1 << lb) - 1)) | ((lane >> (lb + 1)) << lb));
+    const IT fbase = LOW ? pair_base<IT>((IT)frow, p) + (IT)p.off[4 * h + amp0] : IT(0);
+    const IT step16 = LOW ? pair_base<IT>((IT)16, p) : IT(0), step2 = (IT)p.off[2];
+    double2* const st = &sm.stage[0][0][0];
+    const int slot0 = chain_slot(4 * h + (int)amp0, frow), slot1 = chain_slot(4 * h + (int)amp0, frow + 16);
     // tile T into stage slot `slot` (its iteration % 2; one commit group per tile, empty past the end)
     auto fetch = [&](uint64_t T, IT tb, uint32_t slot) {
       if (T < ntiles) {
-        const IT gbase = tb | rbase;
+        if (LOW) {
+          const double2* src = psi + (tb | fbase);
+          double2* d = st + slot * (16 * UM_M);
+          cp_async16(d + slot0, src);
+          cp_async16(d + slot1, src + step16);
+          cp_async16(d + 2 * UM_M + slot0, src + step2);
+          cp_async16(d + 2 * UM_M + slot1, src + (step2 + step16));
+        } else {
+          const IT gbase = tb | rbase;
 #pragma unroll
-        for (int c = 4 * h; c < 4 * h + 4; ++c) cp_async16(&sm.stage[slot][c][r], psi + (gbase + (IT)p.off[c]));
+          for (int c = 4 * h; c < 4 * h + 4; ++c) cp_async16(&sm.stage[slot][c][r], psi + (gbase + (IT)p.off[c]));
+        }
       }
       cp_async_commit();
     };
     uint32_t okey = 0, ohi = 0;
+    // amplitudes 4h + a, a even, and 4h + a + 1 are neighbours in the output: stored as one sector
+    const bool pairs = LOW && neighbours != 0;
     // level sums from accumulator set b -> the outputs 4h .. 4h + 3 of group r of the tile
     // whose tile part is tb
     auto recombine = [&](IT tb, uint32_t b) {
@@ -696,6 +741,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) gate_pair_chain_kernel(void* __
 #pragma unroll
       for (int l = 0; l < NL; ++l) tmem_ld8(tbase + (uint32_t)(32 * l), v[l]);
       tmem_wait_ld();
+      int64_t Pr = 0, Pi = 0;  // the outputs of the even amplitude before
 #pragma unroll
       for (int a = 0; a < 4; ++a) {
         float cr[NL], ci[NL];
@@ -716,7 +762,12 @@ __global__ void __launch_bounds__(CH_THREADS, 1) gate_pair_chain_kernel(void* __
             Yr = (Tr + rh) >> k, Yi = (Ti + rh) >> k;
           }
           ohi |= oz::fixed_hi_mag(Yr) | oz::fixed_hi_mag(Yi);  // its bit length is the largest's
-          *reinterpret_cast<longlong2*>(pyo + 2 * (uint64_t)ix) = make_longlong2(Yr, Yi);
+          if (!pairs)
+            *reinterpret_cast<longlong2*>(pyo + 2 * (uint64_t)ix) = make_longlong2(Yr, Yi);
+          else if (a & 1)
+            st_pair(pyo + 2 * (uint64_t)(ix - 1), Pr, Pi, Yr, Yi);
+          else
+            Pr = Yr, Pi = Yi;
         } else {
           const int e = (common ? max_erow : sm.erow[4 * h + a]) + Ein - 2060;
           const double2 vv = make_double2(oz::fixed_to_double(Tr, e), oz::fixed_to_double(Ti, e));
@@ -733,12 +784,14 @@ __global__ void __launch_bounds__(CH_THREADS, 1) gate_pair_chain_kernel(void* __
     bool ok = true;
     for (; tile_of(m) < ntiles; ++m) {
       const uint32_t b = (uint32_t)(m & 1);
-      cp_async_wait_one();  // tile m has landed (tile m + 1 may still be in flight)
+      cp_async_wait_one();  // this thread's copies of tile m have landed (tile m + 1 may be in flight)
+      if (LOW) __syncwarp();  // and the warp's
       double2 x[4];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) x[c] = sm.stage[b][4 * h + c][r];
+      for (int c = 0; c < 4; ++c) x[c] = LOW ? st[b * (16 * UM_M) + chain_slot(4 * h + c, r)] : sm.stage[b][4 * h + c][r];
+      if (LOW) __syncwarp();  // the warp has read its slots
       const IT tb_next2 = tile_part(tile_of(m + 2));
-      fetch(tile_of(m + 2), tb_next2, b);  // only this thread reads its stage slots
+      fetch(tile_of(m + 2), tb_next2, b);  // only this thread (LOW: its warp) reads its stage slots
       // digits of this thread's 8 reals: digit j of amplitude 4h + a as one fp16x2 word (real,
       // imaginary); the four words of digit j fill the thread's core-matrix row
       uint32_t w[4][CH_ND];
@@ -1541,17 +1594,26 @@ void launch_umma(double2* psi, const double2* ga, const double2* gb, const PairP
   }
 }
 
-template <typename IT, int NL, bool PO>
-void launch_chain(void* psi, const double2* ga, const double2* gb, const PairParams& p, cudaStream_t s,
-                  const ChainRec* rin, ChainRec* rout, bool want_fixed, void* out, const BitPerm* perm) {
+template <typename IT, int NL, bool PO, bool LOW>
+void launch_chain_form(void* psi, const double2* ga, const double2* gb, const PairParams& p, cudaStream_t s,
+                  const ChainRec* rin, ChainRec* rout, bool want_fixed, void* out, const BitPerm* perm, uint32_t order,
+                  bool neighbours) {
   const size_t smem = sizeof(ChSmem);
-  check_cuda(cudaFuncSetAttribute(gate_pair_chain_kernel<IT, PAIR_KRON, NL, PO>,
+  check_cuda(cudaFuncSetAttribute(gate_pair_chain_kernel<IT, PAIR_KRON, NL, PO, LOW>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
              "gate_pair_chain_kernel shared memory");
   const uint64_t ntiles = p.ngroups / UM_M;
   const int grid = (int)std::min<uint64_t>(ntiles, (uint64_t)sm_count());  // one CTA per SM (all its TMEM)
-  gate_pair_chain_kernel<IT, PAIR_KRON, NL, PO>
-      <<<grid, CH_THREADS, smem, s>>>(psi, ga, gb, p, rin, rout, want_fixed ? 1 : 0, out, perm);
+  gate_pair_chain_kernel<IT, PAIR_KRON, NL, PO, LOW>
+      <<<grid, CH_THREADS, smem, s>>>(psi, ga, gb, p, rin, rout, want_fixed ? 1 : 0, out, perm, order, neighbours ? 1 : 0);
+}
+
+template <typename IT, int NL, bool PO>
+void launch_chain(void* psi, const double2* ga, const double2* gb, const PairParams& p, cudaStream_t s,
+                  const ChainRec* rin, ChainRec* rout, bool want_fixed, void* out, const BitPerm* perm, uint32_t order,
+                  bool neighbours, bool low) {
+  if (low) launch_chain_form<IT, NL, PO, true>(psi, ga, gb, p, s, rin, rout, want_fixed, out, perm, order, neighbours);
+  else launch_chain_form<IT, NL, PO, false>(psi, ga, gb, p, s, rin, rout, want_fixed, out, perm, order, neighbours);
 }
 
 int chain_levels() {
@@ -1566,8 +1628,32 @@ int chain_levels() {
 
 bool chain_applies(const PairParams& p) { return p.ngroups >= (uint64_t)UM_M && p.ngroups % UM_M == 0; }
 
-void launch_pair_chain(void* psi, const double2* ga, const double2* gb, const PairParams& p, cudaStream_t s,
-                       const ChainRec* rin, ChainRec* rout, bool want_fixed, void* out, const BitPerm* perm) {
+void launch_pair_chain(void* psi, const double2* ga, const double2* gb, const PairParams& gp, cudaStream_t s,
+                       const ChainRec* rin, ChainRec* rout, bool want_fixed, void* out, const BitPerm* gperm) {
+  // LOW form only where it gains: the exchange between the lanes of a warp costs the other passes
+  // 4 % (all passes in this form: 28 qubits 84.5 ms against 81.2; by this rule 80.6)
+  const bool low = gp.ins_pos[0] == 0 || (gp.ins_pos[0] == 1 && gp.ins_pos[1] == 2);
+  // amplitude index bits by descending target bit: bit j of the pass is target bit ins_pos[j]
+  PairParams p = gp;
+  uint32_t order = low ? 0 : 0x3210;
+  for (int j = 0; low && j < 4; ++j)
+    for (uint32_t b = 0; b < 4; ++b)
+      if ((uint64_t)gp.off[1 << b] == 1ull << gp.ins_pos[j]) order |= b << (4 * j);
+  auto gate_index = [&](int c) {
+    int g = 0;
+    for (int j = 0; j < 4; ++j) g |= ((c >> j) & 1) << ((order >> (4 * j)) & 15u);
+    return g;
+  };
+  for (int c = 0; c < 16; ++c) p.off[c] = gp.off[gate_index(c)];
+  BitPerm permuted;
+  const BitPerm* perm = nullptr;
+  if (gperm) {
+    permuted = *gperm;
+    for (int c = 0; c < 16; ++c) permuted.poff[c] = gperm->poff[gate_index(c)];
+    perm = &permuted;
+  }
+  // the two amplitudes of index bit 0 are neighbours where they are stored, at whole sectors
+  const bool nb = (perm ? perm->poff[1] == 1 : p.off[1] == 1) && ((uintptr_t)(perm ? out : psi) & 31) == 0;
   const bool i32 = p.ngroups * 16 <= (1ull << 32);
   if (perm) {
     if (!i32 || !out || out == psi) throw Error(QTNH_ERR_UNSUPPORTED, "permuted chain output");
@@ -1576,9 +1662,9 @@ void launch_pair_chain(void* psi, const double2* ga, const double2* gb, const Pa
     cudaError_t e = cudaMemcpyAsync(dperm, perm, sizeof(BitPerm), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) {
       if (chain_levels() == 6)
-        launch_chain<uint32_t, 6, true>(psi, ga, gb, p, s, rin, rout, want_fixed, out, dperm);
+        launch_chain<uint32_t, 6, true>(psi, ga, gb, p, s, rin, rout, want_fixed, out, dperm, order, nb, low);
       else
-        launch_chain<uint32_t, 7, true>(psi, ga, gb, p, s, rin, rout, want_fixed, out, dperm);
+        launch_chain<uint32_t, 7, true>(psi, ga, gb, p, s, rin, rout, want_fixed, out, dperm, order, nb, low);
       e = cudaGetLastError();
     }
     workspace_free(dperm, s);
@@ -1587,14 +1673,14 @@ void launch_pair_chain(void* psi, const double2* ga, const double2* gb, const Pa
   }
   if (chain_levels() == 6) {
     if (i32)
-      launch_chain<uint32_t, 6, false>(psi, ga, gb, p, s, rin, rout, want_fixed, nullptr, nullptr);
+      launch_chain<uint32_t, 6, false>(psi, ga, gb, p, s, rin, rout, want_fixed, nullptr, nullptr, order, nb, low);
     else
-      launch_chain<uint64_t, 6, false>(psi, ga, gb, p, s, rin, rout, want_fixed, nullptr, nullptr);
+      launch_chain<uint64_t, 6, false>(psi, ga, gb, p, s, rin, rout, want_fixed, nullptr, nullptr, order, nb, low);
   } else {
     if (i32)
-      launch_chain<uint32_t, 7, false>(psi, ga, gb, p, s, rin, rout, want_fixed, nullptr, nullptr);
+      launch_chain<uint32_t, 7, false>(psi, ga, gb, p, s, rin, rout, want_fixed, nullptr, nullptr, order, nb, low);
     else
-      launch_chain<uint64_t, 7, false>(psi, ga, gb, p, s, rin, rout, want_fixed, nullptr, nullptr);
+      launch_chain<uint64_t, 7, false>(psi, ga, gb, p, s, rin, rout, want_fixed, nullptr, nullptr, order, nb, low);
   }
 }
 
