@@ -129,10 +129,11 @@ void zgemm(const c128* A, const c128* B, c128* C, uint64_t M, uint64_t N, uint64
   // tiles) 261 / 262 on either, 2048 x 2048 1784 in tiles.
   const uint64_t sms = (uint64_t)sm_count(), waves = (gx * gy + sms - 1) / sms;
   if (10 * (M * N) < 9 * (waves * sms * BM * BN)) {
-    // as many outputs a block as leaves every SM one, at most 64 (coalesced loads of B); no more
-    // threads an output than K has terms
-    int out_log2 = 6;
-    while (out_log2 > 0 && (M * N) >> out_log2 < sms && (256ull >> out_log2) < K) --out_log2;
+    // as many outputs a block as leaves every SM one, at most 64 (coalesced loads of B), but no
+    // thread with fewer than 8 terms: the sums of shorter chains round more often than one
+    // chain does (K 2 to 8 in four parts: 1.4 times its error), longer ones less
+    int out_log2 = 8;
+    while (out_log2 > 0 && (out_log2 > 6 || (M * N) >> out_log2 < sms) && (512ull >> out_log2) * 8 <= K) --out_log2;
     const uint64_t blocks = (M * N + (1ull << out_log2) - 1) >> out_log2;
     if (blocks < (1ull << 31)) {
       zgemm_spread_kernel<<<(unsigned)blocks, 256, 0, s>>>(A, B, C, M, N, K, out_log2);
