@@ -1175,7 +1175,8 @@ __device__ __noinline__ bool chain_team_pass(IT rbase, IT tb, uint32_t sc) {
         ohi |= oz::fixed_hi_mag(Tr) | oz::fixed_hi_mag(Ti);  // its bit length is the largest's
         static_cast<longlong2*>(out)[ix] = make_longlong2(Tr, Ti);
       } else {
-        const int e = gd.max_erow - (int)((kk >> (8 * a)) & 0xFFu) + chain_scale_ein(sc) - 2060;
+        // (the row's own exponent: kk is a shift, held below 63, and rows may lie further apart)
+        const int e = (common ? gd.max_erow : gd.erow[4 * h + a]) + chain_scale_ein(sc) - 2060;
         const double2 vv = make_double2(oz::fixed_to_double(Tr, e), oz::fixed_to_double(Ti, e));
         okey = max(okey, amp_key(vv));
         static_cast<double2*>(out)[ix] = vv;
