@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(256) rdm4_sum_kernel(const double* __restrict_
   if (e >= 120) {
     const int d = im ? b : a;
     rho[2 * (17 * d)] = s;
-    rho[2 * (17 * d) + 1] = 0.0;
+    rho[2 * (17 * d) + 1] = s - s;  // 0; NaN where the state holds an infinity or a NaN, as its product is
   } else {
     rho[2 * (16 * a + b) + im] = s;
     rho[2 * (16 * b + a) + im] = im ? -s : s;
