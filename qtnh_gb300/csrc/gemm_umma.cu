@@ -28,15 +28,13 @@
 // the two TMEM accumulators and commits the stage back to the producer, and warps 2-9
 // read the finished accumulators (tcgen05.ld) into registers, free them, and then store
 // the FP32 partials or (one slice) pair the Re/Im rows with a shuffle and store complex128.
-// A K-step takes the tensor cores 768 cycles, in which 36 KB per SM from L2 is more than L2
-// gives all SMs; so where the row tiles are even in number two CTAs form a cluster, take
-// neighbouring row tiles and load half of B's blocks each into both (24 KB from L2). Measured
-// at M 4096, N 4096, K 2048: 880 us, what cuBLAS's rate allows for the operations is 873;
-// without pairs and with four epilogue warps that stored before freeing 1047 us. The
-// partials' sum is 255 us more (1.3 GB, 5.2 TB/s); summing a tile's slices inside this
-// kernel as they become complete took 1055 us in all instead of 880 + 255, for the whole
-// contraction 1312 us against 1340: not worth its code. Every wait is bounded by a clock
-// limit (device error flags).
+// Measured at M 4096, N 4096, K 2048: 864 us, what cuBLAS's rate allows for the operations is 873;
+// with four epilogue warps that stored before freeing 1032 us. Pairs of CTAs that share B's
+// blocks (one MMA of M 256 over both) take 858 us there, but 2 us more than single ones wherever
+// a CTA has fewer than seven tiles (26 us instead of 24 at 64 tiles, 43 instead of 40 at 256): not worth
+// their code. The partials' sum is 255 us more (1.3 GB, 5.2 TB/s); summing a tile's slices
+// inside this kernel as they become complete took 1055 us in all: not worth its code
+// either. Every wait is bounded by a clock limit (device error flags).
 
 #include <cuda_bf16.h>
 
@@ -88,6 +86,7 @@ struct GmSmem {
   uint64_t empty[GM_STAGES];                 // stage consumed by the MMAs
   uint64_t tfull;                            // accumulators complete
   uint64_t tempty;                           // accumulators read by the epilogue
+  uint64_t last;                             // all MMAs issued are complete (after an expired wait)
   uint32_t tmem_base;
   int abort;
 };
@@ -144,23 +143,6 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
       : "memory");
 }
 
-// The same into this CTA and the other one of the pair, at the same offsets.
-__device__ __forceinline__ void bulk_g2s_pair(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.multicast::cluster [%0], [%1], %2, [%3], "
-      "%4;" ::"r"(smem_u32(dst)),
-      "l"(src), "r"(bytes), "r"(smem_u32(bar)), "h"((uint16_t)3)
-      : "memory");
-}
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
@@ -185,15 +167,6 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
                : "memory");
 }
 
-// The arrival in both CTAs of the pair.
-__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
-  asm volatile(
-      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
-          smem_u32(bar)),
-      "h"((uint16_t)3)
-      : "memory");
-}
-
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
@@ -213,20 +186,15 @@ __device__ __forceinline__ void store_sector(float* dst, const uint32_t* v) {
                : "memory");
 }
 
-// PAIR: the two CTAs of a cluster take neighbouring row tiles of one column tile and share B's
-// blocks: each loads half of every block into both.
-template <bool PAIR>
 __global__ void __launch_bounds__(GM_THREADS, 1) gemm_bf16x3_umma_kernel(const __grid_constant__ GemmParams p) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   GmSmem& sm = *reinterpret_cast<GmSmem*>(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  constexpr uint32_t CL = PAIR ? 2 : 1;
-  const uint32_t rank = PAIR ? cluster_rank() : 0;
-  const uint64_t ntiles = (uint64_t)(p.MT / CL) * p.NT * p.S, first = blockIdx.x / CL, stride = gridDim.x / CL;
-  // tile (of the pair) -> (row tile, column tile, K-slice), row tiles fastest (neighbours share B)
+  const uint64_t ntiles = (uint64_t)p.MT * p.NT * p.S;
+  // tile -> (row tile, column tile, K-slice), row tiles fastest (neighbours share B)
   auto tile_coords = [&](uint64_t tile, uint64_t& mt, uint64_t& nt, uint32_t& k0, uint32_t& k1) {
-    mt = tile % (p.MT / CL) * CL + rank;
-    const uint64_t rest = tile / (p.MT / CL);
+    mt = tile % p.MT;
+    const uint64_t rest = tile / p.MT;
     nt = rest % p.NT;
     const uint32_t sl = (uint32_t)(rest / p.NT);
     k0 = sl * p.SK;
@@ -237,10 +205,11 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_bf16x3_umma_kernel(const _
     sm.abort = 0;
     for (int s = 0; s < GM_STAGES; ++s) {
       mbar_init(&sm.full[s], 1);
-      mbar_init(&sm.empty[s], CL);
+      mbar_init(&sm.empty[s], 1);
     }
     mbar_init(&sm.tfull, 1);
     mbar_init(&sm.tempty, GM_EPI_WARPS);
+    mbar_init(&sm.last, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -251,7 +220,6 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_bf16x3_umma_kernel(const _
   }
   tc_fence_before();
   __syncthreads();
-  if (PAIR) cluster_sync_all();  // the other CTA's barriers are ready
   tc_fence_after();
   const uint32_t tmem = sm.tmem_base;
 
@@ -260,7 +228,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_bf16x3_umma_kernel(const _
     if (lane == 0) {
       uint32_t it = 0;
       bool ok = true;
-      for (uint64_t tile = first; ok && tile < ntiles; tile += stride) {
+      for (uint64_t tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x) {
         uint64_t mt, nt;
         uint32_t k0, k1;
         tile_coords(tile, mt, nt, k0, k1);
@@ -280,14 +248,9 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_bf16x3_umma_kernel(const _
           for (int pl = 0; pl < GM_P; ++pl)
             bulk_g2s(&sm.stage[s][pl * GM_A_BLOCK], p.a_planes + pl * p.a_plane_bytes + ablk, GM_A_BLOCK, &sm.full[s]);
 #pragma unroll
-          for (int pl = 0; pl < GM_P; ++pl) {
-            uint8_t* dst = &sm.stage[s][GM_P * GM_A_BLOCK + pl * GM_B_BLOCK];
-            const uint8_t* src = p.b_planes + pl * p.b_plane_bytes + bblk;
-            if (PAIR)
-              bulk_g2s_pair(dst + rank * (GM_B_BLOCK / 2), src + rank * (GM_B_BLOCK / 2), GM_B_BLOCK / 2, &sm.full[s]);
-            else
-              bulk_g2s(dst, src, GM_B_BLOCK, &sm.full[s]);
-          }
+          for (int pl = 0; pl < GM_P; ++pl)
+            bulk_g2s(&sm.stage[s][GM_P * GM_A_BLOCK + pl * GM_B_BLOCK], p.b_planes + pl * p.b_plane_bytes + bblk,
+                     GM_B_BLOCK, &sm.full[s]);
         }
       }
     }
@@ -296,10 +259,11 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_bf16x3_umma_kernel(const _
     if (lane == 0) {
       uint32_t it = 0, lt = 0;
       bool ok = true;
-      for (uint64_t tile = first; ok && tile < ntiles; tile += stride, ++lt) {
+      for (uint64_t tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x, ++lt) {
         if (!mbar_wait_thread(&sm.tempty, (lt & 1u) ^ 1u, &sm.abort)) {
           atomicOr(&g_gemm_error, 2u);
           sm.abort = 1;
+          ok = false;
           break;
         }
         tc_fence_after();
@@ -327,11 +291,16 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_bf16x3_umma_kernel(const _
             else
               umma_bf16(d2, ad, bd, (ks > k0 || q > 1) ? 1u : 0u);
           }
-          // the stage is free once these MMAs (and the other CTA's) have read it
-          if (PAIR) umma_commit_pair(&sm.empty[s]);
-          else umma_commit(&sm.empty[s]);
+          umma_commit(&sm.empty[s]);  // the stage is free once these MMAs have read it
         }
         if (ok) umma_commit(&sm.tfull);
+      }
+      // stopped early: the MMAs issued finish before tensor memory is freed (limited as well)
+      if (!ok) {
+        umma_commit(&sm.last);
+        const long long t0 = clock64();
+        while (!mbar_try_wait(&sm.last, 0) && clock64() - t0 < (1 << 20)) {
+        }
       }
     }
   } else {
@@ -340,7 +309,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_bf16x3_umma_kernel(const _
     const int q = warp & 3, h = (warp - 2) >> 2, r = q * 32 + lane;
     constexpr int CW = GM_N / (GM_EPI_WARPS / 4), NCH = CW / 32;
     uint32_t lt = 0;
-    for (uint64_t tile = first; tile < ntiles; tile += stride, ++lt) {
+    for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++lt) {
       if (!mbar_wait_warp(&sm.tfull, lt & 1u, &sm.abort)) {
         atomicOr(&g_gemm_error, 4u);
         sm.abort = 1;
@@ -402,8 +371,6 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_bf16x3_umma_kernel(const _
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(GM_TMEM_COLS) : "memory");
   }
-  __syncwarp();
-  if (PAIR) cluster_sync_all();  // neither CTA leaves while the other may still copy or arrive here
 }
 
 using bx3::pieces;
@@ -568,14 +535,9 @@ static void gemm_core(const Prep& pa, const Prep& pb, void* Cv, uint64_t M, uint
       count_launch();
     }
     const size_t smem = sizeof(GmSmem);
-    // two CTAs share B where every row tile has a partner (with an odd number the last pair would
-    // work on padding; one in 64 rows of C either way)
-    const bool pair = p.MT % 2 == 0;
-    const auto kernel = pair ? gemm_bf16x3_umma_kernel<true> : gemm_bf16x3_umma_kernel<false>;
-    check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+    check_cuda(cudaFuncSetAttribute(gemm_bf16x3_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                "gemm_bf16x3_umma_kernel shared memory");
-    const uint64_t sms = pair ? (uint64_t)sm_count() & ~1ull : (uint64_t)sm_count();
-    const int grid = (int)std::min<uint64_t>((uint64_t)p.MT * p.NT * p.S, sms);
+    const int grid = (int)std::min<uint64_t>((uint64_t)p.MT * p.NT * p.S, (uint64_t)sm_count());
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     {
       std::lock_guard<std::mutex> lk(g_timing_mu);
@@ -585,18 +547,7 @@ static void gemm_core(const Prep& pa, const Prep& pb, void* Cv, uint64_t M, uint
         check_cuda(cudaEventRecord(e0, s), "event record");
       }
     }
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = pair ? 2 : 1;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(GM_THREADS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    check_cuda(cudaLaunchKernelEx(&cfg, kernel, p), "gemm_bf16x3_umma_kernel launch");
+    gemm_bf16x3_umma_kernel<<<grid, GM_THREADS, smem, s>>>(p);
     if (e0) {
       check_cuda(cudaEventRecord(e1, s), "event record");
       std::lock_guard<std::mutex> lk(g_timing_mu);
