@@ -108,6 +108,7 @@ struct OgSmem {
   uint64_t empty[OG_STAGES];
   uint64_t tfull;   // a chunk's level sums are complete
   uint64_t tempty[OG_L];  // the epilogue has drained a level
+  uint64_t last;          // all MMAs issued are complete (after an expired wait)
   uint32_t tmem_base;
   int abort;
 };
@@ -138,6 +139,13 @@ __device__ __forceinline__ bool mbar_wait_thread(uint64_t* bar, uint32_t parity,
     if (*abort != 0 || clock64() - t0 > OG_WAIT_CYCLES) return false;
   }
   return true;
+}
+// After an expired wait: gives the copies of the stages in flight time to land (~0.5 ms at most).
+__device__ __forceinline__ void mbar_drain(uint64_t* full, uint32_t it) {
+  const long long t0 = clock64();
+  for (uint32_t x = it > (uint32_t)OG_STAGES ? it - OG_STAGES : 0; x < it; ++x)
+    while (!mbar_try_wait(&full[x % OG_STAGES], (x / OG_STAGES) & 1u) && clock64() - t0 < (1 << 20)) {
+    }
 }
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort) {
   const long long t0 = clock64();
@@ -231,6 +239,7 @@ __global__ void __launch_bounds__(OG_THREADS, 1) gemm_oz6_umma_kernel(const __gr
     }
     mbar_init(&sm.tfull, 1);
     for (int l = 0; l < OG_L; ++l) mbar_init(&sm.tempty[l], OG_EPI_WARPS);
+    mbar_init(&sm.last, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -259,6 +268,7 @@ __global__ void __launch_bounds__(OG_THREADS, 1) gemm_oz6_umma_kernel(const __gr
             atomicOr(&g_ozg_error, 1u);
             sm.abort = 1;
             ok = false;
+            mbar_drain(sm.full, it);
             break;
           }
           mbar_arrive_expect_tx(&sm.full[s], (uint32_t)OG_STAGE);
@@ -325,6 +335,13 @@ __global__ void __launch_bounds__(OG_THREADS, 1) gemm_oz6_umma_kernel(const __gr
             break;
           }
           umma_commit(&sm.tfull);
+        }
+      }
+      // stopped early: the MMAs issued finish before tensor memory is freed (limited as well)
+      if (!ok) {
+        umma_commit(&sm.last);
+        const long long t0 = clock64();
+        while (!mbar_try_wait(&sm.last, 0) && clock64() - t0 < (1 << 20)) {
         }
       }
     }
