@@ -482,15 +482,15 @@ bool apply_gate_runs_tc(void* state, void* scratch, dims_t dims, const std::vect
             bool fuse = false;
             if (resident) {
               ChainStep c{sk.p, gate_ptr(sk.g), gate_ptr(sk.g + 1), k + 1 < R, false, {}};
-              fuse = c.perm = next && make_bit_map(next->dims, runs[(size_t)next->perm].ptup, c.dst);
+              fuse = c.perm = next && make_bit_map(next->dims, runs[(size_t)next->perm].ptup, c.map);
               open.push_back(c);
               if ((int)open.size() == chain_resident_passes()) flush();
             } else {
-              BitPerm bp;
-              fuse = next && make_bit_perm(next->dims, runs[(size_t)next->perm].ptup, sk.p, bp);
+              BitMap map;
+              fuse = next && make_bit_map(next->dims, runs[(size_t)next->perm].ptup, map);
               timed_pass(s, 1, [&] {
                 launch_pair_chain(cur, gate_ptr(sk.g), gate_ptr(sk.g + 1), sk.p, s, &recs[k - 1], &recs[k], k + 1 < R,
-                                  fuse ? oth : nullptr, fuse ? &bp : nullptr);
+                                  fuse ? oth : nullptr, fuse ? &map : nullptr);
               });
               count_launch();
               if (fuse) std::swap(cur, oth);

@@ -476,12 +476,22 @@ struct ChSmem {
   int gate_ok;
   int abort;
   int no_abort;                         // stays 0: the final wait for in-flight MMAs
-  uint32_t ptab[4][256];                // PO: the permutation's bit tables (BitPerm)
+  uint32_t ptab[4][256];                // PO: the permutation's byte tables
   uint32_t poff[16];                    // PO: the permuted amplitude offsets
 };
 static_assert(CH_NLMAX * UM_N <= (int)CH_ACC, "chain level sums exceed an accumulator set");
 static_assert(2 * CH_ACC <= CH_TMEM_COLS, "two accumulator sets");
 static_assert(sizeof(ChSmem) + 1024 <= 227 * 1024, "chain shared memory");
+
+// The image under `map` of byte `byte` of an element index having the value v.
+__device__ __forceinline__ uint32_t byte_image(const BitMap& map, int byte, int v) {
+  uint32_t x = 0;
+  for (int j = 0; j < 8; ++j) {
+    const uint32_t d = map.dst[8 * byte + j];
+    if (((v >> j) & 1) && d < 32) x |= 1u << d;
+  }
+  return x;
+}
 
 // Stage slot of amplitude c of row r: rows of odd amplitudes four off, so that neither the
 // fetch in either order nor the reads meet bank conflicts.
@@ -533,7 +543,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) gate_pair_chain_kernel(void* __
                                                                         const ChainRec* __restrict__ rin,
                                                                         ChainRec* __restrict__ rout, int want_fixed,
                                                                         void* __restrict__ outv,
-                                                                        const BitPerm* __restrict__ perm, uint32_t order,
+                                                                        const __grid_constant__ BitMap perm, uint32_t order,
                                                                         int neighbours) {
   static_assert(!PO || sizeof(IT) == 4, "permuted output for states of at most 2^32 elements");
   extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -545,8 +555,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) gate_pair_chain_kernel(void* __
   double2* pso = static_cast<double2*>(PO ? outv : psiv);  // where the outputs go
   int64_t* pyo = static_cast<int64_t*>(PO ? outv : psiv);
   if (PO) {
-    for (int t = tid; t < 4 * 256; t += CH_THREADS) (&sm.ptab[0][0])[t] = (&perm->tab[0][0])[t];
-    if (tid < 16) sm.poff[tid] = perm->poff[tid];
+    for (int t = tid; t < 4 * 256; t += CH_THREADS) sm.ptab[t >> 8][t & 255] = byte_image(perm, t >> 8, t & 255);
   }
   // the image of a (tile or row) part of an element index under the permutation
   auto pimg = [&](uint32_t x) -> uint32_t {
@@ -585,6 +594,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) gate_pair_chain_kernel(void* __
     const uint32_t e = row_exponent(sm.U16, tid, ok);
     sm.erow[tid] = (int32_t)e;
     if (!ok) sm.gate_ok = 0;
+    if (PO) sm.poff[tid] = pimg((uint32_t)p.off[tid]);
   }
   __syncthreads();
   int max_erow = 0, min_erow = 0x7FFFFFFF;
@@ -926,7 +936,7 @@ struct ChainPrepParams {
   const double2* ga[CR_MAXP];
   const double2* gb[CR_MAXP];
   uint8_t mode[CR_MAXP];                // PairGate
-  uint8_t dst[CR_MAXP][32];             // permutation: output bit of every index bit (32: none)
+  BitMap map[CR_MAXP];                  // permutations
 };
 
 // A pass of one launch of the chain kernel (kernel parameter).
@@ -952,15 +962,7 @@ __global__ void __launch_bounds__(128) chain_prep_kernel(const __grid_constant__
   if ((int)blockIdx.x >= npass) {
     const int k = (int)blockIdx.x - npass;
     uint32_t* tab = ptabs + (size_t)k * 1024;
-    for (int t = tid; t < 1024; t += 128) {
-      const int byte = t >> 8, v = t & 255;
-      uint32_t x = 0;
-      for (int j = 0; j < 8; ++j) {
-        const uint32_t d = q.dst[k][8 * byte + j];
-        if (((v >> j) & 1) && d < 32) x |= 1u << d;
-      }
-      tab[t] = x;
-    }
+    for (int t = tid; t < 1024; t += 128) tab[t] = byte_image(q.map[k], t >> 8, t & 255);
     return;
   }
   __shared__ double2 U16[256];
@@ -1597,7 +1599,7 @@ void launch_umma(double2* psi, const double2* ga, const double2* gb, const PairP
 
 template <typename IT, int NL, bool PO, bool LOW>
 void launch_chain_form(void* psi, const double2* ga, const double2* gb, const PairParams& p, cudaStream_t s,
-                  const ChainRec* rin, ChainRec* rout, bool want_fixed, void* out, const BitPerm* perm, uint32_t order,
+                  const ChainRec* rin, ChainRec* rout, bool want_fixed, void* out, const BitMap& perm, uint32_t order,
                   bool neighbours) {
   const size_t smem = sizeof(ChSmem);
   check_cuda(cudaFuncSetAttribute(gate_pair_chain_kernel<IT, PAIR_KRON, NL, PO, LOW>,
@@ -1611,7 +1613,7 @@ void launch_chain_form(void* psi, const double2* ga, const double2* gb, const Pa
 
 template <typename IT, int NL, bool PO>
 void launch_chain(void* psi, const double2* ga, const double2* gb, const PairParams& p, cudaStream_t s,
-                  const ChainRec* rin, ChainRec* rout, bool want_fixed, void* out, const BitPerm* perm, uint32_t order,
+                  const ChainRec* rin, ChainRec* rout, bool want_fixed, void* out, const BitMap& perm, uint32_t order,
                   bool neighbours, bool low) {
   if (low) launch_chain_form<IT, NL, PO, true>(psi, ga, gb, p, s, rin, rout, want_fixed, out, perm, order, neighbours);
   else launch_chain_form<IT, NL, PO, false>(psi, ga, gb, p, s, rin, rout, want_fixed, out, perm, order, neighbours);
@@ -1630,7 +1632,7 @@ int chain_levels() {
 bool chain_applies(const PairParams& p) { return p.ngroups >= (uint64_t)UM_M && p.ngroups % UM_M == 0; }
 
 void launch_pair_chain(void* psi, const double2* ga, const double2* gb, const PairParams& gp, cudaStream_t s,
-                       const ChainRec* rin, ChainRec* rout, bool want_fixed, void* out, const BitPerm* gperm) {
+                       const ChainRec* rin, ChainRec* rout, bool want_fixed, void* out, const BitMap* perm) {
   // LOW form only where it gains: the exchange between the lanes of a warp costs the other passes
   // 4 % (all passes in this form: 28 qubits 84.5 ms against 81.2; by this rule 80.6)
   const bool low = gp.ins_pos[0] == 0 || (gp.ins_pos[0] == 1 && gp.ins_pos[1] == 2);
@@ -1646,42 +1648,27 @@ void launch_pair_chain(void* psi, const double2* ga, const double2* gb, const Pa
     return g;
   };
   for (int c = 0; c < 16; ++c) p.off[c] = gp.off[gate_index(c)];
-  BitPerm permuted;
-  const BitPerm* perm = nullptr;
-  if (gperm) {
-    permuted = *gperm;
-    for (int c = 0; c < 16; ++c) permuted.poff[c] = gperm->poff[gate_index(c)];
-    perm = &permuted;
-  }
   // the two amplitudes of index bit 0 are neighbours where they are stored, at whole sectors
-  const bool nb = (perm ? perm->poff[1] == 1 : p.off[1] == 1) && ((uintptr_t)(perm ? out : psi) & 31) == 0;
+  const bool nb = (perm ? p.off[1] == 1ll << gp.ins_pos[0] && perm->dst[gp.ins_pos[0]] == 0 : p.off[1] == 1) && ((uintptr_t)(perm ? out : psi) & 31) == 0;
   const bool i32 = p.ngroups * 16 <= (1ull << 32);
   if (perm) {
     if (!i32 || !out || out == psi) throw Error(QTNH_ERR_UNSUPPORTED, "permuted chain output");
-    // the tables travel in stream-ordered workspace, freed after the launch
-    BitPerm* dperm = static_cast<BitPerm*>(workspace_alloc(sizeof(BitPerm), s));
-    cudaError_t e = cudaMemcpyAsync(dperm, perm, sizeof(BitPerm), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) {
-      if (chain_levels() == 6)
-        launch_chain<uint32_t, 6, true>(psi, ga, gb, p, s, rin, rout, want_fixed, out, dperm, order, nb, low);
-      else
-        launch_chain<uint32_t, 7, true>(psi, ga, gb, p, s, rin, rout, want_fixed, out, dperm, order, nb, low);
-      e = cudaGetLastError();
-    }
-    workspace_free(dperm, s);
-    check_cuda(e, "permuted chain launch");
+    if (chain_levels() == 6)
+      launch_chain<uint32_t, 6, true>(psi, ga, gb, p, s, rin, rout, want_fixed, out, *perm, order, nb, low);
+    else
+      launch_chain<uint32_t, 7, true>(psi, ga, gb, p, s, rin, rout, want_fixed, out, *perm, order, nb, low);
     return;
   }
   if (chain_levels() == 6) {
     if (i32)
-      launch_chain<uint32_t, 6, false>(psi, ga, gb, p, s, rin, rout, want_fixed, nullptr, nullptr, order, nb, low);
+      launch_chain<uint32_t, 6, false>(psi, ga, gb, p, s, rin, rout, want_fixed, nullptr, BitMap(), order, nb, low);
     else
-      launch_chain<uint64_t, 6, false>(psi, ga, gb, p, s, rin, rout, want_fixed, nullptr, nullptr, order, nb, low);
+      launch_chain<uint64_t, 6, false>(psi, ga, gb, p, s, rin, rout, want_fixed, nullptr, BitMap(), order, nb, low);
   } else {
     if (i32)
-      launch_chain<uint32_t, 7, false>(psi, ga, gb, p, s, rin, rout, want_fixed, nullptr, nullptr, order, nb, low);
+      launch_chain<uint32_t, 7, false>(psi, ga, gb, p, s, rin, rout, want_fixed, nullptr, BitMap(), order, nb, low);
     else
-      launch_chain<uint64_t, 7, false>(psi, ga, gb, p, s, rin, rout, want_fixed, nullptr, nullptr, order, nb, low);
+      launch_chain<uint64_t, 7, false>(psi, ga, gb, p, s, rin, rout, want_fixed, nullptr, BitMap(), order, nb, low);
   }
 }
 
@@ -1718,7 +1705,7 @@ void launch_chain_resident(void* cur, void* oth, const std::vector<ChainStep>& s
     pp.perm = -1;
     if (st.perm) {
       if (!oth || oth == cur) throw Error(QTNH_ERR_UNSUPPORTED, "permuted chain output");
-      std::memcpy(q.dst[nperm], st.dst, sizeof(st.dst));
+      q.map[nperm] = st.map;
       pp.perm = (int16_t)nperm++;
     }
   }
@@ -1756,10 +1743,7 @@ void launch_chain_resident(void* cur, void* oth, const std::vector<ChainStep>& s
 bool chain_resident(const PairParams& p) { return chain_applies(p) && p.ngroups * 16 <= CHAIN_RESIDENT_AMPS; }
 int chain_resident_passes() { return CR_MAXP; }
 
-// dst[b]: the output bit of index bit b under the permutation ptup (Tensor::permute
-// convention) of a state of dims `dims`, 32 for bits above the state; false if the dims are
-// not all powers of two or the state has more than 2^32 elements.
-bool make_bit_map(const dims_t& dims, const std::vector<uint16_t>& ptup, uint8_t dst[32]) {
+bool make_bit_map(const dims_t& dims, const std::vector<uint16_t>& ptup, BitMap& map) {
   const size_t r = dims.size();
   if (ptup.size() != r) return false;
   uint32_t total = 0;
@@ -1779,26 +1763,9 @@ bool make_bit_map(const dims_t& dims, const std::vector<uint16_t>& ptup, uint8_t
   for (size_t i = r; i-- > 0;) in_lo[i] = acc, acc += w[i];
   acc = 0;
   for (size_t j = r; j-- > 0;) out_lo[j] = acc, acc += log2_or_none(nd[j]);
-  for (int b = 0; b < 32; ++b) dst[b] = 32;  // bits above the state: never set
+  for (int b = 0; b < 32; ++b) map.dst[b] = 32;  // bits above the state: never set
   for (size_t i = 0; i < r; ++i)
-    for (uint32_t k = 0; k < w[i]; ++k) dst[in_lo[i] + k] = (uint8_t)(out_lo[ptup[i]] + k);
-  return true;
-}
-
-bool make_bit_perm(const dims_t& dims, const std::vector<uint16_t>& ptup, const PairParams& p, BitPerm& bp) {
-  uint8_t dst[32];
-  if (!make_bit_map(dims, ptup, dst)) return false;
-  for (int t = 0; t < 4; ++t)
-    for (int v = 0; v < 256; ++v) {
-      uint32_t x = 0;
-      for (int k = 0; k < 8; ++k)
-        if (((v >> k) & 1) && dst[8 * t + k] < 32) x |= 1u << dst[8 * t + k];
-      bp.tab[t][v] = x;
-    }
-  for (int c = 0; c < 16; ++c) {
-    const uint32_t o = (uint32_t)p.off[c];
-    bp.poff[c] = bp.tab[0][o & 255u] | bp.tab[1][(o >> 8) & 255u] | bp.tab[2][(o >> 16) & 255u] | bp.tab[3][o >> 24];
-  }
+    for (uint32_t k = 0; k < w[i]; ++k) map.dst[in_lo[i] + k] = (uint8_t)(out_lo[ptup[i]] + k);
   return true;
 }
 
