@@ -152,6 +152,11 @@ void launch_pair_chain(void* psi, const double2* ga, const double2* gb, const Pa
 // 2^21, 1.61 / 1.41 at 2^22, 2.78 / 2.76 at 2^23, 4.90 / 4.99 at 2^24, 19.1 / 20.0 at 2^26
 // (from DRAM the launch per pass, whose CTAs run more out of step, streams faster).
 constexpr uint64_t CHAIN_RESIDENT_AMPS = 1ull << 22;
+// From this many such passes on: the launch has its tables to prepare (a clear, a kernel, a larger
+// workspace). Runs of 1, 2, 3, 5 later passes, in us with the first pass, launch per pass / one
+// launch: 27 / 33, 37 / 37, 47 / 43, 68 / 54 at 2^12 amplitudes; 44 / 51, 62 / 66, 72 / 71,
+// 102 / 91 at 2^20; 98 / 105, 130 / 135, 162 / 162, 239 / 228 at 2^22.
+constexpr size_t CHAIN_RESIDENT_PASSES = 3;
 // One of those passes: two disjoint two-qubit gates, and the permutation after them (perm) if
 // the pass is to write its outputs permuted, out of place.
 struct ChainStep {

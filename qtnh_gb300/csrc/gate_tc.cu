@@ -442,11 +442,12 @@ bool apply_gate_runs_tc(void* state, void* scratch, dims_t dims, const std::vect
       ++j;
     }
     if (R >= 2 && chain_enabled()) {
-      // the first pass is a launch of its own (per-group scales); the later ones of a state that
-      // L2 holds go in launches of up to chain_resident_passes() passes, which end early only at
-      // a permutation that cannot be folded into the pass before it
+      // the first pass is a launch of its own (per-group scales); the later ones of a state that L2
+      // holds go in launches of up to chain_resident_passes() passes, which end early only at a
+      // permutation that cannot be folded into the pass before it, or, if those are fewer than
+      // CHAIN_RESIDENT_PASSES, one by one
       const uint64_t ngroups = steps[i].p.ngroups;
-      const bool resident = chain_resident(steps[i].p);
+      const size_t most = chain_resident(steps[i].p) ? (size_t)chain_resident_passes() : 1;
       // one record per launch
       ChainRec* recs = static_cast<ChainRec*>(workspace_alloc(R * sizeof(ChainRec), stream));
       try {
@@ -454,14 +455,25 @@ bool apply_gate_runs_tc(void* state, void* scratch, dims_t dims, const std::vect
         size_t k = 0, t = i, launches = 0;
         std::vector<ChainStep> open;
         auto flush = [&] {
-          if (open.empty()) return;
-          timed_pass(s, open.size(), [&] {
-            launch_chain_resident(cur, oth, open, ngroups, &recs[launches], &recs[launches + 1], s);
-          });
-          ++launches;
-          count_launch(open.size());
-          for (const ChainStep& c : open)
-            if (c.perm) std::swap(cur, oth);
+          if (open.size() >= CHAIN_RESIDENT_PASSES) {
+            timed_pass(s, open.size(), [&] {
+              launch_chain_resident(cur, oth, open, ngroups, &recs[launches], &recs[launches + 1], s);
+            });
+            ++launches;
+            count_launch(open.size());
+            for (const ChainStep& c : open)
+              if (c.perm) std::swap(cur, oth);
+          } else {
+            for (const ChainStep& c : open) {
+              timed_pass(s, 1, [&] {
+                launch_pair_chain(cur, c.ga, c.gb, c.p, s, &recs[launches], &recs[launches + 1], c.want_fixed,
+                                  c.perm ? oth : nullptr, c.perm ? &c.map : nullptr);
+              });
+              ++launches;
+              count_launch();
+              if (c.perm) std::swap(cur, oth);
+            }
+          }
           open.clear();
         };
         for (; t <= last; ++t) {
@@ -479,22 +491,10 @@ bool apply_gate_runs_tc(void* state, void* scratch, dims_t dims, const std::vect
           } else {
             // a permutation after the pass: its outputs go permuted, out of place
             const LayerStep* next = t + 1 < steps.size() && steps[t + 1].perm >= 0 && fuse_permutes() ? &steps[t + 1] : nullptr;
-            bool fuse = false;
-            if (resident) {
-              ChainStep c{sk.p, gate_ptr(sk.g), gate_ptr(sk.g + 1), k + 1 < R, false, {}};
-              fuse = c.perm = next && make_bit_map(next->dims, runs[(size_t)next->perm].ptup, c.map);
-              open.push_back(c);
-              if ((int)open.size() == chain_resident_passes()) flush();
-            } else {
-              BitMap map;
-              fuse = next && make_bit_map(next->dims, runs[(size_t)next->perm].ptup, map);
-              timed_pass(s, 1, [&] {
-                launch_pair_chain(cur, gate_ptr(sk.g), gate_ptr(sk.g + 1), sk.p, s, &recs[k - 1], &recs[k], k + 1 < R,
-                                  fuse ? oth : nullptr, fuse ? &map : nullptr);
-              });
-              count_launch();
-              if (fuse) std::swap(cur, oth);
-            }
+            ChainStep c{sk.p, gate_ptr(sk.g), gate_ptr(sk.g + 1), k + 1 < R, false, {}};
+            const bool fuse = c.perm = next && make_bit_map(next->dims, runs[(size_t)next->perm].ptup, c.map);
+            open.push_back(c);
+            if (open.size() == most) flush();
             if (fuse) ++t;  // the permutation is done
           }
           ++k;
