@@ -172,8 +172,10 @@ bool chain_resident(const PairParams& p);
 int chain_resident_passes();
 // Such a launch: *rin describes the state (what the pass before wrote), *rout receives the
 // record of the last pass (zeroed by the caller). The state moves to the other buffer at
-// every step with a permutation.
-void launch_chain_resident(void* cur, void* oth, const std::vector<ChainStep>& steps, uint64_t ngroups,
+// every step with a permutation. false, and the state as it was, where the SMs that the stream may
+// use are fewer than the launch's CTAs (a context with a share of them; the CTAs wait for one
+// another), or where there is no memory for its tables (up to 1.4 MB; a launch per pass needs none).
+bool launch_chain_resident(void* cur, void* oth, const std::vector<ChainStep>& steps, uint64_t ngroups,
                            const ChainRec* rin, ChainRec* rout, cudaStream_t s);
 
 // Reads and clears the tcgen05 kernel's device error flags (bounded waits that expired).

@@ -345,9 +345,9 @@ struct PassEvents {
 };
 std::vector<PassEvents> g_pass_events;
 
-// Issues `passes` fused passes, one launch.
+// Issues one launch; `launch` returns how many fused passes it makes (0: none was issued).
 template <typename F>
-void timed_pass(cudaStream_t s, uint64_t passes, F&& launch) {
+uint64_t timed_pass(cudaStream_t s, F&& launch) {
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   {
     std::lock_guard<std::mutex> lk(g_pass_mu);
@@ -357,12 +357,16 @@ void timed_pass(cudaStream_t s, uint64_t passes, F&& launch) {
     }
   }
   if (e0) check_cuda(cudaEventRecord(e0, s), "event record");
-  launch();
-  if (e1) {
+  const uint64_t passes = launch();
+  if (e1 && passes) {
     check_cuda(cudaEventRecord(e1, s), "event record");
     std::lock_guard<std::mutex> lk(g_pass_mu);
     g_pass_events.push_back({e0, e1, passes});
+  } else if (e1) {
+    cudaEventDestroy(e0);
+    cudaEventDestroy(e1);
   }
+  return passes;
 }
 
 }  // namespace
@@ -445,7 +449,7 @@ bool apply_gate_runs_tc(void* state, void* scratch, dims_t dims, const std::vect
       // the first pass is a launch of its own (per-group scales); the later ones of a state that L2
       // holds go in launches of up to chain_resident_passes() passes, which end early only at a
       // permutation that cannot be folded into the pass before it, or, if those are fewer than
-      // CHAIN_RESIDENT_PASSES, one by one
+      // CHAIN_RESIDENT_PASSES or the launch is refused, one by one
       const uint64_t ngroups = steps[i].p.ngroups;
       const size_t most = chain_resident(steps[i].p) ? (size_t)chain_resident_passes() : 1;
       // one record per launch
@@ -455,19 +459,20 @@ bool apply_gate_runs_tc(void* state, void* scratch, dims_t dims, const std::vect
         size_t k = 0, t = i, launches = 0;
         std::vector<ChainStep> open;
         auto flush = [&] {
-          if (open.size() >= CHAIN_RESIDENT_PASSES) {
-            timed_pass(s, open.size(), [&] {
-              launch_chain_resident(cur, oth, open, ngroups, &recs[launches], &recs[launches + 1], s);
-            });
+          if (open.size() >= CHAIN_RESIDENT_PASSES && timed_pass(s, [&]() -> uint64_t {
+                return launch_chain_resident(cur, oth, open, ngroups, &recs[launches], &recs[launches + 1], s) ? open.size()
+                                                                                                           : 0;
+              })) {
             ++launches;
             count_launch(open.size());
             for (const ChainStep& c : open)
               if (c.perm) std::swap(cur, oth);
           } else {
             for (const ChainStep& c : open) {
-              timed_pass(s, 1, [&] {
+              timed_pass(s, [&] {
                 launch_pair_chain(cur, c.ga, c.gb, c.p, s, &recs[launches], &recs[launches + 1], c.want_fixed,
                                   c.perm ? oth : nullptr, c.perm ? &c.map : nullptr);
+                return 1;
               });
               ++launches;
               count_launch();
@@ -484,8 +489,9 @@ bool apply_gate_runs_tc(void* state, void* scratch, dims_t dims, const std::vect
             continue;
           }
           if (k == 0) {
-            timed_pass(s, 1, [&] {
+            timed_pass(s, [&] {
               launch_pair_umma(static_cast<double2*>(cur), gate_ptr(sk.g), gate_ptr(sk.g + 1), sk.p, s, PAIR_KRON, &recs[0]);
+              return 1;
             });
             count_launch();
           } else {
@@ -511,8 +517,10 @@ bool apply_gate_runs_tc(void* state, void* scratch, dims_t dims, const std::vect
     }
     const LayerStep& st = steps[i];
     if (st.pair)
-      timed_pass(s, 1, [&] { launch_fused_pair(static_cast<double2*>(cur), gate_ptr(st.g), gate_ptr(st.g + 1), st.p,
-                                            product(st.dims), s); });
+      timed_pass(s, [&] {
+        launch_fused_pair(static_cast<double2*>(cur), gate_ptr(st.g), gate_ptr(st.g + 1), st.p, product(st.dims), s);
+        return 1;
+      });
     else
       apply_gate_device(cur, st.dims, targets[st.g], gates[st.g], stream);
     ++i;

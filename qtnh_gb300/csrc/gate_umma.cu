@@ -1681,7 +1681,7 @@ static uint64_t spread_bits(uint64_t x, const uint32_t (&ins)[4]) {
   return x;
 }
 
-void launch_chain_resident(void* cur, void* oth, const std::vector<ChainStep>& steps, uint64_t ngroups,
+bool launch_chain_resident(void* cur, void* oth, const std::vector<ChainStep>& steps, uint64_t ngroups,
                          const ChainRec* rin, ChainRec* rout, cudaStream_t s) {
   const int npass = (int)steps.size();
   if (npass < 1 || npass > CR_MAXP) throw Error(QTNH_ERR_RUNTIME, "chain launch length");
@@ -1714,7 +1714,14 @@ void launch_chain_resident(void* cur, void* oth, const std::vector<ChainStep>& s
   const size_t words_bytes = (size_t)npass * 128;  // a line each
   const size_t zero_bytes = words_bytes + (size_t)npass * sizeof(ChainRec);
   const size_t gate_off = (zero_bytes + 255) / 256 * 256, gate_bytes = (size_t)npass * sizeof(ChainGate);
-  uint8_t* ws = static_cast<uint8_t*>(workspace_alloc(gate_off + gate_bytes + (size_t)nperm * 4096, s));
+  uint8_t* ws = nullptr;
+  try {
+    ws = static_cast<uint8_t*>(workspace_alloc(gate_off + gate_bytes + (size_t)nperm * 4096, s));
+  } catch (const Error& e) {
+    if (e.code != QTNH_ERR_NO_MEMORY) throw;
+    cudaGetLastError();  // (not sticky)
+    return false;
+  }
   uint64_t* words = reinterpret_cast<uint64_t*>(ws);
   ChainRec* rmid = reinterpret_cast<ChainRec*>(ws + words_bytes);
   ChainGate* gates = reinterpret_cast<ChainGate*>(ws + gate_off);
@@ -1737,7 +1744,12 @@ void launch_chain_resident(void* cur, void* oth, const std::vector<ChainStep>& s
     }
   }
   workspace_free(ws, s);
+  if (e == cudaErrorCooperativeLaunchTooLarge) {
+    cudaGetLastError();  // (not sticky)
+    return false;
+  }
   check_cuda(e, "gate chain launch");
+  return true;
 }
 
 bool chain_resident(const PairParams& p) { return chain_applies(p) && p.ngroups * 16 <= CHAIN_RESIDENT_AMPS; }
