@@ -173,6 +173,66 @@ __global__ void __launch_bounds__(TILE_THREADS, 4) tiled_permute_kernel(const c1
   }
 }
 
+// The same with the bases of a step's tiles decoded at its start, T a power of two: for steps of few
+// large tiles whose bases take little (plan_permute has the rule). 2^13 x 2^13 elements 357 us, in the
+// form above 385; that form with its bases decoded in step 426.
+__global__ void __launch_bounds__(TILE_THREADS, 4) tiled_permute_step_kernel(const c128* __restrict__ in,
+                                                                          c128* __restrict__ out,
+                                                                          const __grid_constant__ TileParams p) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int T = p.T, G = p.G, S = p.tile_slots;
+  c128* tile = reinterpret_cast<c128*>(smem_raw);  // G tiles of S slots
+  uint64_t* s_bin = reinterpret_cast<uint64_t*>(tile + (size_t)G * S);
+  uint64_t* s_bout = s_bin + G;
+  int64_t* s_rin = reinterpret_cast<int64_t*>(s_bout + G);
+  int64_t* s_wout = s_rin + T;
+  int32_t* s_rslot = reinterpret_cast<int32_t*>(s_wout + T);
+  int32_t* s_wslot = s_rslot + T;
+  for (int t = threadIdx.x; t < T; t += blockDim.x) {
+    s_rin[t] = p.rin[t];
+    s_wout[t] = p.wout[t];
+    s_rslot[t] = p.rslot[t];
+    s_wslot[t] = p.wslot[t];
+  }
+  const uint64_t total = p.rest.total;
+  for (uint64_t r0 = (uint64_t)blockIdx.x * G; r0 < total; r0 += (uint64_t)gridDim.x * G) {
+    for (int g = threadIdx.x; g < G && r0 + g < total; g += blockDim.x) {
+      uint64_t bin, bout;
+      decode(r0 + g, p.rest, bin, bout);
+      s_bin[g] = bin;
+      s_bout[g] = bout;
+    }
+    __syncthreads();
+    const uint64_t left = total - r0;
+    const int n = (left < (uint64_t)G ? (int)left : G) * T;  // <= STEP_ELEMS
+    // all of this thread's loads are issued before any is stored to shared memory
+    c128 v[TILE_PER_THREAD];
+    int slot[TILE_PER_THREAD];
+#pragma unroll
+    for (int k = 0; k < TILE_PER_THREAD; ++k) {
+      const int e = threadIdx.x + k * TILE_THREADS;
+      if (e < n) {
+        const int g = G > 1 ? e >> p.T_log2 : 0, t = G > 1 ? e & (T - 1) : e;
+        slot[k] = g * S + s_rslot[t];
+        v[k] = __ldg(in + s_bin[g] + s_rin[t]);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < TILE_PER_THREAD; ++k)
+      if (threadIdx.x + k * TILE_THREADS < n) tile[slot[k]] = v[k];
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < TILE_PER_THREAD; ++k) {
+      const int e = threadIdx.x + k * TILE_THREADS;
+      if (e < n) {
+        const int g = G > 1 ? e >> p.T_log2 : 0, t = G > 1 ? e & (T - 1) : e;
+        out[s_bout[g] + s_wout[t]] = tile[g * S + s_wslot[t]];
+      }
+    }
+    __syncthreads();
+  }
+}
+
 // Innermost axis fixed: copy runs of L elements. When L is a multiple of 128 every warp
 // copies 128 contiguous elements (4 per lane) of a single run per step.
 __global__ void __launch_bounds__(256) run_copy_kernel(const c128* __restrict__ in, c128* __restrict__ out,
@@ -430,6 +490,7 @@ struct Plan {
   int grid = 0;
   RunParams run;
   RestDesc gather;
+  bool ahead = true;  // TILED: tiled_permute_kernel, else tiled_permute_step_kernel
 };
 
 // The launch plan of a permutation. boundary < 0: plain permute (output offsets are
@@ -587,26 +648,25 @@ Plan plan_permute(const dims_t& dims, const std::vector<uint16_t>& ptup, int bou
       return m;
     };
     auto mA = mults(A), mB = mults(B);
-    // Read order: t = b * PA + a.
-    for (uint64_t b = 0; b < PB; ++b) {
-      uint64_t offb = 0, rem = b;
-      for (int k = (int)B.size() - 1; k >= 0; --k) {
-        uint64_t d = rem % c.dims[B[k]];
-        rem /= c.dims[B[k]];
-        offb += d * in_stride[B[k]];
-      }
-      for (uint64_t a = 0; a < PA; ++a) {
-        uint64_t offa = 0, ra = a;
-        for (int k = (int)A.size() - 1; k >= 0; --k) {
-          uint64_t d = ra % c.dims[A[k]];
-          ra /= c.dims[A[k]];
-          offa += d * in_stride[A[k]];
+    // Read order: t = b * PA + a (the offsets over A and over B add).
+    auto offsets = [&](const std::vector<int>& axes, uint64_t n) {
+      std::vector<uint64_t> off(n, 0);
+      for (uint64_t x = 0; x < n; ++x) {
+        uint64_t rem = x;
+        for (int k = (int)axes.size() - 1; k >= 0; --k) {
+          off[x] += rem % c.dims[axes[k]] * in_stride[axes[k]];
+          rem /= c.dims[axes[k]];
         }
-        int t = (int)(b * PA + a);
-        p.rin[t] = (int64_t)(offa + offb);
+      }
+      return off;
+    };
+    const std::vector<uint64_t> offa = offsets(A, PA), offb = offsets(B, PB);
+    for (uint64_t b = 0; b < PB; ++b)
+      for (uint64_t a = 0; a < PA; ++a) {
+        const int t = (int)(b * PA + a);
+        p.rin[t] = (int64_t)(offa[a] + offb[b]);
         p.rslot[t] = slot_of(a, b);
       }
-    }
     // Write order: tile axes by output position, row-major.
     std::vector<int> tax(A);
     tax.insert(tax.end(), B.begin(), B.end());
@@ -629,6 +689,13 @@ Plan plan_permute(const dims_t& dims, const std::vector<uint16_t>& ptup, int bou
       if (!inA[i] && !inB[i]) fill_axis(p.rest.ax[nr++], c.dims[i], in_stride[i], out_stride[i]);
     p.rest.n = nr;
     p.rest.total = N / (uint64_t)T;
+    // Bases in step: steps of two or four tiles of a power of two of elements, with few axes left to
+    // decode them from; a step ahead otherwise. In us, in step / ahead: tiles of 1024 with two axes
+    // left 31.6 / 35.0 at 2^20 elements, 47.2 / 53.3 at 2^22, 357 / 385 at 2^26, with 8 axes 49.4 / 53.3
+    // (2^22), with 14 axes 121.1 / 119.8 (2^24); tiles of 512 with two axes 96.0 / 98.0 (2^24), with 9
+    // 104.9 / 104.5; tiles of 256 with one axis 354 / 327 (2^26).
+    plan.ahead = boundary >= 0 || tl == 0xFFFFFFFFu || T < 512 || STEP_ELEMS / T * nr > 24;
+    if (!plan.ahead) p.G = STEP_ELEMS / T;
     // one axis per lane costs less than divisions in turn, shifts in turn less than the lanes
     // (2^26 elements in a random order: 356 us by shifts, 404 by lanes)
     p.lanes = 0;
@@ -691,10 +758,12 @@ void permute_device(const void* in_v, void* out_v, const dims_t& dims, const std
       return;
     case Plan::TILED:
       if (plan.smem > 48 * 1024)
-        check_cuda(cudaFuncSetAttribute(tiled_permute_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)plan.smem),
+        check_cuda(cudaFuncSetAttribute(plan.ahead ? tiled_permute_kernel : tiled_permute_step_kernel,
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem),
                    "tiled_permute_kernel shared memory");
-      tiled_permute_kernel<<<plan.grid, TILE_THREADS, plan.smem, s>>>(in, out, *plan.tile);
+      // (through a pointer to either kernel the 25 KB of parameters would be copied once more)
+      if (plan.ahead) tiled_permute_kernel<<<plan.grid, TILE_THREADS, plan.smem, s>>>(in, out, *plan.tile);
+      else tiled_permute_step_kernel<<<plan.grid, TILE_THREADS, plan.smem, s>>>(in, out, *plan.tile);
       count_launch();
       check_cuda(cudaGetLastError(), "tiled_permute_kernel launch");
       return;
