@@ -935,14 +935,13 @@ static_assert(sizeof(ChainGate) % 16 == 0 && sizeof(ChainDigits) % 16 == 0, "bul
 struct ChainPrepParams {
   const double2* ga[CR_MAXP];
   const double2* gb[CR_MAXP];
-  uint8_t mode[CR_MAXP];                // PairGate
-  BitMap map[CR_MAXP];                  // permutations
+  BitMap map[CR_MAXP];  // permutations
 };
 
 // A pass of one launch of the chain kernel (kernel parameter).
 struct ChainPassP {
-  uint64_t tgt[4];  // masks of the target bits of amplitude index bits 3, 2, 1, 0
-  uint64_t step;    // from one tile of a CTA to its next: 128 x grid in the group index's bits
+  uint32_t tgt[4];  // masks of the target bits of amplitude index bits 3, 2, 1, 0
+  uint32_t step;    // from one tile of a CTA to its next: 128 x grid in the group index's bits
   uint8_t ins[4];   // the four target bits, ascending
   int16_t perm;     // >= 0: the outputs go to the other buffer, permuted by table `perm`
   uint16_t want_fixed;
@@ -970,13 +969,10 @@ __global__ void __launch_bounds__(128) chain_prep_kernel(const __grid_constant__
   __shared__ int ok_all;
   const double2* ga = q.ga[blockIdx.x];
   const double2* gb = q.gb[blockIdx.x];
-  const uint32_t mode = q.mode[blockIdx.x];
   ChainGate& g = gates[blockIdx.x];
   if (tid == 0) ok_all = 1;
   for (int t = tid; t < 256; t += 128) {
-    const double2 u = mode == PAIR_KRON     ? fused_entry<PAIR_KRON>(ga, gb, t)
-                      : mode == PAIR_FULL   ? fused_entry<PAIR_FULL>(ga, gb, t)
-                                            : fused_entry<PAIR_KRON_I2>(ga, gb, t);
+    const double2 u = fused_entry<PAIR_KRON>(ga, gb, t);
     U16[t] = u;
     g.U16[t] = u;
   }
@@ -1036,14 +1032,12 @@ struct CrSmem {
   uint32_t mine, t0;                     // this CTA's tiles per pass; its tiles of the earlier passes
   const void* in;
   void* out;
-  // the pass's address steps, as IT: s0, s1, step, holes, w0, w1 (s, w: the target bits of
+  // the pass's address steps: s0, s1, step, holes, w0, w1 (s, w: the target bits of
   // amplitude index bits 1 and 0 and their images); held in registers across the tile loop
   // they would spill
-  alignas(16) uint64_t addr[8];
+  uint32_t addr[6];
   uint32_t ptab[4][256];                 // the permutation's bit tables
 };
-static_assert(CH_NLMAX * UM_N <= (int)CH_ACC, "chain level sums exceed an accumulator set");
-static_assert(2 * CH_ACC <= CH_TMEM_COLS, "two accumulator sets");
 static_assert(sizeof(CrSmem) + 1024 <= 227 * 1024, "chain shared memory");
 
 __device__ __forceinline__ uint64_t ld_acquire(const uint64_t* p) {
@@ -1063,36 +1057,31 @@ __device__ __forceinline__ uint32_t chain_image(const uint32_t (*tab)[256], uint
   return tab[0][x & 255u] | tab[1][(x >> 8) & 255u] | tab[2][(x >> 16) & 255u] | tab[3][x >> 24];
 }
 // Zero bits inserted at the four target positions of a group index.
-template <typename IT>
-__device__ __forceinline__ IT chain_base(IT b, const ChainPassP& pp) {
+__device__ __forceinline__ uint32_t chain_base(uint32_t b, const ChainPassP& pp) {
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    const IT low = b & ((IT(1) << pp.ins[j]) - 1);
+    const uint32_t low = b & ((1u << pp.ins[j]) - 1);
     b = ((b >> pp.ins[j]) << (pp.ins[j] + 1)) | low;
   }
   return b;
 }
 // The target bits as one mask, and the tile part of a CTA's next tile: an addition in the
 // group index's bits, the target bits set so that carries run across them.
-template <typename IT>
-__device__ __forceinline__ IT chain_holes(const ChainPassP& pp) {
-  return (IT)(pp.tgt[0] | pp.tgt[1] | pp.tgt[2] | pp.tgt[3]);
+__device__ __forceinline__ uint32_t chain_holes(const ChainPassP& pp) {
+  return pp.tgt[0] | pp.tgt[1] | pp.tgt[2] | pp.tgt[3];
 }
-template <typename IT>
-__device__ __forceinline__ IT chain_next_tile(IT tb, IT step, IT holes) {
+__device__ __forceinline__ uint32_t chain_next_tile(uint32_t tb, uint32_t step, uint32_t holes) {
   return ((tb | holes) + step) & ~holes;
 }
 // Index of amplitude 4h of row r relative to the tile's first group.
-template <typename IT>
-__device__ __forceinline__ IT chain_row(const ChainPassP& pp, int h, int r) {
-  return chain_base<IT>((IT)r, pp) | ((h & 2) ? (IT)pp.tgt[0] : IT(0)) | ((h & 1) ? (IT)pp.tgt[1] : IT(0));
+__device__ __forceinline__ uint32_t chain_row(const ChainPassP& pp, int h, int r) {
+  return chain_base((uint32_t)r, pp) | ((h & 2) ? pp.tgt[0] : 0u) | ((h & 1) ? pp.tgt[1] : 0u);
 }
 
 // The four amplitudes of row r at `at` into stage slot `slot` (one commit group per tile,
 // empty past the end); s0, s1: the target bits of amplitude index bits 1 and 0.
-template <typename IT>
-__device__ __forceinline__ void chain_fetch(CrSmem& sm, const void* in, bool live, IT at, IT s0, IT s1, uint32_t slot,
-                                            int h, int r) {
+__device__ __forceinline__ void chain_fetch(CrSmem& sm, const void* in, bool live, uint32_t at, uint32_t s0,
+                                            uint32_t s1, uint32_t slot, int h, int r) {
   if (live) {
     const double2* src = static_cast<const double2*>(in) + at;
     double2* dst = &sm.stage[slot][4 * h][r];
@@ -1122,21 +1111,21 @@ __device__ __forceinline__ int chain_scale_ein(uint32_t sc) { return (int)sc >> 
 // form's further registers would spill in the loop. Not inlined for the same reason: the
 // kernel's own state stays out of the loop (and few arguments, or they come from the stack in
 // the loop; the rest is in shared memory). sc: chain_scale. false: a wait expired.
-template <typename IT, int NL, bool FAST, bool PO>
-__device__ __noinline__ bool chain_team_pass(IT rbase, IT tb, uint32_t sc) {
+template <int NL, bool FAST, bool PO>
+__device__ __noinline__ bool chain_team_pass(uint32_t rbase, uint32_t tb, uint32_t sc) {
   CrSmem& sm = *reinterpret_cast<CrSmem*>(resident_smem);
   const int h = (int)(threadIdx.x >> 7), r = (int)(threadIdx.x & 127);
   // this thread's 8 reals (amplitudes 4h .. 4h + 3, real and imaginary parts interleaved)
   // are row r of K core h: K-step h / 2, core h % 2
   const uint32_t row_off = (uint32_t)((r >> 3) * 256 + (r & 7) * 16 + (h & 1) * 128);
-  const IT* ad = reinterpret_cast<const IT*>(sm.addr);  // s0, s1, step, holes, w0, w1
+  const uint32_t* ad = sm.addr;  // s0, s1, step, holes, w0, w1
   const void* in = sm.in;
   void* out = sm.out;
   const uint32_t t0 = sm.t0, t1 = t0 + sm.mine;
   const int32_t sh = chain_scale_sh(sc);
   const uint64_t cadd = oz::fixed_addend(sh);
   // where amplitude 4h of row r goes, relative to the image of the tile part
-  const IT wbase = PO ? (IT)chain_image(sm.ptab, (uint32_t)rbase) : rbase;
+  const uint32_t wbase = PO ? chain_image(sm.ptab, rbase) : rbase;
   const bool in_fixed = FAST || (sc & CH_IN_FIXED), out_fixed = FAST || (sc & CH_OUT_FIXED), common = FAST || (sc & CH_COMMON);
   const ChainDigits& gd = sm.gd[(sc & CH_ODD) ? 1 : 0];
   // per output 4h + a: the row shift to the common output scale, 8 bits each
@@ -1149,12 +1138,12 @@ __device__ __noinline__ bool chain_team_pass(IT rbase, IT tb, uint32_t sc) {
   const uint32_t tlane = sm.tmem_base + ((uint32_t)(r & ~31) << 16) + (uint32_t)(8 * h);
   // level sums from accumulator set b -> the outputs 4h .. 4h + 3 of group r of the tile
   // whose tile part is tp
-  auto recombine = [&](IT tp, uint32_t b) {
+  auto recombine = [&](uint32_t tp, uint32_t b) {
     uint32_t v[NL][8];  // level l, output real 8h + 2a + part
 #pragma unroll
     for (int l = 0; l < NL; ++l) tmem_ld8(tlane + b * CH_ACC + (uint32_t)(32 * l), v[l]);
-    const IT obase = (PO ? (IT)chain_image(sm.ptab, (uint32_t)tp) : tp) | wbase;
-    const IT w0 = ad[4], w1 = ad[5];
+    const uint32_t obase = (PO ? chain_image(sm.ptab, tp) : tp) | wbase;
+    const uint32_t w0 = ad[4], w1 = ad[5];
     tmem_wait_ld();
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
@@ -1167,7 +1156,7 @@ __device__ __noinline__ bool chain_team_pass(IT rbase, IT tb, uint32_t sc) {
       } else {
         Tr = oz::fixed_levels<NL>(cr), Ti = oz::fixed_levels<NL>(ci);
       }
-      const IT ix = obase + ((a & 2) ? w0 : IT(0)) + ((a & 1) ? w1 : IT(0));
+      const uint32_t ix = obase + ((a & 2) ? w0 : 0u) + ((a & 1) ? w1 : 0u);
       if (out_fixed) {
         if (!FAST && !common) {
           const uint32_t sk = (kk >> (8 * a)) & 0xFFu;
@@ -1185,7 +1174,8 @@ __device__ __noinline__ bool chain_team_pass(IT rbase, IT tb, uint32_t sc) {
       }
     }
   };
-  IT tb_f = chain_next_tile(tb, ad[2], ad[3]);  // tile part of the last tile fetched; tb: of the next one to store
+  // tb_f: tile part of the last tile fetched; tb: of the next one to store
+  uint32_t tb_f = chain_next_tile(tb, ad[2], ad[3]);
   bool ok = true;
   for (uint32_t t = t0; t < t1; ++t) {
     const uint32_t b = t & 1u;
@@ -1194,7 +1184,7 @@ __device__ __noinline__ bool chain_team_pass(IT rbase, IT tb, uint32_t sc) {
 #pragma unroll
     for (int c = 0; c < 4; ++c) x[c] = sm.stage[b][4 * h + c][r];
     tb_f = chain_next_tile(tb_f, ad[2], ad[3]);
-    chain_fetch<IT>(sm, in, t + 2 < t1, tb_f | rbase, ad[0], ad[1], b, h, r);  // only this thread reads its stage slots
+    chain_fetch(sm, in, t + 2 < t1, tb_f | rbase, ad[0], ad[1], b, h, r);  // only this thread reads its stage slots
     // digits of this thread's 8 reals: digit j of amplitude 4h + a as one fp16x2 word (real,
     // imaginary); the four words of digit j fill the thread's core-matrix row
     uint32_t w[4][CH_ND];
@@ -1257,21 +1247,20 @@ __device__ __noinline__ bool chain_team_pass(IT rbase, IT tb, uint32_t sc) {
 // Every group of a pass in FP64 (no tensor cores): thread per group, doubles out; the
 // output range is recorded like the first pass's, so a later pass starts no chain on it.
 // Loads bypass L1, which may hold lines of an earlier pass.
-template <typename IT>
 __device__ __noinline__ void chain_pass_fp64(CrSmem& sm, const ChainPassP& pp, const void* in, double2* out,
                                              const double2* U16, uint64_t ngroups, int in_fixed, int32_t F) {
   uint32_t okey = 0, ominc = 0;
   for (uint64_t grp = (uint64_t)blockIdx.x * CH_THREADS + threadIdx.x; grp < ngroups;
        grp += (uint64_t)gridDim.x * CH_THREADS) {
-    const IT base = chain_base<IT>((IT)grp, pp);
-    auto at = [&](int c) -> IT {
-      return base | ((c & 8) ? (IT)pp.tgt[0] : IT(0)) | ((c & 4) ? (IT)pp.tgt[1] : IT(0)) |
-             ((c & 2) ? (IT)pp.tgt[2] : IT(0)) | ((c & 1) ? (IT)pp.tgt[3] : IT(0));
+    const uint32_t base = chain_base((uint32_t)grp, pp);
+    auto at = [&](int c) -> uint32_t {
+      return base | ((c & 8) ? pp.tgt[0] : 0u) | ((c & 4) ? pp.tgt[1] : 0u) | ((c & 2) ? pp.tgt[2] : 0u) |
+             ((c & 1) ? pp.tgt[3] : 0u);
     };
     double2 x[16];
 #pragma unroll
     for (int c = 0; c < 16; ++c) {
-      const IT ix = at(c);
+      const uint32_t ix = at(c);
       if (in_fixed) {
         const longlong2 y = __ldcg(static_cast<const longlong2*>(in) + ix);
         x[c] = make_double2(oz::fixed_to_double(y.x, 40 - F), oz::fixed_to_double(y.y, 40 - F));
@@ -1284,8 +1273,8 @@ __device__ __noinline__ void chain_pass_fp64(CrSmem& sm, const ChainPassP& pp, c
     for (int o = 0; o < 16; ++o) {
       const double2 v = group_output_fp64(U16, x, o);
       gkey = max(gkey, amp_key(v));
-      const IT ix = at(o);
-      out[pp.perm >= 0 ? (IT)chain_image(sm.ptab, (uint32_t)ix) : ix] = v;
+      const uint32_t ix = at(o);
+      out[pp.perm >= 0 ? chain_image(sm.ptab, ix) : ix] = v;
     }
     okey = max(okey, gkey);
     if (gkey) ominc = max(ominc, 2047u - oz::key_exponent(gkey));
@@ -1340,7 +1329,7 @@ __device__ __noinline__ void chain_pass_fp64(CrSmem& sm, const ChainPassP& pp, c
 // buffer, element x to index P(x) (bit tables in shared memory; P(tile part | row part |
 // offset) is the OR of the three parts' images), so the pass and the permutation after it
 // take one pass over the state.
-template <typename IT, int NL>
+template <int NL>
 __global__ void __launch_bounds__(CH_THREADS, 1) gate_chain_resident_kernel(void* buf0, void* buf1,
                                                                         const ChainGate* __restrict__ gates,
                                                                         const uint32_t* __restrict__ ptabs,
@@ -1387,28 +1376,28 @@ __global__ void __launch_bounds__(CH_THREADS, 1) gate_chain_resident_kernel(void
 
   // what pass k needs besides its input's range: this thread's row and first tile (rbase, tb),
   // the address steps, the permutation's tables, the gate digits
-  IT rbase, tb, s0, s1, tb1;
+  uint32_t rbase, tb, s0, s1, tb1;
   auto prepare = [&](int k, void* in, void* other, uint32_t t0) {
     const ChainPassP& pp = ps.p[k];
-    rbase = chain_row<IT>(pp, h, r);
-    tb = chain_base<IT>((IT)((uint64_t)blockIdx.x * UM_M), pp);
-    tb1 = chain_next_tile(tb, (IT)pp.step, chain_holes<IT>(pp));
-    s0 = (IT)pp.tgt[2], s1 = (IT)pp.tgt[3];
+    rbase = chain_row(pp, h, r);
+    tb = chain_base(blockIdx.x * (uint32_t)UM_M, pp);
+    tb1 = chain_next_tile(tb, pp.step, chain_holes(pp));
+    s0 = pp.tgt[2], s1 = pp.tgt[3];
     const bool po = pp.perm >= 0;
     const uint32_t* src = ptabs + (size_t)(po ? pp.perm : 0) * 1024;
     if (po) {
       for (int t = tid; t < 1024; t += CH_THREADS) (&sm.ptab[0][0])[t] = __ldg(src + t);
     }
     if (tid == CH_TEAM) {
-      auto image = [&](uint32_t x) -> IT {
-        return (IT)(__ldg(src + (x & 255u)) | __ldg(src + 256 + ((x >> 8) & 255u)) | __ldg(src + 512 + ((x >> 16) & 255u)) |
-                    __ldg(src + 768 + (x >> 24)));
+      auto image = [&](uint32_t x) {
+        return __ldg(src + (x & 255u)) | __ldg(src + 256 + ((x >> 8) & 255u)) | __ldg(src + 512 + ((x >> 16) & 255u)) |
+               __ldg(src + 768 + (x >> 24));
       };
       sm.in = in, sm.out = po ? other : in, sm.t0 = t0;
-      IT* ad = reinterpret_cast<IT*>(sm.addr);
-      ad[0] = s0, ad[1] = s1, ad[2] = (IT)pp.step, ad[3] = chain_holes<IT>(pp);
-      ad[4] = po ? image((uint32_t)s0) : s0;
-      ad[5] = po ? image((uint32_t)s1) : s1;
+      uint32_t* ad = sm.addr;
+      ad[0] = s0, ad[1] = s1, ad[2] = pp.step, ad[3] = chain_holes(pp);
+      ad[4] = po ? image(s0) : s0;
+      ad[5] = po ? image(s1) : s1;
     }
     if (!mbar_wait_warp(&sm.gate[k & 1], (uint32_t)((k >> 1) & 1), &sm.no_abort)) {
       atomicOr(&g_umma_error, 1u);
@@ -1429,8 +1418,8 @@ __global__ void __launch_bounds__(CH_THREADS, 1) gate_chain_resident_kernel(void
   for (; k < npass && sm.abort == 0; ++k) {
     // the first two tiles are on their way before anything else
     if (warp < CH_WARPS) {
-      chain_fetch<IT>(sm, in, true, tb | rbase, s0, s1, t0 & 1u, h, r);
-      chain_fetch<IT>(sm, in, 1 < mine, tb1 | rbase, s0, s1, (t0 + 1) & 1u, h, r);
+      chain_fetch(sm, in, true, tb | rbase, s0, s1, t0 & 1u, h, r);
+      chain_fetch(sm, in, 1 < mine, tb1 | rbase, s0, s1, (t0 + 1) & 1u, h, r);
     }
     const bool po = ps.p[k].perm >= 0;
     void* out = po ? other : in;
@@ -1502,12 +1491,10 @@ __global__ void __launch_bounds__(CH_THREADS, 1) gate_chain_resident_kernel(void
                                           (common ? CH_COMMON : 0u) | ((k & 1) ? CH_ODD : 0u),
                                       sh, Ein);
       bool ok;
-      if (sizeof(IT) == 4 && po)
-        ok = fast ? chain_team_pass<IT, NL, true, sizeof(IT) == 4>(rbase, tb, sc)
-                  : chain_team_pass<IT, NL, false, sizeof(IT) == 4>(rbase, tb, sc);
+      if (po)
+        ok = fast ? chain_team_pass<NL, true, true>(rbase, tb, sc) : chain_team_pass<NL, false, true>(rbase, tb, sc);
       else
-        ok = fast ? chain_team_pass<IT, NL, true, false>(rbase, tb, sc)
-                  : chain_team_pass<IT, NL, false, false>(rbase, tb, sc);
+        ok = fast ? chain_team_pass<NL, true, false>(rbase, tb, sc) : chain_team_pass<NL, false, false>(rbase, tb, sc);
       if (!ok) {
         atomicOr(&g_umma_error, 2u);
         sm.abort = 1;
@@ -1516,7 +1503,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) gate_chain_resident_kernel(void
       cp_async_wait_all();
     }
     if (!uni)
-      chain_pass_fp64<IT>(sm, ps.p[k], in, static_cast<double2*>(out), gates[k].U16, ngroups, in_fixed ? 1 : 0, F_in);
+      chain_pass_fp64(sm, ps.p[k], in, static_cast<double2*>(out), gates[k].U16, ngroups, in_fixed ? 1 : 0, F_in);
     else
       t0 += mine;
     if (po) other = in, in = out;
@@ -1649,7 +1636,8 @@ void launch_pair_chain(void* psi, const double2* ga, const double2* gb, const Pa
   };
   for (int c = 0; c < 16; ++c) p.off[c] = gp.off[gate_index(c)];
   // the two amplitudes of index bit 0 are neighbours where they are stored, at whole sectors
-  const bool nb = (perm ? p.off[1] == 1ll << gp.ins_pos[0] && perm->dst[gp.ins_pos[0]] == 0 : p.off[1] == 1) && ((uintptr_t)(perm ? out : psi) & 31) == 0;
+  const bool adjacent = perm ? p.off[1] == 1ll << gp.ins_pos[0] && perm->dst[gp.ins_pos[0]] == 0 : p.off[1] == 1;
+  const bool nb = adjacent && ((uintptr_t)(perm ? out : psi) & 31) == 0;
   const bool i32 = p.ngroups * 16 <= (1ull << 32);
   if (perm) {
     if (!i32 || !out || out == psi) throw Error(QTNH_ERR_UNSUPPORTED, "permuted chain output");
@@ -1694,13 +1682,12 @@ bool launch_chain_resident(void* cur, void* oth, const std::vector<ChainStep>& s
     const ChainStep& st = steps[(size_t)k];
     q.ga[k] = st.ga;
     q.gb[k] = st.gb;
-    q.mode[k] = PAIR_KRON;
     ChainPassP& pp = ps.p[k];
     for (int j = 0; j < 4; ++j) {
       pp.ins[j] = (uint8_t)st.p.ins_pos[j];
-      pp.tgt[j] = (uint64_t)st.p.off[8 >> j];
+      pp.tgt[j] = (uint32_t)st.p.off[8 >> j];
     }
-    pp.step = spread_bits((uint64_t)grid * UM_M, st.p.ins_pos);
+    pp.step = (uint32_t)spread_bits((uint64_t)grid * UM_M, st.p.ins_pos);
     pp.want_fixed = st.want_fixed ? 1 : 0;
     pp.perm = -1;
     if (st.perm) {
@@ -1733,8 +1720,7 @@ bool launch_chain_resident(void* cur, void* oth, const std::vector<ChainStep>& s
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) {
-    const void* fn = nl == 6 ? (const void*)gate_chain_resident_kernel<uint32_t, 6>
-                             : (const void*)gate_chain_resident_kernel<uint32_t, 7>;
+    const void* fn = nl == 6 ? (const void*)gate_chain_resident_kernel<6> : (const void*)gate_chain_resident_kernel<7>;
     const int smem = (int)sizeof(CrSmem);
     e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess) {
