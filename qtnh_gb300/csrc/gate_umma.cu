@@ -1246,13 +1246,20 @@ __device__ __noinline__ bool chain_team_pass(uint32_t rbase, uint32_t tb, uint32
 
 // Every group of a pass in FP64 (no tensor cores): thread per group, doubles out; the
 // output range is recorded like the first pass's, so a later pass starts no chain on it.
-// Loads bypass L1, which may hold lines of an earlier pass.
+// Loads bypass L1, which may hold lines of an earlier pass. The whole CTA calls it, with nothing in
+// flight to the stage once its threads have met: the operator is read from there. Bound by the FP64
+// unit and, on small states, by one thread's chain of 1024 multiply-adds: a warp takes 32
+// neighbouring groups, the first warps of all CTAs before the second ones.
 __device__ __noinline__ void chain_pass_fp64(CrSmem& sm, const ChainPassP& pp, const void* in, double2* out,
-                                             const double2* U16, uint64_t ngroups, int in_fixed, int32_t F) {
+                                             const double2* gate, uint64_t ngroups, int in_fixed, int32_t F) {
+  double2* U16 = &sm.stage[0][0][0];
+  __syncthreads();
+  for (int t = (int)threadIdx.x; t < 256; t += CH_THREADS) U16[t] = gate[t];
+  __syncthreads();
   uint32_t okey = 0, ominc = 0;
-  for (uint64_t grp = (uint64_t)blockIdx.x * CH_THREADS + threadIdx.x; grp < ngroups;
-       grp += (uint64_t)gridDim.x * CH_THREADS) {
-    const uint32_t base = chain_base((uint32_t)grp, pp);
+  for (uint32_t c32 = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; c32 < (uint32_t)(ngroups / 32);
+       c32 += gridDim.x * (CH_THREADS / 32)) {
+    const uint32_t base = chain_base(c32 * 32 + (threadIdx.x & 31), pp);
     auto at = [&](int c) -> uint32_t {
       return base | ((c & 8) ? pp.tgt[0] : 0u) | ((c & 4) ? pp.tgt[1] : 0u) | ((c & 2) ? pp.tgt[2] : 0u) |
              ((c & 1) ? pp.tgt[3] : 0u);
