@@ -155,8 +155,9 @@ constexpr uint64_t CHAIN_RESIDENT_AMPS = 1ull << 22;
 // From this many such passes on: the launch has its tables to prepare (a clear, a kernel, a larger
 // workspace). Runs of 1, 2, 3, 5 later passes, in us with the first pass, launch per pass / one
 // launch: 27 / 33, 37 / 37, 47 / 43, 68 / 54 at 2^12 amplitudes; 44 / 51, 62 / 66, 72 / 71,
-// 102 / 91 at 2^20; 98 / 105, 130 / 135, 162 / 162, 239 / 228 at 2^22.
-constexpr size_t CHAIN_RESIDENT_PASSES = 3;
+// 102 / 91 at 2^20; 98 / 105, 130 / 135, 162 / 162, 239 / 228 at 2^22, there with one permutation
+// 162 / 167 with 3 and 198 / 193 with 4.
+constexpr size_t chain_resident_least(uint64_t amps) { return amps > (1ull << 21) ? 4 : 3; }
 // One of those passes: two disjoint two-qubit gates, and the permutation after them (perm) if
 // the pass is to write its outputs permuted, out of place.
 struct ChainStep {

@@ -449,7 +449,7 @@ bool apply_gate_runs_tc(void* state, void* scratch, dims_t dims, const std::vect
       // the first pass is a launch of its own (per-group scales); the later ones of a state that L2
       // holds go in launches of up to chain_resident_passes() passes, which end early only at a
       // permutation that cannot be folded into the pass before it, or, if those are fewer than
-      // CHAIN_RESIDENT_PASSES or the launch is refused, one by one
+      // chain_resident_least() or the launch is refused, one by one
       const uint64_t ngroups = steps[i].p.ngroups;
       const size_t most = chain_resident(steps[i].p) ? (size_t)chain_resident_passes() : 1;
       // one record per launch
@@ -459,7 +459,7 @@ bool apply_gate_runs_tc(void* state, void* scratch, dims_t dims, const std::vect
         size_t k = 0, t = i, launches = 0;
         std::vector<ChainStep> open;
         auto flush = [&] {
-          if (open.size() >= CHAIN_RESIDENT_PASSES && timed_pass(s, [&]() -> uint64_t {
+          if (open.size() >= chain_resident_least(ngroups * 16) && timed_pass(s, [&]() -> uint64_t {
                 return launch_chain_resident(cur, oth, open, ngroups, &recs[launches], &recs[launches + 1], s) ? open.size()
                                                                                                            : 0;
               })) {
