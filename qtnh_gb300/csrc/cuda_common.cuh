@@ -83,6 +83,10 @@ __device__ __forceinline__ void decode(uint64_t idx, const RestDesc& r, uint64_t
 __device__ __forceinline__ uint32_t fast_div(uint32_t x, uint32_t mul, uint32_t shift) {
   return (__umulhi(x, mul) + x) >> shift;
 }
+// The same for any 32-bit x: the sum's carry kept.
+__device__ __forceinline__ uint32_t fast_div_wide(uint32_t x, uint32_t mul, uint32_t shift) {
+  return (uint32_t)(((uint64_t)__umulhi(x, mul) + x) >> shift);
+}
 inline void fast_divisor(uint64_t d, uint32_t& mul, uint32_t& shift) {
   shift = 0;
   while ((1ull << shift) < d) ++shift;
