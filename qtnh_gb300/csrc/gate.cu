@@ -9,10 +9,10 @@
 // fixed), loads them with 128-bit loads, applies the D x D gate from shared memory and
 // stores them back. Consecutive threads own consecutive groups, so loads and stores are
 // coalesced unless a target is the innermost index, in which case every thread touches D
-// contiguous elements. The float-float form also takes D = 9 that way; for D = 8 and 16 (and 9
-// in FP64) the threads of a block share the groups through shared memory, one thread per
-// (output, group) (gate_coop_kernel); any other D runs a general FP64 kernel out of a copy
-// of the state (gate_kernel_any).
+// contiguous elements. The float-float form also takes D = 9 that way where the groups fill the
+// SMs; for D = 8 and 16 (and 9 in FP64 or on few groups) the threads of a block share the groups
+// through shared memory, one thread per (output, group) (gate_coop_kernel); any other D runs a
+// general FP64 kernel out of a copy of the state (gate_kernel_any).
 //
 // DiagTensor contraction (the reference stubs DiagTensor: src/tensor/diag.cpp:65-117)
 // is defined as contraction with D[in, out] = d[in] * delta(in, out); with the in-place
@@ -33,6 +33,7 @@ namespace qtnh_impl {
 namespace {
 
 constexpr int GATE_MAX_D = 16;
+constexpr uint64_t GATE9_GROUPS = 400;  // per SM, from where a thread holds a group of 9
 
 struct GateParams {
   RestDesc other;              // indices that are not gate targets, merged, with state strides in s_in
@@ -213,7 +214,7 @@ __global__ void __launch_bounds__(256, B) gate_kernel_f32x2(c128* __restrict__ p
   }
 }
 
-// Gates of 8 or 16 amplitudes per group (and 9 in FP64): the threads of a block share the groups'
+// Gates of 8 or 16 amplitudes per group (and 9 in FP64 or on few groups): the threads of a block share the groups'
 // amplitudes through shared memory, one thread per (output, group) and GB = 256 / D
 // groups per batch, instead of one thread holding a whole group in registers (which spills
 // in FP64 and leaves one 8-warp block per SM in float-float). Thread t takes group t % GB
@@ -348,11 +349,6 @@ struct Index32 {
     return idx;
   }
 };
-struct Index32Pow2 {
-  typedef uint32_t type;
-  static __device__ __forceinline__ uint32_t of(uint32_t e, const DiagParams& p) {
-    uint32_t idx = 0;
-    for (int j = 0; j < p.k; ++j) idx += ((e >> p.stride_log2[j]) & ((uint32_t)p.dim[j] - 1)) * (uint32_t)p.mult[j];
 // (3^20 elements, two targets: 21.3 ms; by 64-bit divisions 35.5, by 32-bit ones 31.9.)
 struct Index32Wide {
   typedef uint32_t type;
