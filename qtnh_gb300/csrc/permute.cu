@@ -173,8 +173,8 @@ __global__ void __launch_bounds__(TILE_THREADS, 4) tiled_permute_kernel(const c1
   }
 }
 
-// The same with the bases of a step's tiles decoded at its start, T a power of two: for steps of few
-// large tiles whose bases take little (plan_permute has the rule). 2^13 x 2^13 elements 357 us, in the
+// The same with the bases of a step's tiles decoded at its start, T a power of two or G 1: for blocks of
+// one step and for steps of few large tiles whose bases take little (plan_permute has the rule). 2^13 x 2^13 elements 357 us, in the
 // form above 385; that form with its bases decoded in step 426.
 __global__ void __launch_bounds__(TILE_THREADS, 4) tiled_permute_step_kernel(const c128* __restrict__ in,
                                                                           c128* __restrict__ out,
@@ -623,10 +623,17 @@ Plan plan_permute(const dims_t& dims, const std::vector<uint16_t>& ptup, int bou
     };
     p.tile_slots = (int)(swz ? PB * PA : PB * (PA + 1));
     const uint32_t tl = log2_or_none((uint64_t)T);
-    p.G = (tl != 0xFFFFFFFFu || boundary < 0) ? std::min(STEP_ELEMS / T, 256) : 1;
-    // a small tensor: fewer tiles per step rather than SMs without a block
-    if (boundary < 0) p.G = (int)std::max<uint64_t>(1, std::min<uint64_t>(p.G, N / T / (uint64_t)sm_count()));
-    p.T_log2 = tl == 0xFFFFFFFFu ? 0 : tl;
+    const bool pow2 = tl != 0xFFFFFFFFu;
+    p.G = (pow2 || boundary < 0) ? std::min(STEP_ELEMS / T, 256) : 1;
+    // a small tensor (one step for each SM, or less): fewer tiles per step rather than SMs without a
+    // block. Tiles of 512 and 1024 elements stay together: 128 blocks of one are slower than 64 of two
+    // (2^17 elements 10.7 us against 9.3). Tiles of 64, 2^13 elements: 4.3 us in 4 blocks, 2.9 in 128.
+    const uint64_t tiles = N / (uint64_t)T, sms = (uint64_t)sm_count();
+    const bool small = boundary < 0 && tiles <= (uint64_t)p.G * sms;
+    if (boundary < 0 && !pow2) p.G = (int)std::max<uint64_t>(1, std::min<uint64_t>(p.G, tiles / sms));
+    else if (small && T < 512)
+      for (; p.G > 1 && (uint64_t)(p.G / 2) * sms >= tiles;) p.G /= 2;
+    p.T_log2 = pow2 ? tl : 0;
     fast_divisor((uint64_t)T, p.T_mul, p.T_shift);
     // fused split: the tile's trailing output positions that are column axes form a run
     // of consecutive columns (stride 1 innermost); if its length is a multiple of 4,
@@ -689,13 +696,16 @@ Plan plan_permute(const dims_t& dims, const std::vector<uint16_t>& ptup, int bou
       if (!inA[i] && !inB[i]) fill_axis(p.rest.ax[nr++], c.dims[i], in_stride[i], out_stride[i]);
     p.rest.n = nr;
     p.rest.total = N / (uint64_t)T;
-    // Bases in step: steps of two or four tiles of a power of two of elements, with few axes left to
-    // decode them from; a step ahead otherwise. In us, in step / ahead: tiles of 1024 with two axes
+    // Bases in step: where a block has one step, which has no step before it to decode them in (tiles of
+    // other sizes than powers of two only one by one, as the kernel takes them), and for steps of two or
+    // four tiles of a power of two of elements, with few axes left to decode them from; a step ahead
+    // otherwise. One step, in us, in step / ahead: 2^7 elements 2.5 / 3.0, 3^8 3.9 / 4.2, 17 x 1024 5.7 /
+    // 6.3, 2^17 in a random order 7.0 / 9.8, 2^18 8.0 / 10.4. Several, in step / ahead: tiles of 1024 with two axes
     // left 31.6 / 35.0 at 2^20 elements, 47.2 / 53.3 at 2^22, 357 / 385 at 2^26, with 8 axes 49.4 / 53.3
     // (2^22), with 14 axes 121.1 / 119.8 (2^24); tiles of 512 with two axes 96.0 / 98.0 (2^24), with 9
     // 104.9 / 104.5; tiles of 256 with one axis 354 / 327 (2^26).
-    plan.ahead = boundary >= 0 || tl == 0xFFFFFFFFu || T < 512 || STEP_ELEMS / T * nr > 24;
-    if (!plan.ahead) p.G = STEP_ELEMS / T;
+    if (boundary < 0 && (pow2 ? small : p.G == 1)) plan.ahead = false;
+    else plan.ahead = boundary >= 0 || !pow2 || T < 512 || STEP_ELEMS / T * nr > 24;
     // one axis per lane costs less than divisions in turn, shifts in turn less than the lanes
     // (2^26 elements in a random order: 356 us by shifts, 404 by lanes)
     p.lanes = 0;
