@@ -34,7 +34,9 @@
 // a CTA has fewer than seven tiles (26 us instead of 24 at 64 tiles, 43 instead of 40 at 256): not worth
 // their code. The partials' sum is 255 us more (1.3 GB, 5.2 TB/s); summing a tile's slices
 // inside this kernel as they become complete took 1055 us in all: not worth its code
-// either. Every wait is bounded by a clock limit (device error flags).
+// either. Short K, one slice, is bound by C's stores and its conversions to double: 8192 x 8192 with
+// K 64 307 us; in 16-byte stores 635 (512 with the four warps). Every wait is bounded by a clock
+// limit (device error flags).
 
 #include <cuda_bf16.h>
 
@@ -184,6 +186,11 @@ __device__ __forceinline__ void store_sector(float* dst, const uint32_t* v) {
   asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(v[0]), "r"(v[1]), "r"(v[2]),
                "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
                : "memory");
+}
+
+// Two neighbouring elements of C (32 bytes, aligned).
+__device__ __forceinline__ void store_pair(double2* dst, double2 a, double2 b) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(dst), "d"(a.x), "d"(a.y), "d"(b.x), "d"(b.y) : "memory");
 }
 
 __global__ void __launch_bounds__(GM_THREADS, 1) gemm_bf16x3_umma_kernel(const __grid_constant__ GemmParams p) {
@@ -352,14 +359,36 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_bf16x3_umma_kernel(const _
         // the even lane (Re row) writes columns 0..15 of the chunk, the odd lane (Im row)
         // columns 16..31; each receives the other part from its partner
         const uint64_t n0 = nt * GM_N + (uint64_t)(h * CW + ch * 32) + (odd ? 16 : 0);
+        float re[16], im[16];
 #pragma unroll
         for (int x = 0; x < 16; ++x) {
           const uint32_t send = odd ? v[ch][x] : v[ch][16 + x];
           const uint32_t recv = __shfl_xor_sync(0xffffffffu, send, 1);
-          const float re = __uint_as_float(odd ? recv : v[ch][x]);
-          const float im = __uint_as_float(odd ? v[ch][16 + x] : recv);
-          const uint64_t n = n0 + (uint64_t)x;
-          if (m < p.M && n < p.N) p.C[m * p.N + n] = make_double2((double)re, (double)im);
+          re[x] = __uint_as_float(odd ? recv : v[ch][x]);
+          im[x] = __uint_as_float(odd ? v[ch][16 + x] : recv);
+        }
+        if (m >= p.M) continue;
+        double2* dst = p.C + m * p.N + n0;
+        if (n0 + 16 > p.N) {
+#pragma unroll
+          for (int x = 0; x < 16; ++x)
+            if (n0 + (uint64_t)x < p.N) dst[x] = make_double2((double)re[x], (double)im[x]);
+          continue;
+        }
+        // whole sectors, from the second element on where the first is the latter half of one (the
+        // same instructions for both: neighbouring rows of odd length differ, and the conversions
+        // take as long as the stores)
+        const bool al = ((uintptr_t)dst & 31) == 0;
+#pragma unroll
+        for (int x = 0; x < 16; x += 2) {
+          const int y = x < 14 ? x + 2 : x;  // (x = 14 is stored where aligned only)
+          const double2 a = make_double2((double)(al ? re[x] : re[x + 1]), (double)(al ? im[x] : im[x + 1]));
+          const double2 b = make_double2((double)(al ? re[x + 1] : re[y]), (double)(al ? im[x + 1] : im[y]));
+          if (x < 14 || al) store_pair(dst + x + (al ? 0 : 1), a, b);
+        }
+        if (!al) {
+          dst[0] = make_double2((double)re[0], (double)im[0]);
+          dst[15] = make_double2((double)re[15], (double)im[15]);
         }
       }
     }
