@@ -9,10 +9,10 @@
 // fixed), loads them with 128-bit loads, applies the D x D gate from shared memory and
 // stores them back. Consecutive threads own consecutive groups, so loads and stores are
 // coalesced unless a target is the innermost index, in which case every thread touches D
-// contiguous elements. The float-float form also takes D = 9 that way where the groups fill the
-// SMs; for D = 8 and 16 (and 9 in FP64 or on few groups) the threads of a block share the groups
-// through shared memory, one thread per (output, group) (gate_coop_kernel); any other D runs a
-// general FP64 kernel out of a copy of the state (gate_kernel_any).
+// contiguous elements. The float-float form also takes D = 9 that way; for D = 8 and 16 (and 9
+// in FP64) the threads of a block share the groups through shared memory, one thread per
+// (output, group) (gate_coop_kernel); any other D runs a general FP64 kernel out of a copy
+// of the state (gate_kernel_any).
 //
 // DiagTensor contraction (the reference stubs DiagTensor: src/tensor/diag.cpp:65-117)
 // is defined as contraction with D[in, out] = d[in] * delta(in, out); with the in-place
@@ -33,7 +33,6 @@ namespace qtnh_impl {
 namespace {
 
 constexpr int GATE_MAX_D = 16;
-constexpr uint64_t GATE9_GROUPS = 400;  // per SM, from where a thread holds a group of 9
 
 struct GateParams {
   RestDesc other;              // indices that are not gate targets, merged, with state strides in s_in
@@ -214,7 +213,7 @@ __global__ void __launch_bounds__(256, B) gate_kernel_f32x2(c128* __restrict__ p
   }
 }
 
-// Gates of 8 or 16 amplitudes per group (and 9 in FP64 or on few groups): the threads of a block share the groups'
+// Gates of 8 or 16 amplitudes per group (and 9 in FP64): the threads of a block share the groups'
 // amplitudes through shared memory, one thread per (output, group) and GB = 256 / D
 // groups per batch, instead of one thread holding a whole group in registers (which spills
 // in FP64 and leaves one 8-warp block per SM in float-float). Thread t takes group t % GB
@@ -322,14 +321,10 @@ constexpr int DU = 4;
 // less precise.
 constexpr int DIAG_FP64_SLOTS = 1, DIAG_PAIRS = 1, DIAG_STEPS = 2, DIAG_BLOCKS = 6, DIAG_HIGH_BLOCKS = 5;
 constexpr int LAYER_FP64_SLOTS = 1, LAYER_PAIRS = 1, LAYER_SINGLES = 1, LAYER_STEPS = 2, LAYER_BLOCKS = 3;
-// Blocks of the layer per SM, of which LAYER_BLOCKS at once: the SMs do not run alike, and with no
-// block left to take the slowest ones decide. 2^30 amplitudes, 3 / 9 blocks: 8.14 / 7.72 ms, 2^28
-// 1.98 / 1.88, 2^26 488 / 486 us, 2^16 the same.
-constexpr int LAYER_GRID = 9;
 constexpr uint64_t DIAG_SMEM = 256;  // diagonals of up to this many entries are split by each block
 
-// Index of element e over the targets. Four forms: 64 bits; 32 bits (states of 2^31 to 2^32 elements);
-// indices below 2^31; 32 bits with every extent and stride a power of two.
+// Index of element e over the targets. Three forms: 64 bits; 32 bits; 32 bits with every extent
+// and stride a power of two.
 struct Index64 {
   typedef uint64_t type;
   static __device__ __forceinline__ uint64_t of(uint64_t e, const DiagParams& p) {
@@ -349,18 +344,6 @@ struct Index32 {
     for (int j = 0; j < p.k; ++j) {
       const uint32_t q = fast_div(e, p.stride_mul[j], p.stride_shift[j]);
       idx += (q - fast_div(q, p.dim_mul[j], p.dim_shift[j]) * (uint32_t)p.dim[j]) * (uint32_t)p.mult[j];
-    }
-    return idx;
-  }
-};
-// (3^20 elements, two targets: 21.3 ms; by 64-bit divisions 35.5, by 32-bit ones 31.9.)
-struct Index32Wide {
-  typedef uint32_t type;
-  static __device__ __forceinline__ uint32_t of(uint32_t e, const DiagParams& p) {
-    uint32_t idx = 0;
-    for (int j = 0; j < p.k; ++j) {
-      const uint32_t q = fast_div_wide(e, p.stride_mul[j], p.stride_shift[j]);
-      idx += (q - fast_div_wide(q, p.dim_mul[j], p.dim_shift[j]) * (uint32_t)p.dim[j]) * (uint32_t)p.mult[j];
     }
     return idx;
   }
@@ -851,7 +834,7 @@ void apply_diag_device(void* state, const dims_t& dims, const std::vector<uint16
     p.stride_log2[j] = log2_or_none(p.stride[j]);
     pow2 = pow2 && p.dim_log2[j] != 0xFFFFFFFFu && p.stride_log2[j] != 0xFFFFFFFFu;
     high = high && p.stride[j] % 32 == 0;
-    if (n < (1ull << 32)) {
+    if (n < (1ull << 31)) {
       fast_divisor(p.dim[j], p.dim_mul[j], p.dim_shift[j]);
       fast_divisor(p.stride[j], p.stride_mul[j], p.stride_shift[j]);
     }
@@ -898,7 +881,6 @@ void apply_diag_device(void* state, const dims_t& dims, const std::vector<uint16
   else if (i32g) diag_kernel<Index32><<<grid, 256, 0, s>>>(st_, d_, p);
   else diag_kernel<Index64><<<grid, 256, 0, s>>>(st_, d_, p);
   count_launch();
-    else if (i32) f64 ? run(Index32Wide(), F64()) : run(Index32Wide(), F32());
   check_cuda(cudaGetLastError(), "diag_kernel launch");
 }
 
@@ -908,7 +890,6 @@ void apply_diag_layer_device(void* state, const dims_t& dims, const std::vector<
   if (axes.size() > (size_t)LAYER_MAX_FACTORS) throw Error(QTNH_ERR_UNSUPPORTED, "too many diagonal factors");
   const uint64_t n = product(dims);
   if (n == 0 || axes.empty()) return;
-  else if (i32) diag_kernel<Index32Wide><<<grid, 256, 0, s>>>(st_, d_, p);
   // Split the indices: trailing ones whose extent product is at most 4096 form the
   // low table, the rest the high table.
   const int r = (int)dims.size();
