@@ -323,8 +323,8 @@ constexpr int DIAG_FP64_SLOTS = 1, DIAG_PAIRS = 1, DIAG_STEPS = 2, DIAG_BLOCKS =
 constexpr int LAYER_FP64_SLOTS = 1, LAYER_PAIRS = 1, LAYER_SINGLES = 1, LAYER_STEPS = 2, LAYER_BLOCKS = 3;
 constexpr uint64_t DIAG_SMEM = 256;  // diagonals of up to this many entries are split by each block
 
-// Index of element e over the targets. Three forms: 64 bits; 32 bits; 32 bits with every extent
-// and stride a power of two.
+// Index of element e over the targets. Four forms: 64 bits; 32 bits (states of 2^31 to 2^32 elements);
+// indices below 2^31; 32 bits with every extent and stride a power of two.
 struct Index64 {
   typedef uint64_t type;
   static __device__ __forceinline__ uint64_t of(uint64_t e, const DiagParams& p) {
@@ -344,6 +344,18 @@ struct Index32 {
     for (int j = 0; j < p.k; ++j) {
       const uint32_t q = fast_div(e, p.stride_mul[j], p.stride_shift[j]);
       idx += (q - fast_div(q, p.dim_mul[j], p.dim_shift[j]) * (uint32_t)p.dim[j]) * (uint32_t)p.mult[j];
+    }
+    return idx;
+  }
+};
+// (3^20 elements, two targets: 21.3 ms; by 64-bit divisions 35.5, by 32-bit ones 31.9.)
+struct Index32Wide {
+  typedef uint32_t type;
+  static __device__ __forceinline__ uint32_t of(uint32_t e, const DiagParams& p) {
+    uint32_t idx = 0;
+    for (int j = 0; j < p.k; ++j) {
+      const uint32_t q = fast_div_wide(e, p.stride_mul[j], p.stride_shift[j]);
+      idx += (q - fast_div_wide(q, p.dim_mul[j], p.dim_shift[j]) * (uint32_t)p.dim[j]) * (uint32_t)p.mult[j];
     }
     return idx;
   }
@@ -834,7 +846,7 @@ void apply_diag_device(void* state, const dims_t& dims, const std::vector<uint16
     p.stride_log2[j] = log2_or_none(p.stride[j]);
     pow2 = pow2 && p.dim_log2[j] != 0xFFFFFFFFu && p.stride_log2[j] != 0xFFFFFFFFu;
     high = high && p.stride[j] % 32 == 0;
-    if (n < (1ull << 31)) {
+    if (n < (1ull << 32)) {
       fast_divisor(p.dim[j], p.dim_mul[j], p.dim_shift[j]);
       fast_divisor(p.stride[j], p.stride_mul[j], p.stride_shift[j]);
     }
@@ -870,6 +882,7 @@ void apply_diag_device(void* state, const dims_t& dims, const std::vector<uint16
     using F32 = std::integral_constant<int, 0>;
     if (i32 && pow2) f64 ? run(Index32Pow2(), F64()) : run(Index32Pow2(), F32());
     else if (i32g) f64 ? run(Index32(), F64()) : run(Index32(), F32());
+    else if (i32) f64 ? run(Index32Wide(), F64()) : run(Index32Wide(), F32());
     else f64 ? run(Index64(), F64()) : run(Index64(), F32());
     count_launch();
     const cudaError_t e = cudaGetLastError();
@@ -879,6 +892,7 @@ void apply_diag_device(void* state, const dims_t& dims, const std::vector<uint16
   }
   if (i32 && pow2) diag_kernel<Index32Pow2><<<grid, 256, 0, s>>>(st_, d_, p);
   else if (i32g) diag_kernel<Index32><<<grid, 256, 0, s>>>(st_, d_, p);
+  else if (i32) diag_kernel<Index32Wide><<<grid, 256, 0, s>>>(st_, d_, p);
   else diag_kernel<Index64><<<grid, 256, 0, s>>>(st_, d_, p);
   count_launch();
   check_cuda(cudaGetLastError(), "diag_kernel launch");
