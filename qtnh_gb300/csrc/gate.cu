@@ -9,10 +9,10 @@
 // fixed), loads them with 128-bit loads, applies the D x D gate from shared memory and
 // stores them back. Consecutive threads own consecutive groups, so loads and stores are
 // coalesced unless a target is the innermost index, in which case every thread touches D
-// contiguous elements. The float-float form also takes D = 9 that way; for D = 8 and 16 (and 9
-// in FP64) the threads of a block share the groups through shared memory, one thread per
-// (output, group) (gate_coop_kernel); any other D runs a general FP64 kernel out of a copy
-// of the state (gate_kernel_any).
+// contiguous elements. The float-float form also takes D = 9 that way where the groups fill the
+// SMs; for D = 8 and 16 (and 9 in FP64 or on few groups) the threads of a block share the groups
+// through shared memory, one thread per (output, group) (gate_coop_kernel); any other D runs a
+// general FP64 kernel out of a copy of the state (gate_kernel_any).
 //
 // DiagTensor contraction (the reference stubs DiagTensor: src/tensor/diag.cpp:65-117)
 // is defined as contraction with D[in, out] = d[in] * delta(in, out); with the in-place
@@ -33,6 +33,7 @@ namespace qtnh_impl {
 namespace {
 
 constexpr int GATE_MAX_D = 16;
+constexpr uint64_t GATE9_GROUPS = 400;  // per SM, from where a thread holds a group of 9
 
 struct GateParams {
   RestDesc other;              // indices that are not gate targets, merged, with state strides in s_in
@@ -213,7 +214,7 @@ __global__ void __launch_bounds__(256, B) gate_kernel_f32x2(c128* __restrict__ p
   }
 }
 
-// Gates of 8 or 16 amplitudes per group (and 9 in FP64): the threads of a block share the groups'
+// Gates of 8 or 16 amplitudes per group (and 9 in FP64 or on few groups): the threads of a block share the groups'
 // amplitudes through shared memory, one thread per (output, group) and GB = 256 / D
 // groups per batch, instead of one thread holding a whole group in registers (which spills
 // in FP64 and leaves one 8-warp block per SM in float-float). Thread t takes group t % GB
@@ -794,8 +795,14 @@ void apply_gate_device(void* state, const dims_t& dims, const std::vector<uint16
     QTNH_GATE_CASE(4, 3)
     QTNH_GATE_COOP_CASE(8)
     case 9: {
-      if (ff) QTNH_GATE_FF(9, 2)
-      else gate_coop_kernel<9, false><<<grid_for((p.other.total + 27) / 28, 8), 256, 0, s>>>(psi, g, p);
+      // a thread per group where that occupies most of the SMs' threads: below, its chain of 81 products is
+      // all the time there is. In us, cooperative / thread per group, the targets first: 3.5 / 8.1 on 3^7,
+      // 6.3 / 8.2 on 3^11, 13.1 / 13.2 on 9 x 50000, 13.9 / 13.4 on 3^12 (the targets last 14.2 / 14.9),
+      // 16.7 / 13.3 on 9 x 70000, 38 / 30 on 3^13, 108 / 80 on 3^14
+      const int cg = grid_for((p.other.total + 27) / 28, 8);
+      if (ff && p.other.total >= GATE9_GROUPS * (uint64_t)sm_count()) QTNH_GATE_FF(9, 2)
+      else if (ff) gate_coop_kernel<9, true><<<cg, 256, 0, s>>>(psi, g, p);
+      else gate_coop_kernel<9, false><<<cg, 256, 0, s>>>(psi, g, p);
       break;
     }
     QTNH_GATE_COOP_CASE(16)
