@@ -322,6 +322,10 @@ constexpr int DU = 4;
 // less precise.
 constexpr int DIAG_FP64_SLOTS = 1, DIAG_PAIRS = 1, DIAG_STEPS = 2, DIAG_BLOCKS = 6, DIAG_HIGH_BLOCKS = 5;
 constexpr int LAYER_FP64_SLOTS = 1, LAYER_PAIRS = 1, LAYER_SINGLES = 1, LAYER_STEPS = 2, LAYER_BLOCKS = 3;
+// Blocks of the layer per SM, of which LAYER_BLOCKS at once: the SMs do not run alike, and with no
+// block left to take the slowest ones decide. 2^30 amplitudes, 3 / 9 blocks: 8.14 / 7.72 ms, 2^28
+// 1.98 / 1.88, 2^26 488 / 486 us, 2^16 the same.
+constexpr int LAYER_GRID = 9;
 constexpr uint64_t DIAG_SMEM = 256;  // diagonals of up to this many entries are split by each block
 
 // Index of element e over the targets. Four forms: 64 bits; 32 bits (states of 2^31 to 2^32 elements);
@@ -957,7 +961,7 @@ void apply_diag_layer_device(void* state, const dims_t& dims, const std::vector<
       typedef decltype(idx) IT;
       constexpr int NF = decltype(slots)::value, E = NF + 2 * LAYER_PAIRS + LAYER_SINGLES;
       layer_apply_kernel_f32x2<IT, NF, LAYER_PAIRS, LAYER_SINGLES, LAYER_STEPS, LAYER_BLOCKS>
-          <<<grid_for((n + 256 * E - 1) / (256 * E), LAYER_BLOCKS), 256, 0, s>>>(st_, hi_t, tables, his, split_tab, n,
+          <<<grid_for((n + 256 * E - 1) / (256 * E), LAYER_GRID), 256, 0, s>>>(st_, hi_t, tables, his, split_tab, n,
                                                                              lo_size, lo_log2);
     };
     using F64 = std::integral_constant<int, LAYER_FP64_SLOTS>;
