@@ -463,7 +463,7 @@ def rdm4(precision, state, n, qubits, stream=None):
     """16 x 16 reduced density matrix of 4 qubits (complex128 CUDA tensor, FP64 sums)."""
     import torch
     _check_state(state, precision)
-    out = torch.empty(256, dtype=torch.complex128, device="cuda")
+    out = torch.empty((16, 16), dtype=torch.complex128, device="cuda")
     check(lib().qtnh_rdm4(ctypes.c_int32(precision), _ptr(state), ctypes.c_int32(n), _u16(qubits), _ptr(out),
                           _stream(stream)))
-    return out.reshape(16, 16)
+    return out

@@ -299,7 +299,8 @@ void group_renorm(int32_t ns, void* const* states, const int32_t* nq, cudaStream
 // and two diagonal entries (real) for each of the last 8 -- and two such sets on
 // alternate columns. The blocks' sums go to `part` (256 values a block: value 2 e and 2 e + 1
 // of thread e) and are added by rdm4_sum_kernel, a warp per value: atomic additions of all
-// blocks to the same 512 addresses cost more than the sums of small states. Bound: the
+// blocks to the same 512 addresses cost more than the sums of small states (they serve where there
+// is no memory for `part`). Bound: the
 // FP64 unit, 512 multiply-adds a column (0.72 of its rate at 23 qubits). All 256 entries with
 // atomic sums / this, us: 22.9 / 5.6 at 12 qubits, 24.9 / 16.0 at 17, 72 / 52 at 19, 919 / 625
 // at 23.
@@ -318,7 +319,7 @@ __device__ __forceinline__ void rdm_entry(int e, int& a, int& b) {
 
 template <typename T, int RDM_RCH>
 __global__ void __launch_bounds__(256) rdm4_kernel(const T* __restrict__ psi, uint64_t R, uint4 qbits, uint4 sorted,
-                                                   double* __restrict__ part) {
+                                                   double* __restrict__ part, double* __restrict__ rho) {
   __shared__ double2 M[16][RDM_RCH + 1];
   __shared__ double2 other[128];
   const int tid = threadIdx.x, e = tid & 127, set = tid >> 7;
@@ -362,8 +363,17 @@ __global__ void __launch_bounds__(256) rdm4_kernel(const T* __restrict__ psi, ui
   if (set == 1) other[e] = make_double2(re, im);
   __syncthreads();
   if (set == 0) {
-    part[(uint64_t)(2 * e) * gridDim.x + blockIdx.x] = re + other[e].x;
-    part[(uint64_t)(2 * e + 1) * gridDim.x + blockIdx.x] = im + other[e].y;
+    re += other[e].x, im += other[e].y;
+    if (part) {
+      part[(uint64_t)(2 * e) * gridDim.x + blockIdx.x] = re;
+      part[(uint64_t)(2 * e + 1) * gridDim.x + blockIdx.x] = im;
+    } else {
+      const int second = diag ? 17 * b : 16 * b + a;  // rho[b][b] or the mirror image
+      atomicAdd(&rho[2 * (diag ? 17 * a : 16 * a + b)], re);
+      atomicAdd(&rho[2 * (diag ? 17 * a : 16 * a + b) + 1], diag ? re - re : im);
+      atomicAdd(&rho[2 * second], diag ? im : re);
+      atomicAdd(&rho[2 * second + 1], diag ? im - im : -im);
+    }
   }
 }
 
@@ -491,18 +501,29 @@ int qtnh_rdm4(int32_t precision, const void* state, int32_t nqubits, const uint1
     const uint4 q4 = make_uint4(qb[0], qb[1], qb[2], qb[3]), s4 = make_uint4(sb[0], sb[1], sb[2], sb[3]);
     const float2* p32 = static_cast<const float2*>(state);
     const double2* p64 = static_cast<const double2*>(state);
-    double* part = static_cast<double*>(workspace_alloc(256 * sizeof(double) * (size_t)grid, stream));
-    if (precision == QTNH_STATE_C64) {
-      if (small) rdm4_kernel<float2, 8><<<grid, 256, 0, s>>>(p32, R, q4, s4, part);
-      else rdm4_kernel<float2, 64><<<grid, 256, 0, s>>>(p32, R, q4, s4, part);
-    } else {
-      if (small) rdm4_kernel<double2, 8><<<grid, 256, 0, s>>>(p64, R, q4, s4, part);
-      else rdm4_kernel<double2, 64><<<grid, 256, 0, s>>>(p64, R, q4, s4, part);
+    double* rho = static_cast<double*>(out_c128);
+    double* part = nullptr;
+    try {
+      part = static_cast<double*>(workspace_alloc(256 * sizeof(double) * (size_t)grid, stream));
+    } catch (const Error& e) {
+      if (e.code != QTNH_ERR_NO_MEMORY) throw;
+      cudaGetLastError();  // (not sticky)
+      check_cuda(cudaMemsetAsync(rho, 0, 256 * sizeof(double2), s), "rdm reset");
     }
-    rdm4_sum_kernel<<<32, 256, 0, s>>>(part, grid, static_cast<double*>(out_c128));
+    if (precision == QTNH_STATE_C64) {
+      if (small) rdm4_kernel<float2, 8><<<grid, 256, 0, s>>>(p32, R, q4, s4, part, rho);
+      else rdm4_kernel<float2, 64><<<grid, 256, 0, s>>>(p32, R, q4, s4, part, rho);
+    } else {
+      if (small) rdm4_kernel<double2, 8><<<grid, 256, 0, s>>>(p64, R, q4, s4, part, rho);
+      else rdm4_kernel<double2, 64><<<grid, 256, 0, s>>>(p64, R, q4, s4, part, rho);
+    }
+    count_launch();
+    if (part) {
+      rdm4_sum_kernel<<<32, 256, 0, s>>>(part, grid, rho);
+      count_launch();
+    }
     const cudaError_t e = cudaGetLastError();
-    workspace_free(part, stream);
-    count_launch(2);
+    if (part) workspace_free(part, stream);
     check_cuda(e, "rdm launch");
     return QTNH_OK;
   });
