@@ -33,6 +33,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 
 #include <cuda_fp16.h>
 
@@ -436,6 +437,7 @@ __global__ void __launch_bounds__(UM_THREADS, 2) gate_pair_umma_kernel(double2* 
 // (QTNH_CHAIN_LEVELS=6).
 constexpr int CH_ND = oz::NS;
 constexpr int CH_NLMAX = 7;
+constexpr uint64_t CHAIN_LOW_AMPS = 1ull << 21;  // launch_pair_chain
 constexpr int CH_WARPS = 16;                // team warps: four per TMEM lane quarter
 constexpr int CH_TEAM = CH_WARPS * 32;      // two tiles in flight: digits of one, MMAs of the other
 constexpr int CH_THREADS = CH_TEAM + 32;    // + the MMA warp
@@ -528,13 +530,12 @@ __device__ __forceinline__ void st_pair(void* p, int64_t a, int64_t b, int64_t c
 // part | offset) is the OR of the three parts' images, the row part's and the offsets'
 // computed once), so the pass and the permutation after it take one pass over the state.
 //
-// LOW (bit 0 among the targets, or bits 1 and 2): with the gates' order of amplitudes and rows
-// on the lanes such a pass moves half sectors (bits 1 and 2: scattered ones). Here amplitude
-// index bits go by descending target bit (`order`), so the lowest target bit's two values are
-// neighbouring amplitudes of one thread: fetched as whole sectors by neighbouring lanes and, at
-// bit 0, stored as one (`neighbours`: the output's base allows 32-byte stores). Such a pass took
-// 1.46 times the others' time and takes 1.37 times it; circuits of eight layers on 27 qubits
-// 44.06 -> 43.63 and 41.87 -> 41.18 ms.
+// LOW (bit 0 among the targets): with the gates' order of amplitudes and rows on the lanes such a pass
+// moves half sectors. Here amplitude index bits go by descending target bit (`order`), so the values
+// of bit 0 are neighbouring amplitudes of one thread: fetched as whole sectors by neighbouring lanes
+// and stored as one. In us, without / with it, two later passes with their first pass: 143 / 140 at 2^22
+// amplitudes, 1770 / 1733 at 2^26; circuits of eight layers, five of each size: 24 qubits 0.7 to 2.0 %, 26
+// 0.6 to 1.8, 27 0.3 to 1.1, 28 0.7 to 1.1 (runs of one circuit differ by 0.1, at 28 by 0.3).
 template <typename IT, uint32_t MODE, int NL, bool PO, bool LOW>
 __global__ void __launch_bounds__(CH_THREADS, 1) gate_pair_chain_kernel(void* __restrict__ psiv,
                                                                         const double2* __restrict__ ga,
@@ -543,8 +544,9 @@ __global__ void __launch_bounds__(CH_THREADS, 1) gate_pair_chain_kernel(void* __
                                                                         const ChainRec* __restrict__ rin,
                                                                         ChainRec* __restrict__ rout, int want_fixed,
                                                                         void* __restrict__ outv,
-                                                                        const __grid_constant__ BitMap perm, uint32_t order,
-                                                                        int neighbours) {
+                                                                        const __grid_constant__ BitMap perm,
+                                                                        uint32_t order) {
+  static_assert(!(PO && LOW), "whole sectors go where they came from");
   static_assert(!PO || sizeof(IT) == 4, "permuted output for states of at most 2^32 elements");
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   ChSmem& sm = *reinterpret_cast<ChSmem*>(smem_raw);
@@ -579,8 +581,9 @@ __global__ void __launch_bounds__(CH_THREADS, 1) gate_pair_chain_kernel(void* __
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  // amplitude index bit j of this pass is bit (order >> 4 j) & 15 of the gates' (a0 a1 b0 b1)
+  // LOW: amplitude index bit j of this pass is bit (order >> 4 j) & 15 of the gates' (a0 a1 b0 b1)
   auto gate_index = [&](int c) {
+    if (!LOW) return c;
     int g = 0;
 #pragma unroll
     for (int j = 0; j < 4; ++j) g |= ((c >> j) & 1) << ((order >> (4 * j)) & 15u);
@@ -712,14 +715,13 @@ __global__ void __launch_bounds__(CH_THREADS, 1) gate_pair_chain_kernel(void* __
     uint32_t kk = 0;
 #pragma unroll
     for (int a = 0; a < 4; ++a) kk |= (common ? 0u : (uint32_t)min(62, max_erow - sm.erow[4 * h + a])) << (8 * a);
-    // LOW: lane bit lb takes the place of amplitude index bit 0, so that a load covers both values
-    // of it in 16 of the warp's rows and its lanes read whole sectors
-    const uint32_t lb = p.ins_pos[0], amp0 = (uint32_t)(lane >> lb) & 1u;  // (lb < 3)
-    const int frow = q * 32 + ((lane & ((1 << lb) - 1)) | ((lane >> (lb + 1)) << lb));
+    // LOW: the lane's lowest bit takes the place of amplitude index bit 0, so that a load covers both
+    // values of it in 16 of the warp's rows and its lanes read whole sectors
+    const int amp0 = lane & 1, frow = q * 32 + (lane >> 1);
     const IT fbase = LOW ? pair_base<IT>((IT)frow, p) + (IT)p.off[4 * h + amp0] : IT(0);
     const IT step16 = LOW ? pair_base<IT>((IT)16, p) : IT(0), step2 = (IT)p.off[2];
     double2* const st = &sm.stage[0][0][0];
-    const int slot0 = chain_slot(4 * h + (int)amp0, frow), slot1 = chain_slot(4 * h + (int)amp0, frow + 16);
+    const int slot0 = chain_slot(4 * h + amp0, frow), slot1 = chain_slot(4 * h + amp0, frow + 16);
     // tile T into stage slot `slot` (its iteration % 2; one commit group per tile, empty past the end)
     auto fetch = [&](uint64_t T, IT tb, uint32_t slot) {
       if (T < ntiles) {
@@ -739,8 +741,6 @@ __global__ void __launch_bounds__(CH_THREADS, 1) gate_pair_chain_kernel(void* __
       cp_async_commit();
     };
     uint32_t okey = 0, ohi = 0;
-    // amplitudes 4h + a, a even, and 4h + a + 1 are neighbours in the output: stored as one sector
-    const bool pairs = LOW && neighbours != 0;
     // level sums from accumulator set b -> the outputs 4h .. 4h + 3 of group r of the tile
     // whose tile part is tb
     auto recombine = [&](IT tb, uint32_t b) {
@@ -751,7 +751,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) gate_pair_chain_kernel(void* __
 #pragma unroll
       for (int l = 0; l < NL; ++l) tmem_ld8(tbase + (uint32_t)(32 * l), v[l]);
       tmem_wait_ld();
-      int64_t Pr = 0, Pi = 0;  // the outputs of the even amplitude before
+      int64_t Pr = 0, Pi = 0;  // LOW: the outputs of the even amplitude before, one sector with the odd one's
 #pragma unroll
       for (int a = 0; a < 4; ++a) {
         float cr[NL], ci[NL];
@@ -772,7 +772,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) gate_pair_chain_kernel(void* __
             Yr = (Tr + rh) >> k, Yi = (Ti + rh) >> k;
           }
           ohi |= oz::fixed_hi_mag(Yr) | oz::fixed_hi_mag(Yi);  // its bit length is the largest's
-          if (!pairs)
+          if (!LOW)
             *reinterpret_cast<longlong2*>(pyo + 2 * (uint64_t)ix) = make_longlong2(Yr, Yi);
           else if (a & 1)
             st_pair(pyo + 2 * (uint64_t)(ix - 1), Pr, Pi, Yr, Yi);
@@ -1592,9 +1592,8 @@ void launch_umma(double2* psi, const double2* ga, const double2* gb, const PairP
 }
 
 template <typename IT, int NL, bool PO, bool LOW>
-void launch_chain_form(void* psi, const double2* ga, const double2* gb, const PairParams& p, cudaStream_t s,
-                  const ChainRec* rin, ChainRec* rout, bool want_fixed, void* out, const BitMap& perm, uint32_t order,
-                  bool neighbours) {
+void launch_chain(void* psi, const double2* ga, const double2* gb, const PairParams& p, cudaStream_t s,
+                  const ChainRec* rin, ChainRec* rout, bool want_fixed, void* out, const BitMap& perm, uint32_t order) {
   const size_t smem = sizeof(ChSmem);
   check_cuda(cudaFuncSetAttribute(gate_pair_chain_kernel<IT, PAIR_KRON, NL, PO, LOW>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
@@ -1602,15 +1601,7 @@ void launch_chain_form(void* psi, const double2* ga, const double2* gb, const Pa
   const uint64_t ntiles = p.ngroups / UM_M;
   const int grid = (int)std::min<uint64_t>(ntiles, (uint64_t)sm_count());  // one CTA per SM (all its TMEM)
   gate_pair_chain_kernel<IT, PAIR_KRON, NL, PO, LOW>
-      <<<grid, CH_THREADS, smem, s>>>(psi, ga, gb, p, rin, rout, want_fixed ? 1 : 0, out, perm, order, neighbours ? 1 : 0);
-}
-
-template <typename IT, int NL, bool PO>
-void launch_chain(void* psi, const double2* ga, const double2* gb, const PairParams& p, cudaStream_t s,
-                  const ChainRec* rin, ChainRec* rout, bool want_fixed, void* out, const BitMap& perm, uint32_t order,
-                  bool neighbours, bool low) {
-  if (low) launch_chain_form<IT, NL, PO, true>(psi, ga, gb, p, s, rin, rout, want_fixed, out, perm, order, neighbours);
-  else launch_chain_form<IT, NL, PO, false>(psi, ga, gb, p, s, rin, rout, want_fixed, out, perm, order, neighbours);
+      <<<grid, CH_THREADS, smem, s>>>(psi, ga, gb, p, rin, rout, want_fixed ? 1 : 0, out, perm, order);
 }
 
 int chain_levels() {
@@ -1627,44 +1618,40 @@ bool chain_applies(const PairParams& p) { return p.ngroups >= (uint64_t)UM_M && 
 
 void launch_pair_chain(void* psi, const double2* ga, const double2* gb, const PairParams& gp, cudaStream_t s,
                        const ChainRec* rin, ChainRec* rout, bool want_fixed, void* out, const BitMap* perm) {
-  // LOW form only where it gains: the exchange between the lanes of a warp costs the other passes
-  // 4 % (all passes in this form: 28 qubits 84.5 ms against 81.2; by this rule 80.6)
-  const bool low = gp.ins_pos[0] == 0 || (gp.ins_pos[0] == 1 && gp.ins_pos[1] == 2);
-  // amplitude index bits by descending target bit: bit j of the pass is target bit ins_pos[j]
-  PairParams p = gp;
-  uint32_t order = low ? 0 : 0x3210;
-  for (int j = 0; low && j < 4; ++j)
-    for (uint32_t b = 0; b < 4; ++b)
-      if ((uint64_t)gp.off[1 << b] == 1ull << gp.ins_pos[j]) order |= b << (4 * j);
-  auto gate_index = [&](int c) {
-    int g = 0;
-    for (int j = 0; j < 4; ++j) g |= ((c >> j) & 1) << ((order >> (4 * j)) & 15u);
-    return g;
-  };
-  for (int c = 0; c < 16; ++c) p.off[c] = gp.off[gate_index(c)];
-  // the two amplitudes of index bit 0 are neighbours where they are stored, at whole sectors
-  const bool adjacent = perm ? p.off[1] == 1ll << gp.ins_pos[0] && perm->dst[gp.ins_pos[0]] == 0 : p.off[1] == 1;
-  const bool nb = adjacent && ((uintptr_t)(perm ? out : psi) & 31) == 0;
-  const bool i32 = p.ngroups * 16 <= (1ull << 32);
+  const bool six = chain_levels() == 6;
   if (perm) {
-    if (!i32 || !out || out == psi) throw Error(QTNH_ERR_UNSUPPORTED, "permuted chain output");
-    if (chain_levels() == 6)
-      launch_chain<uint32_t, 6, true>(psi, ga, gb, p, s, rin, rout, want_fixed, out, *perm, order, nb, low);
-    else
-      launch_chain<uint32_t, 7, true>(psi, ga, gb, p, s, rin, rout, want_fixed, out, *perm, order, nb, low);
+    if (gp.ngroups * 16 > (1ull << 32) || !out || out == psi) throw Error(QTNH_ERR_UNSUPPORTED, "permuted chain output");
+    if (six) launch_chain<uint32_t, 6, true, false>(psi, ga, gb, gp, s, rin, rout, want_fixed, out, *perm, 0);
+    else launch_chain<uint32_t, 7, true, false>(psi, ga, gb, gp, s, rin, rout, want_fixed, out, *perm, 0);
     return;
   }
-  if (chain_levels() == 6) {
-    if (i32)
-      launch_chain<uint32_t, 6, false>(psi, ga, gb, p, s, rin, rout, want_fixed, nullptr, BitMap(), order, nb, low);
-    else
-      launch_chain<uint64_t, 6, false>(psi, ga, gb, p, s, rin, rout, want_fixed, nullptr, BitMap(), order, nb, low);
-  } else {
-    if (i32)
-      launch_chain<uint32_t, 7, false>(psi, ga, gb, p, s, rin, rout, want_fixed, nullptr, BitMap(), order, nb, low);
-    else
-      launch_chain<uint64_t, 7, false>(psi, ga, gb, p, s, rin, rout, want_fixed, nullptr, BitMap(), order, nb, low);
+  // LOW only where it gains, from 2^21 amplitudes on: below, its exchange between lanes costs more than L2's
+  // half sectors (2^12 34.2 / 38.3 us, 2^16 36.1 / 37.9, 2^20 60.7 / 61.3, 2^21 86.2 / 84.8). Nor where the
+  // outputs are permuted (2^24 600 / 620) or bits 1 and 2 are the lowest targets (2^26 1583 / 1612).
+  const bool low = gp.ins_pos[0] == 0 && gp.ngroups * 16 >= CHAIN_LOW_AMPS && ((uintptr_t)psi & 31) == 0;
+  // amplitude index bits by descending target bit: bit j of the pass is target bit ins_pos[j]
+  PairParams p = gp;
+  uint32_t order = 0;
+  if (low) {
+    for (int j = 0; j < 4; ++j)
+      for (uint32_t b = 0; b < 4; ++b)
+        if ((uint64_t)gp.off[1 << b] == 1ull << gp.ins_pos[j]) order |= b << (4 * j);
+    for (int c = 0; c < 16; ++c) {
+      p.off[c] = 0;
+      for (int j = 0; j < 4; ++j) p.off[c] |= ((c >> j) & 1) ? (int64_t)(1ull << gp.ins_pos[j]) : 0;
+    }
   }
+  const bool i32 = p.ngroups * 16 <= (1ull << 32);
+  auto run = [&](auto idx, auto levels, auto lowest) {
+    launch_chain<decltype(idx), decltype(levels)::value, false, decltype(lowest)::value>(
+        psi, ga, gb, p, s, rin, rout, want_fixed, nullptr, BitMap(), order);
+  };
+  auto by_levels = [&](auto idx, auto lowest) {
+    if (six) run(idx, std::integral_constant<int, 6>(), lowest);
+    else run(idx, std::integral_constant<int, 7>(), lowest);
+  };
+  if (i32) low ? by_levels(uint32_t(), std::true_type()) : by_levels(uint32_t(), std::false_type());
+  else low ? by_levels(uint64_t(), std::true_type()) : by_levels(uint64_t(), std::false_type());
 }
 
 // The bits of x moved to the positions outside the holes (ascending).
