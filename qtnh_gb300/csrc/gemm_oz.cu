@@ -46,8 +46,8 @@
 // 1.4 PFLOP/s of digit products) against two half tiles, eight drain warps and chunks
 // drained whole. In cycles of a chunk: 9840, of which MMAs 5930, waits for the drain 2180 (it
 // takes 2660) and for stages 1730 (36 KB a K-step from L2). One such K-step instead of two
-// takes 1325 us where two take 1279 and three 1313 (hides less; more in the MMAs); bringing A
-// to L2 ahead of the ring and a sixth stage change nothing.
+// makes the contraction 3.6 % slower (it hides less), three 2.7 % (more MMAs); bringing A to L2
+// ahead of the ring and a sixth stage change nothing.
 // Every wait is bounded by a clock limit; on expiry the CTA records an error flag
 // (qtnh_take_device_errors, bits 16-18), stops and frees its tensor memory.
 //
