@@ -324,8 +324,11 @@ constexpr int DIAG_FP64_SLOTS = 1, DIAG_PAIRS = 1, DIAG_STEPS = 2, DIAG_BLOCKS =
 constexpr int LAYER_FP64_SLOTS = 1, LAYER_PAIRS = 1, LAYER_SINGLES = 1, LAYER_STEPS = 2, LAYER_BLOCKS = 3;
 // Blocks of the layer per SM, of which LAYER_BLOCKS at once: the SMs do not run alike, and with no
 // block left to take the slowest ones decide. 2^30 amplitudes, 3 / 9 blocks: 8.14 / 7.72 ms, 2^28
-// 1.98 / 1.88, 2^26 488 / 486 us, 2^16 the same.
-constexpr int LAYER_GRID = 9;
+// 1.98 / 1.88, 2^26 488 / 486 us, 2^16 the same; 9 / 18 / 36 blocks: 2^33 66.1 / 59.4 / 58.6 ms (8 blocks
+// without the copy ring 64.9), 3^21 108 / 96.7 / 95.4, 2^32 33.1 / 29.6 / 29.1, 2^28 1.91 / 1.88 / 1.88,
+// 2^26 507 / 504 / 511 us. (32-bit indices: three steps of all blocks stay below index32's allowance.)
+constexpr int LAYER_GRID = 18;
+static_assert(3 * LAYER_GRID * (LAYER_FP64_SLOTS + 2 * LAYER_PAIRS + LAYER_SINGLES) <= 8 * 32, "index32");
 constexpr uint64_t DIAG_SMEM = 256;  // diagonals of up to this many entries are split by each block
 
 // Index of element e over the targets. Four forms: 64 bits; 32 bits (states of 2^31 to 2^32 elements);
